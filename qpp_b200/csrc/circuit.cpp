@@ -7,6 +7,7 @@
 
 #include "kernels.hpp"
 #include "ops.hpp"
+#include "reg_tiles.hpp"
 #include "tile_gates.hpp"
 #include "traj.hpp"
 
@@ -512,10 +513,10 @@ static void prepare_tiled_blocks(qgpu_state* s, qgpu_circuit* c) {
     tiled_runs(c, runs);
     for (const TiledRun& r : runs) {
         if (r.step >= 0) {
-            F->runs.push_back({r.step, TileProgram{}});
+            F->runs.push_back({r.step, RegProgram{}});
         } else if (!r.gates.empty()) {
-            TileProgram P;
-            plan_tile_program(schedule_gates(r.gates, int(c->nq), Tmax), int(c->nq), Tmax, P);
+            RegProgram P;
+            plan_reg_program(schedule_reg_gates(r.gates, int(c->nq), Tmax), int(c->nq), Tmax, P);
             F->runs.push_back({-1, std::move(P)});
         }
     }
@@ -529,7 +530,7 @@ static void launch_tiled_blocks(qgpu_state* s, qgpu_circuit* c) {
     prepare_tiled_blocks(s, c);
     for (const auto& r : c->ftiles->runs) {
         if (r.first >= 0) apply_step(s, c->steps[size_t(r.first)]);
-        else run_tile_program(s, r.second);
+        else run_reg_program(s, r.second);
     }
 }
 

@@ -1,6 +1,6 @@
 // kernels_tile.cu -- cache-blocked tile passes: runs of 1- and 2-qubit gates
-// (controlled or not) applied to a qubit ket in one read and one write of the
-// state.
+// (controlled or not) applied to a complex64 qubit ket in one read and one
+// write of the state (complex128 kets: kernels_regtile.cu).
 //
 // Replaces, for runs of consecutive gates, the one-pass-per-gate loops of
 // include/qpp/internal/kernels/qubit/apply.hpp:57-265 (apply_psi_1q/2q) and
@@ -256,30 +256,23 @@ __global__ void __launch_bounds__(kTileThreads, 1)
     }
 }
 
-size_t tile_pass_smem(qgpu_prec prec, const TilePassParams& p) {
-    const size_t elem = prec == QGPU_C128 ? 16 : 8;
-    return (elem << p.T) + ((sizeof(uint64_t) << (p.T - p.L)) + 15) / 16 * 16 +
-           (sizeof(TileGate) * p.ngates + 15) / 16 * 16 + elem * p.mat_elems;
+size_t tile_pass_smem(const TilePassParams& p) {
+    return (sizeof(float2) << p.T) + ((sizeof(uint64_t) << (p.T - p.L)) + 15) / 16 * 16 +
+           (sizeof(TileGate) * p.ngates + 15) / 16 * 16 + sizeof(float2) * p.mat_elems;
 }
 
-void launch_tile_pass(qgpu_ctx* ctx, qgpu_prec prec, void* data, const TilePassParams& p,
-                      const TileGate* gates, const TileSweep* sweeps, const void* mats) {
-    const size_t smem = tile_pass_smem(prec, p);
+void launch_tile_pass(qgpu_ctx* ctx, void* data, const TilePassParams& p, const TileGate* gates,
+                      const TileSweep* sweeps, const void* mats) {
+    const size_t smem = tile_pass_smem(p);
     if (smem > kTileSmemMax)
         raise(QGPU_ERR_NOT_SUPPORTED, "qgpu_run_gates()", "tile above the shared memory");
-    ensure_smem(prec == QGPU_C128 ? reinterpret_cast<const void*>(k_tile_pass<double>)
-                                  : reinterpret_cast<const void*>(k_tile_pass<float>),
-                kTileSmemMax);
+    ensure_smem(reinterpret_cast<const void*>(k_tile_pass<float>), kTileSmemMax);
     // residency per SM from shared memory (228 KB, 1 KB reserved per CTA)
     // and threads (2048)
     const int per_sm = std::max(1, std::min(2048 / kTileThreads, int(232448 / (smem + 1024))));
     const int grid = int(std::min<uint64_t>(p.ntiles, uint64_t(ctx->num_sms) * per_sm));
-    if (prec == QGPU_C128)
-        k_tile_pass<double><<<grid, kTileThreads, smem, ctx->stream>>>(
-            static_cast<double2*>(data), p, gates, sweeps, static_cast<const double2*>(mats));
-    else
-        k_tile_pass<float><<<grid, kTileThreads, smem, ctx->stream>>>(
-            static_cast<float2*>(data), p, gates, sweeps, static_cast<const float2*>(mats));
+    k_tile_pass<float><<<grid, kTileThreads, smem, ctx->stream>>>(
+        static_cast<float2*>(data), p, gates, sweeps, static_cast<const float2*>(mats));
     after_launch(ctx, "k_tile_pass");
 }
 

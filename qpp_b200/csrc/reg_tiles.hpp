@@ -1,0 +1,100 @@
+// reg_tiles.hpp -- complex128 tile passes with the tile held in registers
+// (reg_tiles.cpp plans them on the host, kernels_regtile.cu runs them).
+#pragma once
+
+#include <cstdint>
+#include <vector>
+
+#include "tile_gates.hpp"
+
+namespace qgpu {
+
+// A tile of 2^T amplitudes is spread over one CTA: every tile bit sits in one
+// slot, and slots [0, NR) number a thread's 2^NR registers, [NR, NR + 5) its
+// lane, [NR + 5, T) its warp. A pass is a program of ops that every thread of
+// the CTA runs in lockstep:
+//   kRtG2      4 x 4 on the bits in lane slots 0 and 1 (amplitude index
+//              lane & 3), two FP64 matrix instructions per register
+//   kRtG1R a   2 x 2 on the bit in register slot a
+//   kRtG1L a   2 x 2 on the bit in lane slot a (its partner by a shuffle)
+//   kRtSwap    lane slot a and register slot b trade their bits
+//   kRtPerm    lane slots permuted: slot i takes the bit of slot perm[i]
+//              (coef = perm[i] << 3 i)
+//   kRtLayout  every bit to a new slot through shared memory: written in
+//              layout table coef, read back in table coef + 1
+enum : uint8_t { kRtG2 = 0, kRtG1R = 1, kRtG1L = 2, kRtSwap = 3, kRtPerm = 4, kRtLayout = 5 };
+
+// Controls hold a gate to the amplitudes whose register, lane, warp and
+// out-of-tile index bits under the masks equal the values.
+struct RtOp {
+    uint8_t type, a, b, ctrl;
+    uint32_t coef; // gates: 16-byte units from the pass's coefficients
+    uint8_t rmask, rval, lmask, lval, wmask, wval, pad[2];
+    uint32_t pad2;
+    uint64_t gmask, gval;
+};
+static_assert(sizeof(RtOp) == 40, "op size");
+
+// The swizzled shared-memory position contributed by the bit of each slot
+// (positions are XORs of these). Table 0 is the layout the tile is first read
+// in, the last one the layout it is written back in.
+struct RtLayoutTab {
+    uint16_t img[16];
+};
+
+constexpr int kRtMaxTile = 12; // 64 KB of complex128, two CTAs per SM
+constexpr int kRtMinTile = 7;  // 4 registers per lane, one warp
+// Shared memory of a CTA (two per SM), and what a pass's program may take of
+// it next to the largest tile and its offset table.
+constexpr size_t kRtSmemMax = 112 * 1024;
+constexpr size_t kRtBlobMax = 44 * 1024;
+
+struct RegPass {
+    uint64_t ntiles;
+    int T, L, NR;
+    int hi[16];         // state bits of tile bits L .. T - 1, ascending
+    uint32_t nvalid;    // amplitudes of the tile that exist (states below 2^kRtMinTile)
+    uint32_t nops, nlay;
+    uint32_t blob, blob_bytes; // the pass's ops, layouts and coefficients
+    uint32_t first, ngates;    // its gates in the program
+};
+
+struct RegProgram {
+    int nbits = 0;
+    std::vector<GateDesc> gates; // in pass order
+    std::vector<RegPass> passes;
+    std::vector<unsigned char> blob;
+};
+
+// The tile shape for an nbits-qubit ket: T bits of which the L lowest state
+// bits always belong to the tile, and 2^NR registers per thread.
+void reg_tile_shape(int nbits, int Tmax, int& T, int& L, int& NR);
+// Gates reordered for fewer passes and layouts (list scheduling, see
+// schedule_gates): each bit's gates keep their order.
+std::vector<GateDesc> schedule_reg_gates(const std::vector<GateDesc>& gates, int nbits, int Tmax);
+// Cuts the gates, in order, into passes and compiles each into its program.
+void plan_reg_program(const std::vector<GateDesc>& gates, int nbits, int Tmax, RegProgram& P);
+
+// The fused complex128 tile form of a circuit, planned once: list-scheduled
+// tile programs and the unfused steps between them, for the circuit's first
+// nsteps steps and tiles of at most Tmax bits.
+struct FusedTiles {
+    uint64_t nsteps = 0;
+    int Tmax = 0;
+    std::vector<std::pair<int64_t, RegProgram>> runs; // first >= 0: that step as it is
+};
+
+// Swizzled shared-memory position of tile element e (complex128).
+inline uint32_t rt_swz(uint32_t e) {
+    uint32_t r = e >> 3, h = 0;
+    for (int k = 0; k < 16; k += 3) h ^= r >> k;
+    return e ^ (h & 7u);
+}
+
+// Launches pass p (its tables at device address `blob`) on the ket at data;
+// chained: the previous launch on the stream was the pass before it, so this
+// one may start early and wait for it on the device.
+void launch_reg_pass(qgpu_ctx* ctx, void* data, const RegPass& p, const unsigned char* blob,
+                     bool chained);
+
+} // namespace qgpu
