@@ -415,8 +415,7 @@ typedef enum qgpu_form {
 /* Kets: the unitary steps (measurements and classical control need an
  * engine). QGPU_FORM_FUSED on a qubit ket merges gates into blocks: of <= 6
  * qubits in complex64 (on the tensor cores from 13 qubits); in complex128,
- * of <= 2 qubits run as tile passes up to 22 qubits and of <= 3 qubits as
- * dense passes above. QGPU_FORM_FUSED on a complex64 qubit density matrix of <= 15
+ * of <= 2 qubits run as tile passes. QGPU_FORM_FUSED on a complex64 qubit density matrix of <= 15
  * qubits whose circuit holds only gates and 1- or 2-qubit channels:
  * superoperators on the 2n virtual qubits (column digits, row digits) merged
  * into blocks of <= 4 virtual qubits, one pass over the matrix per block

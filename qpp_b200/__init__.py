@@ -655,9 +655,8 @@ class Circuit:
         """Apply the unitary steps to a resident State (in place). PLAIN keeps
         qpp's arithmetic per gate. FUSED merges gates into blocks: on a
         complex64 qubit ket of <= 6 qubits each (the tensor cores from 13
-        qubits), on a complex128 qubit ket of <= 2 qubits run as tile passes
-        (up to 22 qubits) or <= 3 qubits as dense passes (above); on a
-        complex64 qubit density matrix, gates and channels as superoperator
+        qubits), on a complex128 qubit ket of <= 2 qubits run as tile passes;
+        on a complex64 qubit density matrix, gates and channels as superoperator
         blocks of <= 4 virtual qubits (6 on the tensor cores from 11
         qubits)."""
         check(lib().qgpu_run_gates(state.h, self.h, ct.c_int(form)))

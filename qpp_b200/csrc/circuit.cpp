@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <functional>
 #include <map>
 
 #include "kernels.hpp"
@@ -463,18 +464,15 @@ void launch_program(qgpu_state* s, const TProgram& P) {
     }
 }
 
-// Complex128 qubit kets of up to 22 qubits (64 MiB, half the L2) run the
-// fused form as tile passes over blocks of <= 2 qubits. Such a state is read
-// from the L2, so a pass's time follows its FP64 work per amplitude, and
-// blocks of <= 2 qubits keep that work lowest: a 1-qubit gate merged into a
-// neighbouring 2-qubit block costs nothing, where a 3-qubit block costs as
-// much as two 2-qubit gates. Larger complex128 kets are HBM-bound and take
-// blocks of <= 3 qubits as dense passes, fewer trips through HBM.
-constexpr size_t kFusedTileQubitsC128 = 22;
-
+// Complex128 qubit kets run the fused form as register tile passes over blocks
+// of <= 2 qubits. Such a pass is bound by its FP64 work per amplitude, which
+// blocks of <= 2 qubits keep lowest: a 1-qubit gate merged into a neighbouring
+// 2-qubit block costs nothing, where a 3-qubit block costs as much as two
+// 2-qubit gates. Also above the L2: three layers on 24 / 26 / 27 qubits run in
+// 1.18 / 5.3 / 10.8 ms, as dense passes over blocks of <= 3 qubits (one trip
+// through HBM each) they took 2.61 / 11.7 / 22.1 ms.
 static bool fused_tiles(const qgpu_state* s) {
-    return s->kind == QGPU_KET && s->prec == QGPU_C128 && !s->dims.empty() &&
-           s->dims.size() <= kFusedTileQubitsC128;
+    return s->kind == QGPU_KET && s->prec == QGPU_C128 && !s->dims.empty();
 }
 
 void tiled_runs(const qgpu_circuit* c, std::vector<TiledRun>& out) {
@@ -499,44 +497,59 @@ void tiled_runs(const qgpu_circuit* c, std::vector<TiledRun>& out) {
     }
 }
 
-// Plans the fused plan's blocks (<= 2 qubits, c->plan) and its unfused
-// steps as tile programs once per circuit (again after steps are added or
-// the tile size changes): each run list-scheduled into fewer passes and
-// sweeps, then cut into passes.
-static void prepare_tiled_blocks(qgpu_state* s, qgpu_circuit* c) {
+// Runs the pieces of a complex128 ket circuit -- tile programs, and the steps
+// the passes do not take, run as they are -- planned once per circuit (again
+// after steps are added or the tile size changes). `kept` is the circuit's
+// slot for the plan; the first run launches each pass as it is planned, since
+// planning the 1100-gate benchmark circuit takes about as long on the host as
+// its passes take on the device.
+static void run_tile_pieces(qgpu_state* s, qgpu_circuit* c, std::shared_ptr<const FusedTiles>& kept,
+                            const std::function<void(std::vector<TiledRun>&)>& pieces) {
     const int Tmax = tile_bits_max(s->ctx, s->prec);
-    if (c->ftiles && c->ftiles->nsteps == c->steps.size() && c->ftiles->Tmax == Tmax) return;
+    std::shared_ptr<const FusedTiles> have;
+    {
+        std::lock_guard<std::mutex> lock(c->tiles_mu);
+        if (kept && kept->nsteps == c->steps.size() && kept->Tmax == Tmax) have = kept;
+    }
+    if (have) {
+        for (const auto& r : have->runs) {
+            if (r.first >= 0) apply_step(s, c->steps[size_t(r.first)]);
+            else run_reg_program(s, r.second);
+        }
+        return;
+    }
     auto F = std::make_shared<FusedTiles>();
     F->nsteps = c->steps.size();
     F->Tmax = Tmax;
     std::vector<TiledRun> runs;
-    tiled_runs(c, runs);
+    pieces(runs);
     for (const TiledRun& r : runs) {
         if (r.step >= 0) {
+            apply_step(s, c->steps[size_t(r.step)]);
             F->runs.push_back({r.step, RegProgram{}});
         } else if (!r.gates.empty()) {
-            RegProgram P;
-            plan_reg_program(schedule_reg_gates(r.gates, int(c->nq), Tmax), int(c->nq), Tmax, P);
-            F->runs.push_back({-1, std::move(P)});
+            F->runs.push_back({-1, RegProgram{}});
+            plan_and_run_reg(s, r.gates, Tmax, F->runs.back().second);
         }
     }
-    c->ftiles = std::move(F);
+    std::lock_guard<std::mutex> lock(c->tiles_mu);
+    kept = std::move(F);
 }
 
-// The planned tile programs in order, a step the passes do not take run as
-// it is between them.
-static void launch_tiled_blocks(qgpu_state* s, qgpu_circuit* c) {
-    prepare_plan(s, c, 2); // both no-ops after fused_prepare
-    prepare_tiled_blocks(s, c);
-    for (const auto& r : c->ftiles->runs) {
-        if (r.first >= 0) apply_step(s, c->steps[size_t(r.first)]);
-        else run_reg_program(s, r.second);
+// The plain form's pieces: every step's gates as they are.
+static void plain_runs(const qgpu_circuit* c, std::vector<TiledRun>& out) {
+    out.clear();
+    out.emplace_back();
+    for (size_t i = 0; i < c->steps.size(); ++i) {
+        if (gate_desc_of(c->steps[i], int(c->nq), out.back().gates)) continue;
+        out.emplace_back();
+        out.back().step = int64_t(i);
+        out.emplace_back();
     }
 }
 
 // Kets: qubits only; blocks of up to 6 qubits (complex64: 3-6 qubit blocks on
-// the tensor cores from 13 qubits on); in complex128, 2 (as tile passes) up to
-// 22 qubits and 3 above.
+// the tensor cores from 13 qubits on); in complex128, 2 (as tile passes).
 void fused_prepare(qgpu_state* s, qgpu_circuit* c) {
     if (s->kind == QGPU_RHO) {
         if (rho_tc_prepare(s, c)) {
@@ -547,8 +560,7 @@ void fused_prepare(qgpu_state* s, qgpu_circuit* c) {
     }
     if (c->d != 2)
         raise(QGPU_ERR_NOT_SUPPORTED, "qgpu_run_gates()", "fused form needs a qubit ket");
-    prepare_plan(s, c, s->prec == QGPU_C64 ? 6 : fused_tiles(s) ? 2 : 3);
-    if (fused_tiles(s)) prepare_tiled_blocks(s, c);
+    prepare_plan(s, c, s->prec == QGPU_C64 ? 6 : 2);
     if (!c->block_slot.empty()) ctx_error_flag(s->ctx); // allocated outside any capture
 }
 
@@ -561,7 +573,11 @@ void fused_launch(qgpu_state* s, qgpu_circuit* c) {
         }
         return launch_program(s, *c->rho_prog);
     }
-    if (fused_tiles(s)) return launch_tiled_blocks(s, c);
+    if (fused_tiles(s)) {
+        prepare_plan(s, c, 2); // a no-op after fused_prepare
+        run_tile_pieces(s, c, c->ftiles, [&](std::vector<TiledRun>& out) { tiled_runs(c, out); });
+        return;
+    }
     launch_blocks(s, vspace_ket(s->dims), int(c->nq), c->plan, c->dB, c->block_slot, c->steps);
 }
 
@@ -573,6 +589,10 @@ void run_gates(qgpu_state* s, qgpu_circuit* c, int form, uint64_t first, uint64_
     if (form == 0) {
         // qubit kets: runs of 1- and 2-qubit gates as tile passes
         const bool tiles = s->kind == QGPU_KET && c->d == 2 && !s->dims.empty();
+        if (tiles && s->prec == QGPU_C128 && first == 0 && count >= c->steps.size()) {
+            run_tile_pieces(s, c, c->ptiles, [&](std::vector<TiledRun>& out) { plain_runs(c, out); });
+            return;
+        }
         std::vector<GateDesc> run;
         for (uint64_t i = first; i < first + count && i < c->steps.size(); ++i) {
             if (tiles && gate_desc_of(c->steps[i], int(c->nq), run)) continue;

@@ -17,6 +17,7 @@
 #include <complex>
 #include <cstdint>
 #include <memory>
+#include <mutex>
 #include <vector>
 
 #include "internal.hpp"
@@ -90,7 +91,10 @@ struct qgpu_circuit {
     std::shared_ptr<qgpu::TProgram> rho_prog; // null: the form does not apply
     // fused complex128 ket form as tile passes (blocks of <= 2 qubits),
     // planned for the first ftiles->nsteps steps
-    std::shared_ptr<qgpu::FusedTiles> ftiles;
+    std::shared_ptr<const qgpu::FusedTiles> ftiles;
+    // the same of the plain form (the gates as they are); tiles_mu guards both
+    std::shared_ptr<const qgpu::FusedTiles> ptiles;
+    std::mutex tiles_mu;
     // fused density-matrix form on the tensor cores (complex64, 2n >= 13
     // virtual qubits): superoperator blocks of <= 6 virtual qubits, built for
     // the first rho_tc_steps steps

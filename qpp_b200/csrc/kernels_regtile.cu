@@ -24,8 +24,11 @@
 // memory is needed once in several gates; a tile kept in shared memory, with a
 // trip through it for every three bits, ran at 28% of the FP64 pipe. Measured
 // on one B200 against that form: 1100 gates on 2^20 amplitudes gate by gate
-// 3.00 -> 1.61 ms, merged into 2-qubit blocks 1.40 -> 0.97 ms, 126 gates on
-// 2^28 amplitudes 85.2 -> 45.2 ms.
+// 2.96 -> 1.52 ms, merged into 2-qubit blocks 1.40 -> 0.90 ms, 126 gates on
+// 2^28 amplitudes 88.4 -> 42.6 ms. Per pass over 2^20 amplitudes: about 6 us in
+// and out, 1.1 us per 2-qubit gate (the pipe's time), 0.8 or 1.2 us per 1-qubit
+// gate on a register or lane slot, 0.33 us per swap or permutation, 1.6 us per
+// layout change.
 #include <cuda_runtime.h>
 
 #include <algorithm>

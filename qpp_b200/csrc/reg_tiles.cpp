@@ -7,7 +7,6 @@
 
 #include <algorithm>
 #include <cstring>
-#include <set>
 
 namespace qgpu {
 
@@ -17,20 +16,10 @@ void reg_tile_shape(int nbits, int Tmax, int& T, int& L, int& NR) {
     // fewer amplitudes each: few tiles, bound by latency), the full 2^12 tile
     // 16 (9 bits inside a warp, 8 warps).
     NR = T == kRtMaxTile ? 4 : 2;
-    // runs of 2^L contiguous amplitudes; a tile keeps room for two targets
-    L = T >= nbits ? T : std::min(4, T - 2);
-}
-
-static int target_bits(const GateDesc& g, int (&b)[2]) {
-    b[0] = g.b0;
-    b[1] = g.b1;
-    return g.op == 2 ? 2 : 1;
-}
-
-std::vector<GateDesc> schedule_reg_gates(const std::vector<GateDesc>& gates, int nbits, int Tmax) {
-    int T, L, NR;
-    reg_tile_shape(nbits, Tmax, T, L, NR);
-    return schedule_gates(gates, nbits, L, T - L, NR + 5);
+    // Runs of 2^L contiguous amplitudes (128 bytes, one line) leave 9 bits to
+    // choose; L = 4 ran as fast (42.6 and 43.2 ms for 126 gates on 28 qubits)
+    // with a few passes more. A tile keeps room for two targets.
+    L = T >= nbits ? T : std::min(3, T - 2);
 }
 
 namespace {
@@ -39,6 +28,82 @@ namespace {
 // tables, the gate and its coefficients.
 constexpr size_t kGateBytes[3] = {0, 3 * sizeof(RtOp) + 2 * sizeof(RtLayoutTab) + 64,
                                   4 * sizeof(RtOp) + 2 * sizeof(RtLayoutTab) + 512};
+
+// A gate waiting to be placed: its target bits and all its bits (targets and
+// controls).
+struct Waiting {
+    uint64_t t, a;
+    uint32_t id;
+    uint32_t weight;
+};
+
+// The gates that a pass (or a stretch of it inside a warp) on the bits S can
+// take: in order, every gate whose targets lie in S and which shares no bit
+// with an earlier gate left behind.
+uint32_t reach(const std::vector<Waiting>& g, uint64_t S, uint64_t all) {
+    uint64_t behind = 0;
+    uint32_t sum = 0;
+    for (const Waiting& x : g) {
+        if (!(x.t & ~S) && !(x.a & behind)) {
+            sum += x.weight;
+        } else {
+            behind |= x.a;
+            if (behind == all) break;
+        }
+    }
+    return sum;
+}
+
+// The set of `size` bits (those of `fixed` among them, out of `pool`) whose
+// reach is large: grown in gate order, then improved by trading one bit at a
+// time. Trading costs the bits in times the bits out evaluations of a few
+// dozen gates each; on 1100 random gates of 20 qubits it saves a fifth of the
+// passes that growing alone needs.
+uint64_t choose_bits(const std::vector<Waiting>& g, uint64_t fixed, uint64_t pool, int size) {
+    uint64_t all = 0, S = fixed, behind = 0;
+    for (const Waiting& x : g) all |= x.a;
+    for (const Waiting& x : g) {
+        if (!(x.a & behind) && __builtin_popcountll(S | x.t) <= size) S |= x.t;
+        else if ((behind |= x.a) == all) break;
+    }
+    for (uint64_t r = pool & ~S; r && __builtin_popcountll(S) < size; r &= r - 1) S |= r & (0 - r);
+    uint32_t best = reach(g, S, all);
+    for (int round = 0; round < 8; ++round) {
+        uint64_t top = S;
+        for (uint64_t in = S & ~fixed; in; in &= in - 1)
+            for (uint64_t out = pool & all & ~S; out; out &= out - 1) {
+                const uint64_t S2 = (S ^ (in & (0 - in))) | (out & (0 - out));
+                const uint32_t r = reach(g, S2, all);
+                if (r > best) {
+                    best = r;
+                    top = S2;
+                }
+            }
+        if (top == S) break;
+        S = top;
+    }
+    return S;
+}
+
+// Moves the gates that S reaches from g to `out`, in order, at most `most`
+// program bytes of them.
+void take(std::vector<Waiting>& g, uint64_t S, size_t most, std::vector<Waiting>& out) {
+    uint64_t behind = 0;
+    size_t bytes = 0, keep = 0;
+    bool full = false;
+    for (const Waiting& x : g) {
+        const size_t cost = kGateBytes[x.t & (x.t - 1) ? 2 : 1];
+        if (!full && !(x.t & ~S) && !(x.a & behind) && bytes + cost <= most) {
+            bytes += cost;
+            out.push_back(x);
+        } else {
+            full = full || bytes + cost > most;
+            behind |= x.a;
+            g[keep++] = x;
+        }
+    }
+    g.resize(keep);
+}
 
 // One pass's program under construction.
 struct Builder {
@@ -68,28 +133,19 @@ struct Builder {
         return ops.back();
     }
 
-    // The layout for the gates [i, e) (their bits fit in a warp), `later` the
-    // order in which the pass's other bits are wanted afterwards.
-    void choose(const std::vector<GateDesc>& g, size_t i, size_t e, const std::vector<int>& later,
-                bool first) {
+    // The layout for a stretch of gates inside the bits `in` of a warp.
+    void choose(const std::vector<const GateDesc*>& g, const std::vector<int>& in, bool first) {
         int use[16] = {0};
-        std::vector<int> in; // bits of these gates
         int pair[2] = {-1, -1};
-        for (size_t k = i; k < e; ++k) {
-            int b[2];
-            const int nb = target_bits(g[k], b);
-            if (nb == 2 && pair[0] < 0) {
-                pair[0] = b[0];
-                pair[1] = b[1];
-            }
-            for (int x = 0; x < nb; ++x) {
-                if (!use[b[x]]++) in.push_back(b[x]);
+        for (const GateDesc* x : g) {
+            ++use[x->b0];
+            if (x->op != 2) continue;
+            ++use[x->b1];
+            if (pair[0] < 0) {
+                pair[0] = x->b0;
+                pair[1] = x->b1;
             }
         }
-        for (int b : later)
-            if (int(in.size()) < inwarp && std::find(in.begin(), in.end(), b) == in.end()) in.push_back(b);
-        for (int b = 0; b < T && int(in.size()) < inwarp; ++b)
-            if (std::find(in.begin(), in.end(), b) == in.end()) in.push_back(b);
         int next[16], n = 0;
         bool used[16] = {false};
         std::fill(next, next + 16, -1);
@@ -169,6 +225,18 @@ struct Builder {
         op(kRtPerm, 0, 0, c);
     }
 
+    // The moves that gate g (bits local to the tile) needs now.
+    int moves(const GateDesc& g) const {
+        if (g.op == 1) return slot_of(g.b0) < NR ? 0 : 3; // a shuffle of every register
+        int m = 0;
+        for (int b : {g.b0, g.b1}) {
+            const int s = slot_of(b);
+            m += s == NR || s == NR + 1 ? 0 : 1;
+        }
+        return m;
+    }
+
+    // Applies g with its controls on tile bits (local) and on others.
     void gate(const GateDesc& g, const std::vector<std::pair<int, int>>& local,
               const std::vector<std::pair<int, int>>& outside) {
         RtOp o;
@@ -219,88 +287,122 @@ struct Builder {
 
 } // namespace
 
-void plan_reg_program(const std::vector<GateDesc>& gates, int nbits, int Tmax, RegProgram& P) {
+size_t reg_program_bytes(const std::vector<GateDesc>& gates) {
+    size_t b = 0; // every gate at most in a pass of its own
+    for (const GateDesc& g : gates) b += kGateBytes[g.op] + 64;
+    return b;
+}
+
+void plan_reg_program(const std::vector<GateDesc>& gates, int nbits, int Tmax, RegProgram& P,
+                      const std::function<void(const RegPass&)>& planned) {
     P.nbits = nbits;
-    P.gates = gates;
     P.passes.clear();
+    P.single.clear();
     P.blob.clear();
+    P.blob.reserve(reg_program_bytes(gates));
     int T, L, NR;
     reg_tile_shape(nbits, Tmax, T, L, NR);
     const int nfree = T - L;
-    for (size_t i = 0; i < gates.size();) {
-        // the pass: gates in order while their bits above the low L fit
-        uint64_t hi = 0;
-        size_t j = i, bytes = 0;
-        for (; j < gates.size(); ++j) {
-            int b[2];
-            const int nb = target_bits(gates[j], b);
-            uint64_t h2 = hi;
-            for (int x = 0; x < nb; ++x)
-                if (b[x] >= L) h2 |= uint64_t(1) << b[x];
-            bytes += kGateBytes[nb];
-            if (__builtin_popcountll(h2) > nfree || bytes > kRtBlobMax) break;
-            hi = h2;
-        }
-        if (j == i) raise(QGPU_ERR_NOT_SUPPORTED, "qgpu_run_gates()", "tile too small");
-        // bits left over: the lowest others, for longer runs
-        for (int b = L; __builtin_popcountll(hi) < nfree; ++b) hi |= uint64_t(1) << b;
+    const uint64_t low = (uint64_t(1) << L) - 1, every = (uint64_t(1) << std::max(nbits, T)) - 1;
+    std::vector<Waiting> wait, pass, run;
+    wait.reserve(gates.size());
+    for (size_t k = 0; k < gates.size(); ++k) {
+        const GateDesc& g = gates[k];
+        Waiting w;
+        w.t = uint64_t(1) << g.b0;
+        if (g.op == 2) w.t |= uint64_t(1) << g.b1;
+        w.a = w.t;
+        for (const auto& c : g.ctrl) w.a |= uint64_t(1) << c.first;
+        w.id = uint32_t(k);
+        w.weight = uint32_t(g.op);
+        wait.push_back(w);
+    }
+    std::vector<GateDesc> loc; // the pass's gates on tile bits
+    while (!wait.empty()) {
+        const uint64_t S = choose_bits(wait, low, every, T);
+        pass.clear();
+        take(wait, S, kRtBlobMax - 64, pass);
+        if (pass.empty()) raise(QGPU_ERR_NOT_SUPPORTED, "qgpu_run_gates()", "tile too small");
         RegPass p;
         std::memset(&p, 0, sizeof(p));
         p.T = T;
         p.L = L;
         p.NR = NR;
         int nh = 0;
-        for (int b = 0; b < 64; ++b)
-            if ((hi >> b) & 1u) p.hi[nh++] = b;
+        for (int b = L; b < 64 && nh < nfree; ++b)
+            if ((S >> b) & 1u) p.hi[nh++] = b;
         p.ntiles = nbits > T ? uint64_t(1) << (nbits - T) : 1;
         p.nvalid = nbits < T ? 1u << nbits : 1u << T;
-        p.first = uint32_t(i);
-        p.ngates = uint32_t(j - i);
+        p.ngates = uint32_t(pass.size());
+        p.single = -1;
+        if (pass.size() == 1 && gates[pass[0].id].ctrl.empty()) {
+            p.single = int(P.single.size());
+            P.single.push_back(gates[pass[0].id]);
+        }
         auto local = [&](int b) {
             return b < L ? b : L + int(std::find(p.hi, p.hi + nh, b) - p.hi);
         };
-        // the gates on tile bits
-        std::vector<GateDesc> g(gates.begin() + ptrdiff_t(i), gates.begin() + ptrdiff_t(j));
-        for (GateDesc& x : g) {
-            x.b0 = local(x.b0);
-            if (x.op == 2) x.b1 = local(x.b1);
+        // the gates on tile bits, numbered within the pass; controls outside
+        // the tile stay where they are (and order nothing inside it: a gate
+        // on such a bit is not in this pass)
+        loc.resize(pass.size());
+        for (size_t k = 0; k < pass.size(); ++k) {
+            loc[k] = gates[pass[k].id];
+            Waiting w;
+            w.id = uint32_t(k);
+            loc[k].b0 = local(loc[k].b0);
+            w.t = uint64_t(1) << loc[k].b0;
+            if (loc[k].op == 2) {
+                loc[k].b1 = local(loc[k].b1);
+                w.t |= uint64_t(1) << loc[k].b1;
+            }
+            w.a = w.t;
+            for (const auto& c : loc[k].ctrl)
+                if ((S >> c.first) & 1u) w.a |= uint64_t(1) << local(c.first);
+            w.weight = pass[k].weight;
+            pass[k] = w;
         }
         Builder B;
         B.T = T;
         B.NR = NR;
         B.inwarp = NR + 5;
-        for (size_t k = 0; k < g.size();) {
-            // the longest run whose bits fit in a warp
-            uint32_t bits = 0;
-            size_t e = k;
-            for (; e < g.size(); ++e) {
-                int b[2];
-                const int nb = target_bits(g[e], b);
-                uint32_t w = bits;
-                for (int x = 0; x < nb; ++x) w |= 1u << b[x];
-                if (__builtin_popcount(w) > B.inwarp) break;
-                bits = w;
-            }
-            bool fits = k > 0;
-            for (int s = B.inwarp; s < T && fits; ++s) fits = !((bits >> B.at[s]) & 1u);
-            if (!fits) {
-                std::vector<int> later;
-                for (size_t x = e; x < g.size() && later.size() < 16; ++x) {
-                    int b[2];
-                    const int nb = target_bits(g[x], b);
-                    for (int y = 0; y < nb; ++y)
-                        if (std::find(later.begin(), later.end(), b[y]) == later.end()) later.push_back(b[y]);
+        bool first = true;
+        while (!pass.empty()) {
+            // a stretch of gates on the bits of one warp
+            const uint64_t W = choose_bits(pass, 0, (uint64_t(1) << T) - 1, B.inwarp);
+            run.clear();
+            take(pass, W, ~size_t(0), run);
+            std::vector<int> in;
+            for (int b = 0; b < T; ++b)
+                if ((W >> b) & 1u) in.push_back(b);
+            std::vector<const GateDesc*> rg;
+            for (const Waiting& w : run) rg.push_back(&loc[w.id]);
+            B.choose(rg, in, first);
+            first = false;
+            // next the gate that needs the fewest moves among those whose
+            // bits no earlier one of the stretch still waits for
+            while (!run.empty()) {
+                uint64_t seen = 0;
+                size_t pick = 0;
+                int least = 99;
+                for (size_t k = 0; k < run.size() && least; ++k) {
+                    if (!(run[k].a & seen)) {
+                        const int m = B.moves(loc[run[k].id]);
+                        if (m < least) {
+                            least = m;
+                            pick = k;
+                        }
+                    }
+                    seen |= run[k].a;
                 }
-                B.choose(g, k, e, later, k == 0);
-            }
-            for (; k < e; ++k) {
-                std::vector<std::pair<int, int>> in, out;
-                for (auto& c : g[k].ctrl) {
-                    const bool tile = c.first < L || ((hi >> c.first) & 1u);
-                    if (tile) in.push_back({local(c.first), c.second});
-                    else out.push_back(c);
+                const GateDesc& g = loc[run[pick].id];
+                std::vector<std::pair<int, int>> inside, outside;
+                for (auto& c : g.ctrl) {
+                    if ((S >> c.first) & 1u) inside.push_back({local(c.first), c.second});
+                    else outside.push_back(c);
                 }
-                B.gate(g[k], in, out);
+                B.gate(g, inside, outside);
+                run.erase(run.begin() + ptrdiff_t(pick));
             }
         }
         B.table();
@@ -316,7 +418,7 @@ void plan_reg_program(const std::vector<GateDesc>& gates, int nbits, int Tmax, R
         std::memcpy(d + b_ops, B.lays.data(), b_lay);
         std::memcpy(d + b_ops + b_lay, B.coef.data(), B.coef.size() * sizeof(cd));
         P.passes.push_back(p);
-        i = j;
+        if (planned) planned(p);
     }
 }
 

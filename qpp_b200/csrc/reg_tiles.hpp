@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cstdint>
+#include <functional>
 #include <vector>
 
 #include "tile_gates.hpp"
@@ -56,24 +57,29 @@ struct RegPass {
     uint32_t nvalid;    // amplitudes of the tile that exist (states below 2^kRtMinTile)
     uint32_t nops, nlay;
     uint32_t blob, blob_bytes; // the pass's ops, layouts and coefficients
-    uint32_t first, ngates;    // its gates in the program
+    uint32_t ngates;
+    int single;                // index of its only gate in RegProgram::single, or -1
 };
 
 struct RegProgram {
     int nbits = 0;
-    std::vector<GateDesc> gates; // in pass order
     std::vector<RegPass> passes;
+    std::vector<GateDesc> single; // passes of one uncontrolled gate
     std::vector<unsigned char> blob;
 };
 
 // The tile shape for an nbits-qubit ket: T bits of which the L lowest state
 // bits always belong to the tile, and 2^NR registers per thread.
 void reg_tile_shape(int nbits, int Tmax, int& T, int& L, int& NR);
-// Gates reordered for fewer passes and layouts (list scheduling, see
-// schedule_gates): each bit's gates keep their order.
-std::vector<GateDesc> schedule_reg_gates(const std::vector<GateDesc>& gates, int nbits, int Tmax);
-// Cuts the gates, in order, into passes and compiles each into its program.
-void plan_reg_program(const std::vector<GateDesc>& gates, int nbits, int Tmax, RegProgram& P);
+// Cuts the gates into passes and compiles each into its program. Gates on
+// disjoint bits trade places (list scheduling); each bit's gates keep their
+// order, so the product is the same up to rounding.
+// `planned`, when given, is called after each pass with its tables in P.blob,
+// so that the device can start while the host plans on.
+void plan_reg_program(const std::vector<GateDesc>& gates, int nbits, int Tmax, RegProgram& P,
+                      const std::function<void(const RegPass&)>& planned = nullptr);
+// An upper bound of the program's bytes.
+size_t reg_program_bytes(const std::vector<GateDesc>& gates);
 
 // The fused complex128 tile form of a circuit, planned once: list-scheduled
 // tile programs and the unfused steps between them, for the circuit's first

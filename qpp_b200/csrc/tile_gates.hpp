@@ -41,10 +41,6 @@ void plan_gate_tiles(const std::vector<GateDesc>& gates, int nbits, int Tmax,
 // every ready gate whose targets fit the tile, those that extend the current
 // sweep first. For forms that do not promise the gate-by-gate arithmetic.
 std::vector<GateDesc> schedule_gates(const std::vector<GateDesc>& gates, int nbits, int Tmax);
-// The same for tiles of the low L bits and nfree others, and sweeps of
-// sweep_bits bits.
-std::vector<GateDesc> schedule_gates(const std::vector<GateDesc>& gates, int nbits, int L, int nfree,
-                                     int sweep_bits);
 // Largest tile (bits) for this context and precision: 13 for complex128 and
 // 14 for complex64 (128 KB of shared memory), or qgpu_ctx_set_tile_bits's.
 int tile_bits_max(const qgpu_ctx* ctx, qgpu_prec prec);
@@ -64,6 +60,8 @@ void plan_tile_program(const std::vector<GateDesc>& gates, int nbits, int Tmax, 
 void run_tile_program(qgpu_state* s, const TileProgram& P);
 struct RegProgram;
 void run_reg_program(qgpu_state* s, const RegProgram& P);
+// Plans the gates into P, each pass launched as soon as it is planned.
+void plan_and_run_reg(qgpu_state* s, const std::vector<GateDesc>& gates, int Tmax, RegProgram& P);
 // Runs `gates` on the qubit ket s as planned tile passes (stream order).
 void run_tiled_gates(qgpu_state* s, const std::vector<GateDesc>& gates);
 

@@ -1,5 +1,4 @@
-// CPU check of the complex128 register tile passes (qgpu::schedule_reg_gates,
-// qgpu::plan_reg_program): a host model of k_reg_tile -- the tile spread over
+// CPU check of the complex128 register tile passes (qgpu::plan_reg_program): a host model of k_reg_tile -- the tile spread over
 // registers, lanes and warps, the shuffles, the layout changes through shared
 // memory and the matrix fragments of the 2-qubit gates -- runs the planned
 // programs of random 1- and 2-qubit gates with 0-3 controls on kets of 1-15
@@ -194,27 +193,26 @@ int main() {
             for (auto& x : psi) x = C(nd(rng), nd(rng));
             std::vector<C> ref = psi;
             for (const auto& g : gates) apply_direct(ref, g);
-            for (bool sched : {false, true}) {
-                RegProgram P;
-                plan_reg_program(sched ? schedule_reg_gates(gates, nbits, Tmax) : gates, nbits, Tmax, P);
-                std::vector<C> got = psi;
-                uint32_t covered = 0;
-                for (const RegPass& p : P.passes) {
-                    EXPECT(p.first == covered && p.blob % 16 == 0 && p.blob + p.blob_bytes <= P.blob.size());
-                    covered += p.ngates;
-                    std::vector<int> visits(psi.size(), 0);
-                    run_pass(got, p, P.blob.data() + p.blob, visits);
-                    for (int x : visits) EXPECT(x == 1);
-                }
-                EXPECT(covered == gates.size());
-                double top = 0, err = 0;
-                for (size_t i = 0; i < ref.size(); ++i) {
-                    top = std::max(top, std::abs(ref[i]));
-                    err = std::max(err, std::abs(got[i] - ref[i]));
-                }
-                EXPECT(err <= 1e-13 * top);
-                ++cases;
+            RegProgram P;
+            plan_reg_program(gates, nbits, Tmax, P);
+            std::vector<C> got = psi;
+            uint32_t covered = 0;
+            for (const RegPass& p : P.passes) {
+                EXPECT(p.blob % 16 == 0 && p.blob + p.blob_bytes <= P.blob.size());
+                EXPECT(p.single < 0 || (p.ngates == 1 && P.single[size_t(p.single)].ctrl.empty()));
+                covered += p.ngates;
+                std::vector<int> visits(psi.size(), 0);
+                run_pass(got, p, P.blob.data() + p.blob, visits);
+                for (int x : visits) EXPECT(x == 1);
             }
+            EXPECT(covered == gates.size());
+            double top = 0, err = 0;
+            for (size_t i = 0; i < ref.size(); ++i) {
+                top = std::max(top, std::abs(ref[i]));
+                err = std::max(err, std::abs(got[i] - ref[i]));
+            }
+            EXPECT(err <= 1e-13 * top);
+            ++cases;
         }
     if (fails) {
         std::printf("%d failures\n", fails);
