@@ -107,11 +107,10 @@ void* qgpu_ctx_stream(qgpu_ctx* ctx);
 qgpu_status qgpu_ctx_set_wait_test(qgpu_ctx* ctx, uint32_t spin_limit, int stall_next);
 /* Largest tile, in state bits (5..14), of the tile passes that run the plain
  * form of qgpu_run_gates on qubit kets (runs of 1- and 2-qubit gates, each run
- * one read and one write of the state); 0 restores the default, which is
- * also the cap: 12 for complex128 (64 KB, held in registers; tiles of fewer
- * than 7 bits run as 7) and 14 for complex64 (128 KB of shared memory). No
- * counterpart
- * in Quantum++, which applies one gate per pass. */
+ * one read and one write of the state); 0 restores the default, which is also
+ * the cap: 12 (64 KB in complex128, 32 KB in complex64, held in registers;
+ * tiles of fewer than 7 bits run as 7). No counterpart in Quantum++, which
+ * applies one gate per pass. */
 qgpu_status qgpu_ctx_set_tile_bits(qgpu_ctx* ctx, int bits);
 
 /* ---------------------------------------------------------------- states */

@@ -497,7 +497,7 @@ void tiled_runs(const qgpu_circuit* c, std::vector<TiledRun>& out) {
     }
 }
 
-// Runs the pieces of a complex128 ket circuit -- tile programs, and the steps
+// Runs the pieces of a qubit ket circuit -- tile programs, and the steps
 // the passes do not take, run as they are -- planned once per circuit (again
 // after steps are added or the tile size changes). `kept` is the circuit's
 // slot for the plan; the first run launches each pass as it is planned, since
@@ -505,7 +505,7 @@ void tiled_runs(const qgpu_circuit* c, std::vector<TiledRun>& out) {
 // its passes take on the device.
 static void run_tile_pieces(qgpu_state* s, qgpu_circuit* c, std::shared_ptr<const FusedTiles>& kept,
                             const std::function<void(std::vector<TiledRun>&)>& pieces) {
-    const int Tmax = tile_bits_max(s->ctx, s->prec);
+    const int Tmax = tile_bits_max(s->ctx);
     std::shared_ptr<const FusedTiles> have;
     {
         std::lock_guard<std::mutex> lock(c->tiles_mu);
@@ -589,8 +589,8 @@ void run_gates(qgpu_state* s, qgpu_circuit* c, int form, uint64_t first, uint64_
     if (form == 0) {
         // qubit kets: runs of 1- and 2-qubit gates as tile passes
         const bool tiles = s->kind == QGPU_KET && c->d == 2 && !s->dims.empty();
-        if (tiles && s->prec == QGPU_C128 && first == 0 && count >= c->steps.size()) {
-            run_tile_pieces(s, c, c->ptiles, [&](std::vector<TiledRun>& out) { plain_runs(c, out); });
+        if (tiles && first == 0 && count >= c->steps.size()) {
+            run_tile_pieces(s, c, c->ptiles[s->prec == QGPU_C64], [&](std::vector<TiledRun>& out) { plain_runs(c, out); });
             return;
         }
         std::vector<GateDesc> run;

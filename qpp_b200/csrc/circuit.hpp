@@ -92,8 +92,9 @@ struct qgpu_circuit {
     // fused complex128 ket form as tile passes (blocks of <= 2 qubits),
     // planned for the first ftiles->nsteps steps
     std::shared_ptr<const qgpu::FusedTiles> ftiles;
-    // the same of the plain form (the gates as they are); tiles_mu guards both
-    std::shared_ptr<const qgpu::FusedTiles> ptiles;
+    // the same of the plain form (the gates as they are) in complex128 and
+    // complex64; tiles_mu guards all three
+    std::shared_ptr<const qgpu::FusedTiles> ptiles[2];
     std::mutex tiles_mu;
     // fused density-matrix form on the tensor cores (complex64, 2n >= 13
     // virtual qubits): superoperator blocks of <= 6 virtual qubits, built for

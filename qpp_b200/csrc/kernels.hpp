@@ -39,7 +39,8 @@ void launch_apply_generic(qgpu_ctx* ctx, qgpu_prec prec, void* data,
 void launch_apply_kron4(qgpu_ctx* ctx, qgpu_prec prec, void* data, const SegPlan& outer,
                         const std::vector<uint64_t>& off, const cd* A, const cd* B);
 
-// --- tile passes (kernels_tile.cu) -----------------------------------------
+// --- tile passes as gate lists (plan_gate_tiles): the host description of a
+// run cut into passes and sweeps; the kernels take reg_tiles.hpp's programs ---
 // One gate of a tile pass on a qubit ket: op 1 = 2 x 2 on tile bit t0, op 2 =
 // 4 x 4 on tile bits (t0, t1) with row index 2 * b(t0) + b(t1); the matrix is
 // row-major at mats + mat (state precision). It acts on the amplitudes i of
@@ -75,12 +76,9 @@ struct TilePassParams {
     uint32_t first_sweep, nsweeps;
     uint32_t mat_first, mat_elems;
 };
-size_t tile_pass_smem(const TilePassParams& p);
 // Drops the cached device address of qgpu_ptrace_noalloc's offset table for
 // `device` (kernels_subsys.cu); the next call looks it up again.
 void noalloc_forget(int device);
-void launch_tile_pass(qgpu_ctx* ctx, void* data, const TilePassParams& p,
-                      const TileGate* gates, const TileSweep* sweeps, const void* mats);
 
 // --- subsystem kernels (kernels_subsys.cu) --------------------------------
 // out[o] = in[map(o)], o over map.count.

@@ -1,16 +1,17 @@
-// reg_tiles.cpp -- host planning of the complex128 register tile passes
-// (kernels_regtile.cu): which gates share a pass, and the program that moves
-// their bits into place and applies them. No reference counterpart: Quantum++
+// reg_tiles.cpp -- host planning of the register tile passes
+// (kernels_regtile.cu, kernels_regtile32.cu): which gates share a pass, and the
+// program that moves their bits into place and applies them. No reference counterpart: Quantum++
 // applies every gate as its own pass over the state (QEngine::visit_gate_step_,
 // qengine.hpp:551-578 -> apply / applyCTRL).
 #include "reg_tiles.hpp"
 
 #include <algorithm>
+#include <complex>
 #include <cstring>
 
 namespace qgpu {
 
-void reg_tile_shape(int nbits, int Tmax, int& T, int& L, int& NR) {
+void reg_tile_shape(qgpu_prec prec, int nbits, int Tmax, int& T, int& L, int& NR) {
     T = std::max(kRtMinTile, std::min({nbits, Tmax, kRtMaxTile}));
     // Tiles of up to 2^11 amplitudes run 4 registers per thread (more warps,
     // fewer amplitudes each: few tiles, bound by latency), the full 2^12 tile
@@ -19,7 +20,7 @@ void reg_tile_shape(int nbits, int Tmax, int& T, int& L, int& NR) {
     // Runs of 2^L contiguous amplitudes (128 bytes, one line) leave 9 bits to
     // choose; L = 4 ran as fast (42.6 and 43.2 ms for 126 gates on 28 qubits)
     // with a few passes more. A tile keeps room for two targets.
-    L = T >= nbits ? T : std::min(3, T - 2);
+    L = T >= nbits ? T : std::min(prec == QGPU_C128 ? 3 : 4, T - 2);
 }
 
 namespace {
@@ -107,10 +108,12 @@ void take(std::vector<Waiting>& g, uint64_t S, size_t most, std::vector<Waiting>
 
 // One pass's program under construction.
 struct Builder {
+    bool f32, ordered;
     int T, NR, inwarp;
     std::vector<RtOp> ops;
     std::vector<RtLayoutTab> lays;
     std::vector<cd> coef;
+    std::vector<std::complex<float>> coef32;
     int at[16]; // slot -> tile bit
 
     int slot_of(int bit) const { return int(std::find(at, at + T, bit) - at); }
@@ -118,7 +121,8 @@ struct Builder {
     void table() {
         RtLayoutTab t;
         std::memset(&t, 0, sizeof(t));
-        for (int s = 0; s < T; ++s) t.img[s] = uint16_t(rt_swz(1u << at[s]));
+        for (int s = 0; s < T; ++s)
+            t.img[s] = uint16_t(f32 ? rt_swz32(1u << at[s]) : rt_swz(1u << at[s]));
         lays.push_back(t);
     }
 
@@ -149,35 +153,50 @@ struct Builder {
         int next[16], n = 0;
         bool used[16] = {false};
         std::fill(next, next + 16, -1);
-        // lane slots 0 and 1: the first 2-qubit gate's bits
-        if (pair[0] < 0) { // none: the bits of the fewest gates
-            std::vector<int> r = in;
-            std::stable_sort(r.begin(), r.end(), [&](int x, int y) { return use[x] < use[y]; });
-            pair[0] = r[0];
-            pair[1] = r[1];
-        }
-        next[NR] = pair[0];
-        next[NR + 1] = pair[1];
-        used[pair[0]] = used[pair[1]] = true;
-        // register slots: the most used of the others
         std::vector<int> rest;
-        for (int b : in)
-            if (!used[b]) rest.push_back(b);
-        std::stable_sort(rest.begin(), rest.end(), [&](int x, int y) { return use[x] > use[y]; });
+        if (f32) {
+            // register slots: the first 2-qubit gate's bits, then the most used
+            if (pair[0] >= 0) rest = {pair[1], pair[0]};
+            std::vector<int> r;
+            for (int b : in)
+                if (b != pair[0] && b != pair[1]) r.push_back(b);
+            std::stable_sort(r.begin(), r.end(), [&](int x, int y) { return use[x] > use[y]; });
+            rest.insert(rest.end(), r.begin(), r.end());
+        } else {
+            // lane slots 0 and 1: the first 2-qubit gate's bits
+            if (pair[0] < 0) { // none: the bits of the fewest gates
+                std::vector<int> r = in;
+                std::stable_sort(r.begin(), r.end(), [&](int x, int y) { return use[x] < use[y]; });
+                pair[0] = r[0];
+                pair[1] = r[1];
+            }
+            next[NR] = pair[0];
+            next[NR + 1] = pair[1];
+            used[pair[0]] = used[pair[1]] = true;
+            // register slots: the most used of the others
+            for (int b : in)
+                if (!used[b]) rest.push_back(b);
+            std::stable_sort(rest.begin(), rest.end(), [&](int x, int y) { return use[x] > use[y]; });
+        }
         for (int s = 0; s < NR; ++s) {
             next[s] = rest[size_t(n)];
             used[rest[size_t(n++)]] = true;
         }
-        // lane slot 2: a bit whose shared-memory column differs from lane
-        // slots 0 and 1 (element bits of one class modulo 3 share a column)
+        // the other lane slots: first bits whose shared-memory columns differ
+        // from those of the lane slots before them (element bits of one class
+        // modulo 3, in complex64 above bit 0, share a column)
         std::vector<int> lanes(rest.begin() + n, rest.end());
-        for (size_t x = 0; x < lanes.size(); ++x)
-            if (lanes[x] % 3 != pair[0] % 3 && lanes[x] % 3 != pair[1] % 3) {
-                std::swap(lanes[0], lanes[x]);
-                break;
-            }
+        auto cls = [&](int b) { return !f32 ? b % 3 : b == 0 ? 3 : (b - 1) % 3; };
+        uint32_t cols = f32 ? 0u : (1u << cls(pair[0])) | (1u << cls(pair[1]));
         for (size_t x = 0; x < lanes.size(); ++x) {
-            next[NR + 2 + int(x)] = lanes[x];
+            for (size_t y = x; y < lanes.size(); ++y)
+                if (!((cols >> cls(lanes[y])) & 1u)) {
+                    std::swap(lanes[x], lanes[y]);
+                    break;
+                }
+            cols |= 1u << cls(lanes[x]);
+            const int slot = NR + (f32 ? 0 : 2) + int(x);
+            next[slot] = lanes[x];
             used[lanes[x]] = true;
         }
         n = inwarp;
@@ -225,8 +244,39 @@ struct Builder {
         op(kRtPerm, 0, 0, c);
     }
 
+    // Complex64: brings g's bits into register slots, each for the bit there
+    // whose next use in the stretch (`when`) is the farthest.
+    void to_regs(const GateDesc& g, const std::function<int(int)>& when) {
+        int b[2] = {g.b0, g.op == 2 ? g.b1 : g.b0};
+        for (int x = 0; x < g.op; ++x) {
+            const int s = slot_of(b[x]);
+            if (s < NR) continue;
+            int victim = -1, far = -1;
+            for (int r = 0; r < NR; ++r) {
+                if (at[r] == b[0] || at[r] == b[1]) continue;
+                const int w = when(at[r]);
+                if (w > far) {
+                    far = w;
+                    victim = r;
+                }
+            }
+            op(kRtSwap, s - NR, victim);
+            std::swap(at[s], at[victim]);
+        }
+        if (g.op == 2 && ordered && slot_of(g.b1) > slot_of(g.b0)) {
+            const int lo = slot_of(g.b0), hi = slot_of(g.b1);
+            op(kRtTrade, lo, hi);
+            std::swap(at[lo], at[hi]);
+        }
+    }
+
     // The moves that gate g (bits local to the tile) needs now.
     int moves(const GateDesc& g) const {
+        if (f32) {
+            int m = slot_of(g.b0) < NR ? 0 : 1;
+            if (g.op == 2 && slot_of(g.b1) >= NR) ++m;
+            return m;
+        }
         if (g.op == 1) return slot_of(g.b0) < NR ? 0 : 3; // a shuffle of every register
         int m = 0;
         for (int b : {g.b0, g.b1}) {
@@ -238,10 +288,16 @@ struct Builder {
 
     // Applies g with its controls on tile bits (local) and on others.
     void gate(const GateDesc& g, const std::vector<std::pair<int, int>>& local,
-              const std::vector<std::pair<int, int>>& outside) {
+              const std::vector<std::pair<int, int>>& outside, const std::function<int(int)>& when) {
         RtOp o;
         std::memset(&o, 0, sizeof(o));
-        if (g.op == 2) {
+        if (f32) {
+            to_regs(g, when);
+            const int s0 = slot_of(g.b0), s1 = g.op == 2 ? slot_of(g.b1) : s0;
+            o.type = g.op == 2 ? kRtG2 : kRtG1R;
+            o.a = uint8_t(std::min(s0, s1));
+            o.b = uint8_t(std::max(s0, s1));
+        } else if (g.op == 2) {
             to_pair(g.b0, g.b1);
             o.type = kRtG2;
         } else {
@@ -249,7 +305,7 @@ struct Builder {
             o.type = s < NR ? kRtG1R : kRtG1L;
             o.a = uint8_t(s < NR ? s : s - NR);
         }
-        o.coef = uint32_t(coef.size());
+        o.coef = uint32_t(f32 ? coef32.size() / 2 : coef.size());
         o.ctrl = !local.empty() || !outside.empty();
         for (auto& c : local) {
             const int s = slot_of(c.first);
@@ -264,6 +320,17 @@ struct Builder {
             if (c.second) o.gval |= uint64_t(1) << c.first;
         }
         ops.push_back(o);
+        if (f32) { // row-major over the index bit a + 2 bit b
+            const int D = g.op == 1 ? 2 : 4;
+            const bool turn = g.op == 2 && o.a == slot_of(g.b0); // b0 is the low bit
+            auto at4 = [&](int k) { return turn ? (k & 1) << 1 | k >> 1 : k; };
+            for (int r = 0; r < D; ++r)
+                for (int c = 0; c < D; ++c) {
+                    const cd u = g.op == 1 ? g.A[r + 2 * c] : g.A[at4(r) + 4 * at4(c)];
+                    coef32.push_back({float(u.real()), float(u.imag())});
+                }
+            return;
+        }
         if (g.op == 1) {
             for (int r = 0; r < 2; ++r)
                 for (int c = 0; c < 2; ++c) coef.push_back(g.A[r + 2 * c]);
@@ -289,19 +356,20 @@ struct Builder {
 
 size_t reg_program_bytes(const std::vector<GateDesc>& gates) {
     size_t b = 0; // every gate at most in a pass of its own
-    for (const GateDesc& g : gates) b += kGateBytes[g.op] + 64;
+    for (const GateDesc& g : gates) b += kGateBytes[g.op] + 64 + kRtHeadBytes;
     return b;
 }
 
 void plan_reg_program(const std::vector<GateDesc>& gates, int nbits, int Tmax, RegProgram& P,
-                      const std::function<void(const RegPass&)>& planned) {
+                      const std::function<void(const RegPass&)>& planned, bool ordered) {
+    const bool f32 = P.prec == QGPU_C64;
     P.nbits = nbits;
     P.passes.clear();
     P.single.clear();
     P.blob.clear();
     P.blob.reserve(reg_program_bytes(gates));
     int T, L, NR;
-    reg_tile_shape(nbits, Tmax, T, L, NR);
+    reg_tile_shape(P.prec, nbits, Tmax, T, L, NR);
     const int nfree = T - L;
     const uint64_t low = (uint64_t(1) << L) - 1, every = (uint64_t(1) << std::max(nbits, T)) - 1;
     std::vector<Waiting> wait, pass, run;
@@ -321,7 +389,7 @@ void plan_reg_program(const std::vector<GateDesc>& gates, int nbits, int Tmax, R
     while (!wait.empty()) {
         const uint64_t S = choose_bits(wait, low, every, T);
         pass.clear();
-        take(wait, S, kRtBlobMax - 64, pass);
+        take(wait, S, (f32 ? kRt32BlobMax - kRtHeadBytes : kRtBlobMax) - 64, pass);
         if (pass.empty()) raise(QGPU_ERR_NOT_SUPPORTED, "qgpu_run_gates()", "tile too small");
         RegPass p;
         std::memset(&p, 0, sizeof(p));
@@ -363,6 +431,8 @@ void plan_reg_program(const std::vector<GateDesc>& gates, int nbits, int Tmax, R
             pass[k] = w;
         }
         Builder B;
+        B.f32 = f32;
+        B.ordered = ordered;
         B.T = T;
         B.NR = NR;
         B.inwarp = NR + 5;
@@ -401,7 +471,15 @@ void plan_reg_program(const std::vector<GateDesc>& gates, int nbits, int Tmax, R
                     if ((S >> c.first) & 1u) inside.push_back({local(c.first), c.second});
                     else outside.push_back(c);
                 }
-                B.gate(g, inside, outside);
+                const uint32_t id = run[pick].id;
+                B.gate(g, inside, outside, [&](int bit) { // gates until the bit is used next
+                    int n = 0;
+                    for (const Waiting& w : run) {
+                        if (w.id != id && ((w.t >> bit) & 1u)) return n;
+                        ++n;
+                    }
+                    return 1000;
+                });
                 run.erase(run.begin() + ptrdiff_t(pick));
             }
         }
@@ -409,14 +487,30 @@ void plan_reg_program(const std::vector<GateDesc>& gates, int nbits, int Tmax, R
         p.nops = uint32_t(B.ops.size());
         p.nlay = uint32_t(B.lays.size());
         p.blob = uint32_t(P.blob.size());
+        const size_t b_head = f32 ? kRtHeadBytes : 0;
         const size_t b_ops = (B.ops.size() * sizeof(RtOp) + 15) / 16 * 16;
         const size_t b_lay = B.lays.size() * sizeof(RtLayoutTab);
-        p.blob_bytes = uint32_t(b_ops + b_lay + B.coef.size() * sizeof(cd));
+        const size_t b_coef = f32 ? B.coef32.size() * 8 : B.coef.size() * sizeof(cd);
+        p.blob_bytes = uint32_t(b_head + b_ops + b_lay + b_coef);
         P.blob.resize(P.blob.size() + p.blob_bytes);
         unsigned char* d = P.blob.data() + p.blob;
+        if (f32) {
+            RtHead h;
+            std::memset(&h, 0, sizeof(h));
+            h.nops = p.nops;
+            h.nlay = p.nlay;
+            h.nvalid = p.nvalid;
+            h.T = p.T;
+            h.L = p.L;
+            h.NR = p.NR;
+            std::copy(p.hi, p.hi + 16, h.hi);
+            std::memcpy(d, &h, sizeof(h));
+            d += b_head;
+        }
         std::memcpy(d, B.ops.data(), B.ops.size() * sizeof(RtOp));
         std::memcpy(d + b_ops, B.lays.data(), b_lay);
-        std::memcpy(d + b_ops + b_lay, B.coef.data(), B.coef.size() * sizeof(cd));
+        if (f32) std::memcpy(d + b_ops + b_lay, B.coef32.data(), b_coef);
+        else std::memcpy(d + b_ops + b_lay, B.coef.data(), b_coef);
         P.passes.push_back(p);
         if (planned) planned(p);
     }

@@ -1,5 +1,6 @@
-// reg_tiles.hpp -- complex128 tile passes with the tile held in registers
-// (reg_tiles.cpp plans them on the host, kernels_regtile.cu runs them).
+// reg_tiles.hpp -- tile passes with the tile held in registers (reg_tiles.cpp
+// plans them on the host; kernels_regtile.cu runs the complex128 ones,
+// kernels_regtile32.cu the complex64 ones).
 #pragma once
 
 #include <cstdint>
@@ -14,16 +15,22 @@ namespace qgpu {
 // slot, and slots [0, NR) number a thread's 2^NR registers, [NR, NR + 5) its
 // lane, [NR + 5, T) its warp. A pass is a program of ops that every thread of
 // the CTA runs in lockstep:
-//   kRtG2      4 x 4 on the bits in lane slots 0 and 1 (amplitude index
-//              lane & 3), two FP64 matrix instructions per register
+//   kRtG2      4 x 4. Complex128: on the bits in lane slots 0 and 1 (amplitude
+//              index lane & 3), two FP64 matrix instructions per register.
+//              Complex64: on the bits in register slots a < b (index bit a
+//              plus 2 x bit b)
 //   kRtG1R a   2 x 2 on the bit in register slot a
-//   kRtG1L a   2 x 2 on the bit in lane slot a (its partner by a shuffle)
+//   kRtG1L a   2 x 2 on the bit in lane slot a (its partner by a shuffle;
+//              complex128 only)
 //   kRtSwap    lane slot a and register slot b trade their bits
 //   kRtPerm    lane slots permuted: slot i takes the bit of slot perm[i]
-//              (coef = perm[i] << 3 i)
+//              (coef = perm[i] << 3 i; complex128 only)
 //   kRtLayout  every bit to a new slot through shared memory: written in
 //              layout table coef, read back in table coef + 1
-enum : uint8_t { kRtG2 = 0, kRtG1R = 1, kRtG1L = 2, kRtSwap = 3, kRtPerm = 4, kRtLayout = 5 };
+//   kRtTrade   register slots a < b trade their bits (complex64 only)
+enum : uint8_t {
+    kRtG2 = 0, kRtG1R = 1, kRtG1L = 2, kRtSwap = 3, kRtPerm = 4, kRtLayout = 5, kRtTrade = 6
+};
 
 // Controls hold a gate to the amplitudes whose register, lane, warp and
 // out-of-tile index bits under the masks equal the values.
@@ -49,6 +56,9 @@ constexpr int kRtMinTile = 7;  // 4 registers per lane, one warp
 // it next to the largest tile and its offset table.
 constexpr size_t kRtSmemMax = 112 * 1024;
 constexpr size_t kRtBlobMax = 44 * 1024;
+// Complex64: 32 KB tiles, three CTAs per SM.
+constexpr size_t kRt32SmemMax = 75 * 1024;
+constexpr size_t kRt32BlobMax = 38 * 1024;
 
 struct RegPass {
     uint64_t ntiles;
@@ -61,7 +71,25 @@ struct RegPass {
     int single;                // index of its only gate in RegProgram::single, or -1
 };
 
+// What a complex64 pass's tables begin with (its RegPass, on the device).
+struct RtHead {
+    uint32_t nops, nlay, nvalid;
+    int32_t T, L, NR;
+    int32_t hi[16];
+};
+static_assert(sizeof(RtHead) % 8 == 0, "head size");
+constexpr size_t kRtHeadBytes = (sizeof(RtHead) + 15) / 16 * 16;
+
+// One register's pass in a complex64 launch: tiles [first_tile, next one's) of
+// the launch are its tiles.
+struct RtInst {
+    float2* psi;
+    const unsigned char* blob;
+    uint32_t first_tile, blob_bytes;
+};
+
 struct RegProgram {
+    qgpu_prec prec = QGPU_C128;
     int nbits = 0;
     std::vector<RegPass> passes;
     std::vector<GateDesc> single; // passes of one uncontrolled gate
@@ -70,14 +98,16 @@ struct RegProgram {
 
 // The tile shape for an nbits-qubit ket: T bits of which the L lowest state
 // bits always belong to the tile, and 2^NR registers per thread.
-void reg_tile_shape(int nbits, int Tmax, int& T, int& L, int& NR);
-// Cuts the gates into passes and compiles each into its program. Gates on
-// disjoint bits trade places (list scheduling); each bit's gates keep their
-// order, so the product is the same up to rounding.
+void reg_tile_shape(qgpu_prec prec, int nbits, int Tmax, int& T, int& L, int& NR);
+// Cuts the gates into passes and compiles each into its program (P.prec set
+// by the caller). Gates on disjoint bits trade places (list scheduling); each
+// bit's gates keep their order, so the product is the same up to rounding.
 // `planned`, when given, is called after each pass with its tables in P.blob,
-// so that the device can start while the host plans on.
+// so that the device can start while the host plans on. ordered (complex64):
+// every 2-qubit product adds its four terms in the order of the matrix columns.
 void plan_reg_program(const std::vector<GateDesc>& gates, int nbits, int Tmax, RegProgram& P,
-                      const std::function<void(const RegPass&)>& planned = nullptr);
+                      const std::function<void(const RegPass&)>& planned = nullptr,
+                      bool ordered = false);
 // An upper bound of the program's bytes.
 size_t reg_program_bytes(const std::vector<GateDesc>& gates);
 
@@ -90,17 +120,27 @@ struct FusedTiles {
     std::vector<std::pair<int64_t, RegProgram>> runs; // first >= 0: that step as it is
 };
 
-// Swizzled shared-memory position of tile element e (complex128).
+// Swizzled shared-memory position of tile element e: 16-byte columns of the
+// 128-byte rows XORed with the folded row number; a complex64 pair stays one
+// column.
 inline uint32_t rt_swz(uint32_t e) {
     uint32_t r = e >> 3, h = 0;
     for (int k = 0; k < 16; k += 3) h ^= r >> k;
     return e ^ (h & 7u);
 }
+inline uint32_t rt_swz32(uint32_t e) { return rt_swz(e >> 1) << 1 | (e & 1u); }
 
 // Launches pass p (its tables at device address `blob`) on the ket at data;
 // chained: the previous launch on the stream was the pass before it, so this
 // one may start early and wait for it on the device.
 void launch_reg_pass(qgpu_ctx* ctx, void* data, const RegPass& p, const unsigned char* blob,
                      bool chained);
+// One launch over the complex64 passes of ninst registers (dinsts: a device
+// table sorted by first_tile; null: the one register `one`), ntiles tiles in
+// all, every pass of T tile bits and NR register slots and tables of at most
+// blob_max bytes.
+void launch_reg_pass32(qgpu_ctx* ctx, const RtInst* dinsts, const RtInst& one, int ninst,
+                       uint32_t ntiles, int T, int L, int NR, uint32_t blob_max, cudaStream_t stream,
+                       bool chained);
 
 } // namespace qgpu

@@ -1,18 +1,15 @@
 // tile_gates.cpp -- the plain form of qgpu_run_gates on qubit kets as
-// cache-blocked tile passes (kernels_tile.cu).
+// cache-blocked tile passes (kernels_regtile.cu, kernels_regtile32.cu).
 //
 // qpp applies every gate of a circuit as its own pass over the state
 // (QEngine::visit_gate_step_, qengine.hpp:551-578 -> apply / applyCTRL). Here
 // consecutive 1- and 2-qubit gates (plain, fan, controlled with any number of
-// controls) are grouped into passes: a pass keeps the L lowest state bits and
-// up to T - L other bits in shared memory, and takes gates in circuit order
-// while the union of their target bits outside the low L stays within T - L
-// (controls may be anywhere). Each pass reads and writes the state once,
-// however many gates it holds, and applies each gate with the one-gate
-// kernels' arithmetic, so the result is the gate-by-gate result. That is the
-// complex64 form; complex128 kets take the register tiles of reg_tiles.cpp,
-// where gates on disjoint bits also trade places (each gate still its own
-// product): 1100 gates on 20 qubits in 29 passes instead of 88.
+// controls) are grouped into passes that read and write the state once,
+// however many gates they hold. Each gate stays its own product; gates on
+// disjoint bits trade places (reg_tiles.cpp), so the result is the gate-by-gate
+// result up to rounding. plan_gate_tiles is the same cut in circuit order, one
+// tile in shared memory per pass: the plan that the register programs replace,
+// kept as the reference for the planners' tests.
 #include "tile_gates.hpp"
 
 #include <algorithm>
@@ -300,65 +297,8 @@ void plan_gate_tiles(const std::vector<GateDesc>& gates, int nbits, int Tmax,
     }
 }
 
-int tile_bits_max(const qgpu_ctx* ctx, qgpu_prec prec) {
-    // complex128: 64 KB tiles held in registers (two CTAs per SM);
-    // complex64: 128 KB tiles in shared memory (one)
-    const int cap = prec == QGPU_C128 ? kRtMaxTile : 14;
-    if (ctx->tile_bits > 0) return std::min(ctx->tile_bits, cap);
-    return cap;
-}
-
-void plan_tile_program(const std::vector<GateDesc>& gates, int nbits, int Tmax, TileProgram& P) {
-    P.nbits = nbits;
-    P.Tmax = Tmax;
-    P.gates = gates;
-    plan_gate_tiles(gates, nbits, Tmax, P.passes, P.dev, P.sweeps, P.mats);
-}
-
-void run_tile_program(qgpu_state* s, const TileProgram& P) {
-    if (P.gates.empty()) return;
-    if (P.nbits != int(s->dims.size()) || s->prec != QGPU_C64)
-        raise(QGPU_ERR_DIMS_MISMATCH_CVECTOR, "qgpu_run_gates()", "tile program / state");
-    const int nbits = P.nbits;
-    const auto& passes = P.passes;
-    const auto& dev = P.dev;
-    const auto& sweeps = P.sweeps;
-    const auto& mats = P.mats;
-    // a pass of one uncontrolled gate runs on the one-gate kernels
-    bool any_tiled = false;
-    for (const auto& p : passes)
-        if (p.ngates > 1 || dev[p.first].lmask || dev[p.first].gmask) any_tiled = true;
-    unsigned char* buf = nullptr;
-    const size_t b_gates = (dev.size() * sizeof(TileGate) + 255) / 256 * 256;
-    const size_t b_sweeps = (sweeps.size() * sizeof(TileSweep) + 255) / 256 * 256;
-    const size_t o_mats = b_gates + b_sweeps;
-    if (any_tiled) {
-        QG_CUDA(ctx_malloc(s->ctx, reinterpret_cast<void**>(&buf), o_mats + mats.size() * 8));
-        QG_CUDA(cudaMemcpyAsync(buf, dev.data(), dev.size() * sizeof(TileGate),
-                                cudaMemcpyHostToDevice, s->ctx->stream));
-        QG_CUDA(cudaMemcpyAsync(buf + b_gates, sweeps.data(), sweeps.size() * sizeof(TileSweep),
-                                cudaMemcpyHostToDevice, s->ctx->stream));
-        std::vector<float> mf(2 * mats.size());
-        for (size_t k = 0; k < mats.size(); ++k) {
-            mf[2 * k] = float(mats[k].real());
-            mf[2 * k + 1] = float(mats[k].imag());
-        }
-        QG_CUDA(cudaMemcpyAsync(buf + o_mats, mf.data(), mf.size() * sizeof(float),
-                                cudaMemcpyHostToDevice, s->ctx->stream));
-    }
-    size_t gi = 0;
-    for (const auto& p : passes) {
-        const GateDesc& g0 = P.gates[gi];
-        if (p.ngates == 1 && g0.ctrl.empty()) {
-            if (g0.op == 1) launch_qubit_1q(s->ctx, s->prec, s->data, nbits, g0.b0, g0.A);
-            else launch_qubit_2q(s->ctx, s->prec, s->data, nbits, g0.b0, g0.b1, g0.A);
-        } else {
-            launch_tile_pass(s->ctx, s->data, p, reinterpret_cast<TileGate*>(buf),
-                             reinterpret_cast<TileSweep*>(buf + b_gates), buf + o_mats);
-        }
-        gi += p.ngates;
-    }
-    if (buf) QG_CUDA(cudaFreeAsync(buf, s->ctx->stream));
+int tile_bits_max(const qgpu_ctx* ctx) {
+    return ctx->tile_bits > 0 ? std::min(ctx->tile_bits, kRtMaxTile) : kRtMaxTile;
 }
 
 static void launch_reg(qgpu_state* s, const RegProgram& P, const RegPass& p,
@@ -370,7 +310,13 @@ static void launch_reg(qgpu_state* s, const RegProgram& P, const RegPass& p,
         chained = false;
         return;
     }
-    launch_reg_pass(s->ctx, s->data, p, buf + p.blob, chained);
+    if (s->prec == QGPU_C128) {
+        launch_reg_pass(s->ctx, s->data, p, buf + p.blob, chained);
+    } else {
+        const RtInst one{static_cast<float2*>(s->data), buf + p.blob, 0, p.blob_bytes};
+        launch_reg_pass32(s->ctx, nullptr, one, 1, uint32_t(p.ntiles), p.T, p.L, p.NR, p.blob_bytes,
+                          s->ctx->stream, chained);
+    }
     chained = true;
 }
 
@@ -387,7 +333,7 @@ struct StreamBuf {
 
 void run_reg_program(qgpu_state* s, const RegProgram& P) {
     if (P.passes.empty()) return;
-    if (P.nbits != int(s->dims.size()) || s->prec != QGPU_C128)
+    if (P.nbits != int(s->dims.size()) || s->prec != P.prec)
         raise(QGPU_ERR_DIMS_MISMATCH_CVECTOR, "qgpu_run_gates()", "tile program / state");
     StreamBuf buf(s->ctx, P.blob.size());
     QG_CUDA(cudaMemcpyAsync(buf.p, P.blob.data(), P.blob.size(), cudaMemcpyHostToDevice,
@@ -398,6 +344,7 @@ void run_reg_program(qgpu_state* s, const RegProgram& P) {
 
 void plan_and_run_reg(qgpu_state* s, const std::vector<GateDesc>& gates, int Tmax, RegProgram& P) {
     if (gates.empty()) return;
+    P.prec = s->prec;
     StreamBuf buf(s->ctx, reg_program_bytes(gates));
     plan_reg_program(gates, int(s->dims.size()), Tmax, P, [&](const RegPass& p) {
         // the copy between the passes orders them, so none is chained
@@ -411,15 +358,9 @@ void plan_and_run_reg(qgpu_state* s, const std::vector<GateDesc>& gates, int Tma
 
 void run_tiled_gates(qgpu_state* s, const std::vector<GateDesc>& gates) {
     if (gates.empty()) return;
-    const int nbits = int(s->dims.size()), Tmax = tile_bits_max(s->ctx, s->prec);
-    if (s->prec == QGPU_C128) {
-        RegProgram P;
-        plan_and_run_reg(s, gates, Tmax, P);
-        return;
-    }
-    TileProgram P;
-    plan_tile_program(gates, nbits, Tmax, P);
-    run_tile_program(s, P);
+    const int Tmax = tile_bits_max(s->ctx);
+    RegProgram P;
+    plan_and_run_reg(s, gates, Tmax, P);
 }
 
 } // namespace qgpu

@@ -1,5 +1,5 @@
 // tile_gates.hpp -- planning and execution of gate runs as tile passes
-// (tile_gates.cpp, kernels_tile.cu).
+// (tile_gates.cpp, reg_tiles.cpp).
 #pragma once
 
 #include <complex>
@@ -41,23 +41,11 @@ void plan_gate_tiles(const std::vector<GateDesc>& gates, int nbits, int Tmax,
 // every ready gate whose targets fit the tile, those that extend the current
 // sweep first. For forms that do not promise the gate-by-gate arithmetic.
 std::vector<GateDesc> schedule_gates(const std::vector<GateDesc>& gates, int nbits, int Tmax);
-// Largest tile (bits) for this context and precision: 13 for complex128 and
-// 14 for complex64 (128 KB of shared memory), or qgpu_ctx_set_tile_bits's.
-int tile_bits_max(const qgpu_ctx* ctx, qgpu_prec prec);
-// A run of gates planned as tile passes on an nbits-qubit ket (host side;
-// uploaded by run_tile_program each time it runs).
-struct TileProgram {
-    int nbits = 0, Tmax = 0;
-    std::vector<GateDesc> gates; // in pass order
-    std::vector<TilePassParams> passes;
-    std::vector<TileGate> dev;
-    std::vector<TileSweep> sweeps;
-    std::vector<cd> mats;
-};
-void plan_tile_program(const std::vector<GateDesc>& gates, int nbits, int Tmax, TileProgram& P);
-// Uploads P's tables and launches its passes on s (stream order): complex64
-// tiles in shared memory, complex128 tiles in registers (reg_tiles.hpp).
-void run_tile_program(qgpu_state* s, const TileProgram& P);
+// Largest tile (bits) for this context: kRtMaxTile, or qgpu_ctx_set_tile_bits's
+// where that is less.
+int tile_bits_max(const qgpu_ctx* ctx);
+// Uploads P's tables and launches its passes on s (stream order; the tile in
+// registers, reg_tiles.hpp).
 struct RegProgram;
 void run_reg_program(qgpu_state* s, const RegProgram& P);
 // Plans the gates into P, each pass launched as soon as it is planned.

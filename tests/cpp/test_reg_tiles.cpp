@@ -1,10 +1,11 @@
-// CPU check of the complex128 register tile passes (qgpu::plan_reg_program): a host model of k_reg_tile -- the tile spread over
+// CPU check of the register tile passes (qgpu::plan_reg_program): a host model
+// of k_reg_tile and k_reg_tile32 -- the tile spread over
 // registers, lanes and warps, the shuffles, the layout changes through shared
 // memory and the matrix fragments of the 2-qubit gates -- runs the planned
 // programs of random 1- and 2-qubit gates with 0-3 controls on kets of 1-15
 // qubits and must give the gates applied one by one (in circuit order) within
 // 1e-13 (relative, max-norm: 60 gates of unit-norm rows, each at most a few
-// ulp). Every pass must touch each amplitude once, keep its shared memory
+// ulp) in complex128, 3e-5 with complex64 coefficients. Every pass must touch each amplitude once, keep its shared memory
 // inside the kernel's limit and hold only positions inside its tile. Built and
 // run by tests/test_reg_tiles.py.
 #include <algorithm>
@@ -48,15 +49,35 @@ static void apply_direct(std::vector<C>& psi, const GateDesc& g) {
     }
 }
 
-// host model of k_reg_tile on one pass
+// host model of k_reg_tile (f32: of k_reg_tile32, in double arithmetic) on one
+// pass
 static void run_pass(std::vector<C>& psi, const RegPass& p, const unsigned char* blob,
-                     std::vector<int>& visits) {
+                     std::vector<int>& visits, bool f32) {
+    const unsigned char* const end = blob + p.blob_bytes;
+    if (f32) {
+        const auto* h = reinterpret_cast<const RtHead*>(blob);
+        EXPECT(h->nops == p.nops && h->nlay == p.nlay && h->nvalid == p.nvalid && h->T == p.T &&
+               h->L == p.L && h->NR == p.NR && std::equal(p.hi, p.hi + 16, h->hi));
+        blob += kRtHeadBytes;
+    }
+    auto swz = [&](uint32_t e) { return f32 ? rt_swz32(e) : rt_swz(e); };
     const int T = p.T, NR = p.NR, R = 1 << NR, W = 1 << (T - NR - 5), nth = 32 * W, nhi = T - p.L;
     const auto* ops = reinterpret_cast<const RtOp*>(blob);
     const auto* lays = reinterpret_cast<const RtLayoutTab*>(blob + (p.nops * sizeof(RtOp) + 15) / 16 * 16);
-    const auto* coef = reinterpret_cast<const C*>(lays + p.nlay);
-    const C* coef_end = reinterpret_cast<const C*>(blob + p.blob_bytes);
-    EXPECT((size_t(16) << T) + ((size_t(8) << nhi) + 15) / 16 * 16 + p.blob_bytes <= kRtSmemMax);
+    // entry k of the coefficients from 16-byte unit u on
+    const auto* tables = reinterpret_cast<const unsigned char*>(lays + p.nlay);
+    auto entry = [&](uint32_t u, int k) -> C {
+        if (f32) {
+            const auto* x = reinterpret_cast<const std::complex<float>*>(tables) + 2 * u + k;
+            EXPECT(reinterpret_cast<const unsigned char*>(x + 1) <= end);
+            return C(x->real(), x->imag());
+        }
+        const C* x = reinterpret_cast<const C*>(tables) + u + k;
+        EXPECT(reinterpret_cast<const unsigned char*>(x + 1) <= end);
+        return *x;
+    };
+    EXPECT((size_t(f32 ? 8 : 16) << T) + ((size_t(8) << nhi) + 15) / 16 * 16 + p.blob_bytes <=
+           (f32 ? kRt32SmemMax : kRtSmemMax));
     const uint32_t nel = 1u << T;
     std::vector<C> tile(nel), v(size_t(nth) * R), w;
     auto at = [&](int lay, int th, int j) {
@@ -94,42 +115,49 @@ static void run_pass(std::vector<C>& psi, const RegPass& p, const unsigned char*
             return a;
         };
         for (uint32_t e = 0; e < nel; ++e) {
-            tile[rt_swz(e)] = 0;
+            tile[swz(e)] = 0;
             if (e >= p.nvalid) continue;
             EXPECT(addr(e) < psi.size());
-            tile[rt_swz(e)] = psi[addr(e)];
+            tile[swz(e)] = psi[addr(e)];
             ++visits[addr(e)];
         }
         get(0);
         for (uint32_t o = 0; o < p.nops; ++o) {
             const RtOp& op = ops[o];
             if (op.type <= kRtG1L) {
-                EXPECT(coef + op.coef + (op.type == kRtG2 ? 32 : 4) <= coef_end);
                 w = v;
                 for (int th = 0; th < nth; ++th) {
                     const int lane = th & 31, warp = th >> 5;
                     for (int j = 0; j < R; ++j) {
-                        const C* m = coef + op.coef;
                         C r = 0;
-                        if (op.type == kRtG2) {
+                        if (op.type == kRtG2 && f32) {
+                            EXPECT(op.a < op.b && op.b < NR);
+                            const int k = (j >> op.a & 1) | (j >> op.b & 1) << 1;
+                            for (int c = 0; c < 4; ++c) {
+                                const int jc = (j & ~(1 << op.a) & ~(1 << op.b)) | (c & 1) << op.a | (c >> 1) << op.b;
+                                r += entry(op.coef, 4 * k + c) * w[size_t(th) * R + jc];
+                            }
+                        } else if (op.type == kRtG2) {
                             // row lane >> 2 of the 8 x 4 operand, column pair
                             // 2 (lane & 3) of the product
                             double d[2] = {0, 0};
                             for (int x = 0; x < 2; ++x)
                                 for (int k = 0; k < 4; ++k) {
                                     const C a = w[size_t((th & ~3) + k) * R + j];
-                                    const C b = m[4 * (2 * (lane & 3) + x) + k];
+                                    const C b = entry(op.coef, 4 * (2 * (lane & 3) + x) + k);
                                     d[x] += a.real() * b.real() + a.imag() * b.imag();
                                 }
                             r = C(d[0], d[1]);
                         } else if (op.type == kRtG1R) {
                             EXPECT(op.a < NR);
                             const int s = j >> op.a & 1, j0 = j & ~(1 << op.a);
-                            r = m[2 * s] * w[size_t(th) * R + j0] + m[2 * s + 1] * w[size_t(th) * R + (j0 | 1 << op.a)];
+                            r = entry(op.coef, 2 * s) * w[size_t(th) * R + j0] +
+                                entry(op.coef, 2 * s + 1) * w[size_t(th) * R + (j0 | 1 << op.a)];
                         } else {
-                            EXPECT(op.a < 5);
+                            EXPECT(op.a < 5 && !f32);
                             const int s = lane >> op.a & 1;
-                            r = m[3 * s] * w[size_t(th) * R + j] + m[1 + s] * w[size_t(th ^ (1 << op.a)) * R + j];
+                            r = entry(op.coef, 3 * s) * w[size_t(th) * R + j] +
+                                entry(op.coef, 1 + s) * w[size_t(th ^ (1 << op.a)) * R + j];
                         }
                         const bool ok = !op.ctrl || ((base & op.gmask) == op.gval && (warp & op.wmask) == op.wval &&
                                                      (lane & op.lmask) == op.lval && (j & op.rmask) == op.rval);
@@ -145,7 +173,17 @@ static void run_pass(std::vector<C>& psi, const RegPass& p, const unsigned char*
                         const int th2 = (th & ~(1 << op.a)) | y << op.a, j2 = (j & ~(1 << op.b)) | x << op.b;
                         v[size_t(th) * R + j] = w[size_t(th2) * R + j2];
                     }
+            } else if (op.type == kRtTrade) {
+                EXPECT(f32 && op.a < op.b && op.b < NR);
+                w = v;
+                for (int th = 0; th < nth; ++th)
+                    for (int j = 0; j < R; ++j) {
+                        const int x = j >> op.a & 1, y = j >> op.b & 1;
+                        const int j2 = (j & ~(1 << op.a) & ~(1 << op.b)) | y << op.a | x << op.b;
+                        v[size_t(th) * R + j] = w[size_t(th) * R + j2];
+                    }
             } else if (op.type == kRtPerm) {
+                EXPECT(!f32);
                 w = v;
                 for (int th = 0; th < nth; ++th) {
                     int src = th & ~31;
@@ -160,7 +198,7 @@ static void run_pass(std::vector<C>& psi, const RegPass& p, const unsigned char*
         }
         put(int(p.nlay) - 1);
         for (uint32_t e = 0; e < nel; ++e)
-            if (e < p.nvalid) psi[addr(e)] = tile[rt_swz(e)];
+            if (e < p.nvalid) psi[addr(e)] = tile[swz(e)];
     }
 }
 
@@ -193,26 +231,29 @@ int main() {
             for (auto& x : psi) x = C(nd(rng), nd(rng));
             std::vector<C> ref = psi;
             for (const auto& g : gates) apply_direct(ref, g);
-            RegProgram P;
-            plan_reg_program(gates, nbits, Tmax, P);
-            std::vector<C> got = psi;
-            uint32_t covered = 0;
-            for (const RegPass& p : P.passes) {
-                EXPECT(p.blob % 16 == 0 && p.blob + p.blob_bytes <= P.blob.size());
-                EXPECT(p.single < 0 || (p.ngates == 1 && P.single[size_t(p.single)].ctrl.empty()));
-                covered += p.ngates;
-                std::vector<int> visits(psi.size(), 0);
-                run_pass(got, p, P.blob.data() + p.blob, visits);
-                for (int x : visits) EXPECT(x == 1);
+            for (int form = 0; form < 3; ++form) { // complex128; complex64, also ordered
+                RegProgram P;
+                P.prec = form ? QGPU_C64 : QGPU_C128;
+                plan_reg_program(gates, nbits, Tmax, P, nullptr, form == 2);
+                std::vector<C> got = psi;
+                uint32_t covered = 0;
+                for (const RegPass& p : P.passes) {
+                    EXPECT(p.blob % 16 == 0 && p.blob + p.blob_bytes <= P.blob.size());
+                    EXPECT(p.single < 0 || (p.ngates == 1 && P.single[size_t(p.single)].ctrl.empty()));
+                    covered += p.ngates;
+                    std::vector<int> visits(psi.size(), 0);
+                    run_pass(got, p, P.blob.data() + p.blob, visits, form > 0);
+                    for (int x : visits) EXPECT(x == 1);
+                }
+                EXPECT(covered == gates.size());
+                double top = 0, err = 0;
+                for (size_t i = 0; i < ref.size(); ++i) {
+                    top = std::max(top, std::abs(ref[i]));
+                    err = std::max(err, std::abs(got[i] - ref[i]));
+                }
+                EXPECT(err <= (form ? 3e-5 : 1e-13) * top);
+                ++cases;
             }
-            EXPECT(covered == gates.size());
-            double top = 0, err = 0;
-            for (size_t i = 0; i < ref.size(); ++i) {
-                top = std::max(top, std::abs(ref[i]));
-                err = std::max(err, std::abs(got[i] - ref[i]));
-            }
-            EXPECT(err <= 1e-13 * top);
-            ++cases;
         }
     if (fails) {
         std::printf("%d failures\n", fails);
