@@ -7,15 +7,16 @@
 // by register size, and captures everything into a single CUDA graph, so the
 // whole batch is one graph launch. Registers of up to 2^14 amplitudes: one
 // CTA per instance with the register in shared memory, one trajectory-kernel
-// launch per size on its own graph branch. Larger registers whose programs
-// are all gates: cache-blocked tile passes at the tuned width, run
-// layer-synchronously on one more branch -- graph node k applies pass k of
-// every such register, all tiles in parallel, in place in the instances' own
-// states. Larger registers with measurements keep one CTA per instance.
-// Registers of at least 2^18 amplitudes whose programs are all dense gates
-// (kets of 18-22 qubits, density matrices of 9-15 qubits) run block-layered
-// on one more branch instead: every program fused into blocks of <= 4
-// (virtual) qubits, launch j applies block j of every such register. The
+// launch per size on its own graph branch. Larger kets, and density matrices
+// of 8 and 9 qubits, whose programs are 1- and 2-qubit gates run as register
+// tile passes (reg_tiles.hpp), layer-synchronously on one more branch: graph
+// node k applies pass k of every such register, all tiles in parallel, in place
+// in the instances' own states. Larger registers with measurements keep one CTA
+// per instance. Density matrices from 2^18 amplitudes otherwise run
+// block-layered on one more branch: every program fused into blocks of <= 4
+// (virtual) qubits, launch j applies block j of every such register; density
+// matrices of 2^16 amplitudes with wider gates take layered tile passes in
+// shared memory. The
 // plain form loops over the instances with one kernel launch per gate
 // (qgpu_run_gates, QGPU_FORM_PLAIN).
 #include <algorithm>
@@ -32,6 +33,7 @@
 #include "capi_common.hpp"
 #include "circuit.hpp"
 #include "ops.hpp"
+#include "reg_tiles.hpp"
 #include "traj.hpp"
 
 namespace qgpu {
@@ -39,6 +41,10 @@ namespace qgpu {
 // Register bits (kets: qubits; density matrices: twice the qubits) from which
 // batched instances run block-layered.
 constexpr int kBlockMinBits = 18;
+// Register bits from which programs of 1- and 2-qubit gates run as register
+// tile passes (every tile of the same shape), and up to which density matrices
+// do.
+constexpr int kRegMinBits = 15, kRegMaxRhoBits = 19;
 
 bool compile_traj_rho(const qgpu_circuit* c, TProgram& P, int max_nv) {
     const int nq = int(c->nq), nv = 2 * nq;
@@ -183,14 +189,6 @@ extern "C" qgpu_status qgpu_run_batch(qgpu_ctx* ctx, uint32_t n_inst, qgpu_circu
             for (auto& t : th) t.join();
             if (first) std::rethrow_exception(first);
         };
-        std::vector<qgpu::TProgram> progs(n_inst);
-        std::vector<char> ok(n_inst, 0);
-        pfor(n_inst, [&](size_t i) {
-            qgpu::TProgram& P = progs[i];
-            ok[i] = form == 1 && states[i]->prec == QGPU_C64 &&
-                    (states[i]->kind == QGPU_KET ? qgpu::compile_traj(circuits[i], P)
-                                                 : qgpu::compile_traj_rho(circuits[i], P));
-        });
         auto all_gates = [](const qgpu::TProgram& P) {
             for (const auto& I : P.ins)
                 if (I.op != qgpu::kTG1 && I.op != qgpu::kTCG1 && I.op != qgpu::kTG2 &&
@@ -198,6 +196,75 @@ extern "C" qgpu_status qgpu_run_batch(qgpu_ctx* ctx, uint32_t n_inst, qgpu_circu
                     return false;
             return true;
         };
+        // Register-tile registers (no reference counterpart): programs of 1- and
+        // 2-qubit gates and controlled 1-qubit gates, kets from 2^15 amplitudes
+        // and density matrices of 2^15 to 2^19. Gates merge into blocks of <= 2
+        // (virtual) qubits, each register's program is cut into register tile
+        // passes (reg_tiles.hpp), and launch k of one chain runs pass k of every
+        // such register. Against tile passes in shared memory with a barrier per
+        // gate (below 2^18) and blocks of 4 qubits with a trip through HBM each
+        // (from 2^18), depth 20: 40 kets of 18-19 qubits 6.1 -> 4.0 ms, 8 kets of
+        // 22 qubits 12.6 -> 9.9 ms, 20 density matrices of 8-9 qubits 7.1 ->
+        // 1.7 ms on the device. A density matrix of 10 qubits and more stays with the
+        // blocks: a layer's gates and channels on one pair of qubits are one
+        // 4-qubit superoperator there and four 2-qubit ones here (6 of 11
+        // qubits 9.9 and 14.2 ms). Below 2^15 the trajectory kernel keeps a
+        // register on one SM for its whole program. The programs are kept with
+        // their circuits: planning takes about a millisecond each.
+        auto reg_gates = [](const qgpu::TProgram& P) {
+            for (const auto& I : P.ins)
+                if (I.op != qgpu::kTG1 && I.op != qgpu::kTCG1 && I.op != qgpu::kTG2) return false;
+            return true;
+        };
+        std::vector<char> on_reg(n_inst, 0);
+        std::vector<std::shared_ptr<const qgpu::RegProgram>> rprog(n_inst);
+        std::vector<qgpu::TProgram> progs(n_inst);
+        std::vector<char> ok(n_inst, 0);
+        pfor(n_inst, [&](size_t i) {
+            qgpu_circuit* const c = circuits[i];
+            qgpu::TProgram& P = progs[i];
+            if (form != 1 || states[i]->prec != QGPU_C64) return;
+            const bool rho = states[i]->kind == QGPU_RHO;
+            const uint64_t bits = rho ? 2 * uint64_t(c->nq) : c->nq;
+            const bool want = c->d == 2 && states[i]->ctx == ctx && bits >= uint64_t(qgpu::kRegMinBits) &&
+                              bits <= uint64_t(rho ? qgpu::kRegMaxRhoBits : qgpu::kTrajMaxGlobalQubits);
+            if (want) {
+                std::lock_guard<std::mutex> lock(c->tiles_mu);
+                if (c->btiles[rho] && c->btile_steps[rho] == c->steps.size()) rprog[i] = c->btiles[rho];
+            }
+            if (!rprog[i]) {
+                ok[i] = rho ? qgpu::compile_traj_rho(c, P) : qgpu::compile_traj(c, P);
+                if (!ok[i] || !want || !reg_gates(P)) return;
+                qgpu::fuse_blocks(P, 2);
+                auto R = std::make_shared<qgpu::RegProgram>();
+                std::vector<qgpu::GateDesc> g;
+                g.reserve(P.ins.size());
+                for (const qgpu::TInstr& I : P.ins) {
+                    qgpu::GateDesc d;
+                    d.op = I.op == qgpu::kTG2 ? 2 : 1;
+                    d.b0 = I.b0;
+                    d.b1 = I.b1;
+                    if (I.op == qgpu::kTCG1)
+                        for (int b = 0; b < int(P.n); ++b)
+                            if ((I.cmask >> b) & 1u) d.ctrl.push_back({b, int((I.cval >> b) & 1u)});
+                    for (int x = 0; x < (d.op == 2 ? 16 : 4); ++x)
+                        d.A[x] = qgpu::cd(P.mats[2 * (I.mat + x)], P.mats[2 * (I.mat + x) + 1]);
+                    g.push_back(std::move(d));
+                }
+                R->prec = QGPU_C64;
+                qgpu::plan_reg_program(g, int(P.n), qgpu::kRtMaxTile, *R);
+                P = qgpu::TProgram{};
+                rprog[i] = R;
+                std::lock_guard<std::mutex> lock(c->tiles_mu);
+                c->btiles[rho] = rprog[i];
+                c->btile_steps[rho] = c->steps.size();
+            }
+            ok[i] = 0;
+            on_reg[i] = 1;
+        });
+        std::vector<uint32_t> regs;
+        for (uint32_t i = 0; i < n_inst; ++i)
+            if (on_reg[i]) regs.push_back(i);
         // Block-layered registers (no reference counterpart): density matrices
         // of at least kBlockMinBits virtual qubits (up to 15 qubits) and kets
         // of at least kBlockMinBits qubits whose programs are dense gates. Each
@@ -216,7 +283,7 @@ extern "C" qgpu_status qgpu_run_batch(qgpu_ctx* ctx, uint32_t n_inst, qgpu_circu
             std::map<qgpu_circuit*, uint32_t> first_of; // one build per circuit
             for (uint32_t i = 0; i < n_inst; ++i) {
                 const qgpu_state* s = states[i];
-                if (s->kind != QGPU_RHO || s->prec != QGPU_C64 || s->ctx != ctx ||
+                if (on_reg[i] || s->kind != QGPU_RHO || s->prec != QGPU_C64 || s->ctx != ctx ||
                     circuits[i]->d != 2 || 2 * circuits[i]->nq < uint32_t(qgpu::kBlockMinBits))
                     continue;
                 cand.push_back(i);
@@ -269,9 +336,9 @@ extern "C" qgpu_status qgpu_run_batch(qgpu_ctx* ctx, uint32_t n_inst, qgpu_circu
         });
         for (uint32_t i = 0; i < n_inst; ++i) {
             if (ok[i]) prog.emplace_back(i, std::move(progs[i]));
-            else if (!on_block[i]) plain.push_back(i);
+            else if (!on_block[i] && !on_reg[i]) plain.push_back(i);
         }
-        if (!prog.empty() || !blocked.empty()) {
+        if (!prog.empty() || !blocked.empty() || !regs.empty()) {
             // Registers above shared-memory size whose programs are all gates
             // run layer-synchronously: every gate belongs to a tile pass of
             // the tuned width, and launch k runs pass k of every such
@@ -397,6 +464,47 @@ extern "C" qgpu_status qgpu_run_batch(qgpu_ctx* ctx, uint32_t n_inst, qgpu_circu
                     blaunch.push_back({off, {int(binst.size() - off), items}});
                 }
             }
+            // register-tile registers: their programs one after the other, then
+            // launch k's table
+            std::vector<size_t> rbase;
+            size_t nrblob = 0, rkmax = 0;
+            for (uint32_t i : regs) {
+                rbase.push_back(nrblob);
+                nrblob += rprog[i]->blob.size(); // a multiple of 16
+                rkmax = std::max(rkmax, rprog[i]->passes.size());
+            }
+            std::unique_ptr<unsigned char[]> rblob(new unsigned char[std::max<size_t>(nrblob, 1)]);
+            pfor(regs.size(), [&](size_t k) {
+                const auto& B = rprog[regs[k]]->blob;
+                std::copy(B.begin(), B.end(), rblob.get() + rbase[k]);
+            });
+            struct RLaunch {
+                size_t off;
+                int count;
+                uint32_t tiles, blob_max;
+            };
+            std::vector<RLaunch> rlaunch;
+            std::vector<qgpu::RtInst> rinst; // blob: offset for now
+            for (size_t kk = 0; kk < rkmax; ++kk) {
+                RLaunch R{rinst.size(), 0, 0, 0};
+                for (size_t k = 0; k < regs.size(); ++k) {
+                    const qgpu::RegProgram& P = *rprog[regs[k]];
+                    if (kk >= P.passes.size()) continue;
+                    const qgpu::RegPass& ps = P.passes[kk];
+                    qgpu::RtInst q{};
+                    q.psi = static_cast<float2*>(states[regs[k]]->data);
+                    if (reinterpret_cast<uintptr_t>(q.psi) % 16)
+                        raise(QGPU_ERR_INVALID_ARGUMENT, W, "state not 16-byte aligned");
+                    q.blob = reinterpret_cast<const unsigned char*>(rbase[k] + ps.blob);
+                    q.blob_bytes = ps.blob_bytes;
+                    q.first_tile = R.tiles;
+                    R.tiles += uint32_t(ps.ntiles);
+                    R.blob_max = std::max(R.blob_max, ps.blob_bytes);
+                    ++R.count;
+                    rinst.push_back(q);
+                }
+                rlaunch.push_back(R);
+            }
             auto al = [](size_t x) { return (x + 255) / 256 * 256; };
             size_t npass_total = 0;
             for (auto& v : passes) npass_total += v.size();
@@ -409,8 +517,10 @@ extern "C" qgpu_status qgpu_run_batch(qgpu_ctx* ctx, uint32_t n_inst, qgpu_circu
             size_t b_dits = std::max<size_t>(prog.size() * sizeof(uint32_t) * 8, 16);
             size_t b_bmat = std::max<size_t>(nbfloat * sizeof(float), 16);
             size_t b_binst = std::max<size_t>(binst.size() * sizeof(qgpu::BlockInst), 16);
+            size_t b_rblob = std::max<size_t>(nrblob, 16);
+            size_t b_rinst = std::max<size_t>(rinst.size() * sizeof(qgpu::RtInst), 16);
             size_t total = al(b_ins) + al(b_mat) + al(b_work) + al(b_pass) + al(b_samp) +
-                           al(b_dits) + al(b_bmat) + al(b_binst);
+                           al(b_dits) + al(b_bmat) + al(b_binst) + al(b_rblob) + al(b_rinst);
             unsigned char* buf = nullptr;
             QG_CUDA(qgpu::ctx_malloc(ctx, reinterpret_cast<void**>(&buf), total));
             unsigned char* p = buf;
@@ -428,6 +538,9 @@ extern "C" qgpu_status qgpu_run_batch(qgpu_ctx* ctx, uint32_t n_inst, qgpu_circu
             auto* ddits = reinterpret_cast<uint32_t*>(take(b_dits));
             auto* dbmat = reinterpret_cast<float2*>(take(b_bmat));
             auto* dbinst = reinterpret_cast<qgpu::BlockInst*>(take(b_binst));
+            unsigned char* const drblob = take(b_rblob);
+            auto* drinst = reinterpret_cast<qgpu::RtInst*>(take(b_rinst));
+            for (qgpu::RtInst& q : rinst) q.blob = drblob + reinterpret_cast<size_t>(q.blob);
             for (size_t k = 0; k < binst.size(); ++k) binst[k].m = dbmat + bmoff[k];
             std::vector<qgpu::TWork> work;
             std::vector<std::pair<uint32_t, std::pair<size_t, size_t>>> ranges; // n -> [lo, hi)
@@ -500,6 +613,12 @@ extern "C" qgpu_status qgpu_run_batch(qgpu_ctx* ctx, uint32_t n_inst, qgpu_circu
                 QG_CUDA(cudaMemcpyAsync(dbinst, binst.data(), binst.size() * sizeof(qgpu::BlockInst),
                                         cudaMemcpyHostToDevice, ctx->stream));
             }
+            if (!rinst.empty()) {
+                QG_CUDA(cudaMemcpyAsync(drblob, rblob.get(), nrblob, cudaMemcpyHostToDevice,
+                                        ctx->stream));
+                QG_CUDA(cudaMemcpyAsync(drinst, rinst.data(), rinst.size() * sizeof(qgpu::RtInst),
+                                        cudaMemcpyHostToDevice, ctx->stream));
+            }
             int* dflag = launches.empty() ? nullptr : qgpu::ctx_error_flag(ctx);
             // one graph: a k_traj launch per register size on its own branch,
             // and the chain of layer launches on one more branch (all touch
@@ -507,7 +626,8 @@ extern "C" qgpu_status qgpu_run_batch(qgpu_ctx* ctx, uint32_t n_inst, qgpu_circu
             qgpu::traj_prepare();
             cudaGraph_t graph = nullptr;
             cudaGraphExec_t exec = nullptr;
-            const size_t nbr = ranges.size() + (launches.empty() ? 0 : 1) + (blaunch.empty() ? 0 : 1);
+            const size_t nbr = ranges.size() + (launches.empty() ? 0 : 1) + (blaunch.empty() ? 0 : 1) +
+                               (rlaunch.empty() ? 0 : 1);
             std::vector<cudaStream_t> side(nbr, nullptr);
             std::vector<cudaEvent_t> ev(nbr + 1, nullptr);
             struct Rel {
@@ -526,6 +646,17 @@ extern "C" qgpu_status qgpu_run_batch(qgpu_ctx* ctx, uint32_t n_inst, qgpu_circu
             try {
                 QG_CUDA(cudaEventRecord(ev[0], ctx->stream));
                 size_t g = 0;
+                if (!rlaunch.empty()) {
+                    QG_CUDA(cudaStreamWaitEvent(side[g], ev[0], 0));
+                    int T, L, NR; // one shape: every register is larger than the tile
+                    qgpu::reg_tile_shape(QGPU_C64, qgpu::kRegMinBits, qgpu::kRtMaxTile, T, L, NR);
+                    for (const RLaunch& R : rlaunch)
+                        qgpu::launch_reg_pass32(ctx, drinst + R.off, qgpu::RtInst{}, R.count, R.tiles, T,
+                                                L, NR, R.blob_max, side[g], false);
+                    QG_CUDA(cudaEventRecord(ev[g + 1], side[g]));
+                    QG_CUDA(cudaStreamWaitEvent(ctx->stream, ev[g + 1], 0));
+                    ++g;
+                }
                 if (!launches.empty()) { // longest chain first
                     QG_CUDA(cudaStreamWaitEvent(side[g], ev[0], 0));
                     for (auto& L : launches)
@@ -589,7 +720,7 @@ extern "C" qgpu_status qgpu_run_batch(qgpu_ctx* ctx, uint32_t n_inst, qgpu_circu
             if (dflag && qgpu::fused_error(ctx))
                 raise(QGPU_ERR_TIMEOUT, W, "a bounded wait of a batch kernel gave up");
             ctx->batch_ms[5] = ms_since(t_tear);
-            if (graph_kernels) *graph_kernels = ranges.size() + launches.size() + blaunch.size();
+            if (graph_kernels) *graph_kernels = ranges.size() + launches.size() + blaunch.size() + rlaunch.size();
         }
         auto t_plain = clk::now();
         for (uint32_t i : plain) qgpu::run_gates(states[i], circuits[i], 0, 0, circuits[i]->steps.size());

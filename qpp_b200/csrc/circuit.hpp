@@ -27,6 +27,7 @@ namespace qgpu {
 using cd = std::complex<double>;
 struct TProgram;
 struct FusedTiles;
+struct RegProgram;
 
 enum class StepKind {
     Gate,      // apply(U, target)           GType SINGLE/TWO/THREE/JOINT
@@ -93,9 +94,13 @@ struct qgpu_circuit {
     // planned for the first ftiles->nsteps steps
     std::shared_ptr<const qgpu::FusedTiles> ftiles;
     // the same of the plain form (the gates as they are) in complex128 and
-    // complex64; tiles_mu guards all three
+    // complex64
     std::shared_ptr<const qgpu::FusedTiles> ptiles[2];
-    std::mutex tiles_mu;
+    // batched complex64 register programs (blocks of <= 2 (virtual) qubits) of
+    // a ket and of a density matrix, for the first btile_steps steps
+    std::shared_ptr<const qgpu::RegProgram> btiles[2];
+    uint64_t btile_steps[2] = {0, 0};
+    std::mutex tiles_mu; // guards the tile plans
     // fused density-matrix form on the tensor cores (complex64, 2n >= 13
     // virtual qubits): superoperator blocks of <= 6 virtual qubits, built for
     // the first rho_tc_steps steps

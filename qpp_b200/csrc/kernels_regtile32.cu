@@ -14,7 +14,10 @@
 // Measured on one B200 against tiles kept in shared memory (a trip through it
 // for every three bits): 330 gates gate by gate on 14 / 17 / 20 / 22 qubits
 // 0.81 / 0.94 / 1.04 / 2.21 -> 0.21 / 0.22 / 0.48 / 1.47 ms, three layers on 24
-// and 27 qubits 3.14 and 24.1 -> 1.68 and 14.4 ms.
+// and 27 qubits 3.14 and 24.1 -> 1.68 and 14.4 ms. Per pass over 2^20
+// amplitudes of 2^26: 3.5 us in and out, 0.67 us per 2-qubit gate (0.46 at the
+// FP32 peak), 0.38 us per 1-qubit gate, 0.4 us per swap. Swaps pick with a logic
+// operation: as selects on a predicate one took 0.68 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -26,7 +29,9 @@
 
 namespace qgpu {
 
-template <int NR, int NTMAX, int MINB>
+// Tiles of one register (MANY = false: `one`; a pass of a chain, which may start
+// early and waits for the pass before it) or of many (insts).
+template <int NR, int NTMAX, int MINB, bool MANY>
 __global__ void __launch_bounds__(NTMAX, MINB)
     k_reg_tile32(const RtInst* __restrict__ insts, const __grid_constant__ RtInst one, int ninst,
                  uint32_t ntiles, int T, int L) {
@@ -37,12 +42,12 @@ __global__ void __launch_bounds__(NTMAX, MINB)
     unsigned char* const prog = reinterpret_cast<unsigned char*>(hioff) +
                                 ((sizeof(uint64_t) << nhi) + 15) / 16 * 16;
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if constexpr (!MANY) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // a contiguous range of tiles, so that a CTA changes registers rarely
     const uint32_t t0 = uint32_t(uint64_t(ntiles) * blockIdx.x / gridDim.x);
     const uint32_t t1 = uint32_t(uint64_t(ntiles) * (blockIdx.x + 1) / gridDim.x);
     int ri = 0;
-    if (insts) {
+    if constexpr (MANY) {
         int hi = ninst - 1; // last register with first_tile <= t0
         while (ri < hi) {
             const int mid = (ri + hi + 1) >> 1;
@@ -53,10 +58,15 @@ __global__ void __launch_bounds__(NTMAX, MINB)
     int have = -1;
     const RtHead* const head = reinterpret_cast<const RtHead*>(prog);
     const RtOp* const ops = reinterpret_cast<const RtOp*>(prog + kRtHeadBytes);
-    bool waited = false;
+    [[maybe_unused]] bool waited = false;
     for (uint32_t t = t0; t < t1; ++t) {
-        while (ri + 1 < ninst && insts[ri + 1].first_tile <= t) ++ri;
-        const RtInst I = insts ? insts[ri] : one;
+        RtInst I;
+        if constexpr (MANY) {
+            while (ri + 1 < ninst && insts[ri + 1].first_tile <= t) ++ri;
+            I = insts[ri];
+        } else {
+            I = one;
+        }
         if (have != ri) { // the register's tables (uniform over the CTA)
             have = ri;
             for (uint32_t i = tid * 16; i < I.blob_bytes; i += nt * 16) {
@@ -75,9 +85,11 @@ __global__ void __launch_bounds__(NTMAX, MINB)
             }
             __syncthreads();
         }
-        if (!waited) { // the pass before this one has finished
-            asm volatile("griddepcontrol.wait;" ::: "memory");
-            waited = true;
+        if constexpr (!MANY) {
+            if (!waited) { // the pass before this one has finished
+                asm volatile("griddepcontrol.wait;" ::: "memory");
+                waited = true;
+            }
         }
         uint64_t base = uint64_t(t - I.first_tile) << L;
         for (int i = 0; i < nhi; ++i) {
@@ -107,7 +119,7 @@ __global__ void __launch_bounds__(NTMAX, MINB)
         const float4* const coef = reinterpret_cast<const float4*>(lays + head->nlay);
         rt32_load<NR>(v, tile, lays[0], T, lane, warp);
         for (uint32_t o = 0; o < nops; ++o)
-            rt32_op<NR>(v, ops[o], lays, coef, tile, T, lane, warp, base);
+            rt32_op<NR, false>(v, ops[o], lays, coef, tile, T, lane, warp, base);
         __syncwarp();
         rt32_store<NR>(v, tile, lays[head->nlay - 1], T, lane, warp);
         __syncthreads();
@@ -149,12 +161,13 @@ void launch_reg_pass32(qgpu_ctx* ctx, const RtInst* dinsts, const RtInst& one, i
                        bool chained) {
     if (ninst <= 0 || ntiles == 0) return;
     blob_max = (blob_max + 15) / 16 * 16;
-    if (NR == 4)
-        launch_one32(k_reg_tile32<4, 256, 3>, ctx, dinsts, one, ninst, ntiles, T, L, NR, blob_max,
-                     stream, chained, 3);
-    else
-        launch_one32(k_reg_tile32<2, 512, 2>, ctx, dinsts, one, ninst, ntiles, T, L, NR, blob_max,
-                     stream, chained, 2);
+    auto go = [&](auto kernel, int per_sm) {
+        launch_one32(kernel, ctx, dinsts, one, ninst, ntiles, T, L, NR, blob_max, stream, chained, per_sm);
+    };
+    if (dinsts && NR == 4) go(k_reg_tile32<4, 256, 3, true>, 3);
+    else if (dinsts) go(k_reg_tile32<2, 512, 2, true>, 2);
+    else if (NR == 4) go(k_reg_tile32<4, 256, 3, false>, 3);
+    else go(k_reg_tile32<2, 512, 2, false>, 2);
 }
 
 } // namespace qgpu

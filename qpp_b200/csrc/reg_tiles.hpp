@@ -138,7 +138,7 @@ void launch_reg_pass(qgpu_ctx* ctx, void* data, const RegPass& p, const unsigned
 // One launch over the complex64 passes of ninst registers (dinsts: a device
 // table sorted by first_tile; null: the one register `one`), ntiles tiles in
 // all, every pass of T tile bits and NR register slots and tables of at most
-// blob_max bytes.
+// blob_max bytes. chained (dinsts null): as launch_reg_pass.
 void launch_reg_pass32(qgpu_ctx* ctx, const RtInst* dinsts, const RtInst& one, int ninst,
                        uint32_t ntiles, int T, int L, int NR, uint32_t blob_max, cudaStream_t stream,
                        bool chained);

@@ -148,23 +148,24 @@ __device__ __forceinline__ void rt32_g1(float2 (&v)[1 << NR], const float4* m, b
     }
 }
 
+// Bits of a where m is set, of b elsewhere (one three-input logic operation).
+__device__ __forceinline__ float rt32_sel(uint32_t m, float a, float b) {
+    return __uint_as_float((__float_as_uint(a) & m) | (__float_as_uint(b) & ~m));
+}
+
+// up: all ones in lanes whose bit is set
 template <int NR, int B>
-__device__ __forceinline__ void rt32_swap(float2 (&v)[1 << NR], bool up, int xm) {
+__device__ __forceinline__ void rt32_swap(float2 (&v)[1 << NR], uint32_t up, int xm) {
     if constexpr (B < NR) {
 #pragma unroll
         for (int j = 0; j < (1 << NR); ++j) {
             if (j & (1 << B)) continue; // compile-time
             float2 &v0 = v[j], &v1 = v[j | (1 << B)];
             // a lane with bit 0 gives v1 and takes its partner's v0 there
-            float2 s;
-            s.x = up ? v0.x : v1.x;
-            s.y = up ? v0.y : v1.y;
-            s.x = __shfl_xor_sync(0xffffffffu, s.x, xm);
-            s.y = __shfl_xor_sync(0xffffffffu, s.y, xm);
-            v0.x = up ? s.x : v0.x;
-            v0.y = up ? s.y : v0.y;
-            v1.x = up ? v1.x : s.x;
-            v1.y = up ? v1.y : s.y;
+            const float sx = __shfl_xor_sync(0xffffffffu, rt32_sel(up, v0.x, v1.x), xm);
+            const float sy = __shfl_xor_sync(0xffffffffu, rt32_sel(up, v0.y, v1.y), xm);
+            v0 = make_float2(rt32_sel(up, sx, v0.x), rt32_sel(up, sy, v0.y));
+            v1 = make_float2(rt32_sel(up, v1.x, sx), rt32_sel(up, v1.y, sy));
         }
     }
 }
@@ -206,8 +207,10 @@ __device__ __forceinline__ void rt32_gate(float2 (&v)[1 << NR], const RtOp& op, 
 }
 
 // One op; every thread of the CTA calls it with the same op. base: the index
-// bits outside the tile.
-template <int NR>
+// bits outside the tile. TRADE: the program may hold kRtTrade (a kernel that
+// never meets it leaves it out: a case that only renames registers costs every
+// other one about 30 moves to bring them back, 10% of a 2-qubit gate).
+template <int NR, bool TRADE>
 __device__ __forceinline__ void rt32_op(float2 (&v)[1 << NR], const RtOp& op, const RtLayoutTab* lays,
                                         const float4* coef, float2* tile, int T, int lane, int warp,
                                         uint64_t base) {
@@ -221,22 +224,24 @@ __device__ __forceinline__ void rt32_op(float2 (&v)[1 << NR], const RtOp& op, co
             rt32_gate<NR, false>(v, op, m, true, 0, 0);
         }
     } else if (type == kRtSwap) {
-        const bool up = (lane >> op.a) & 1;
         const int xm = 1 << op.a;
+        const uint32_t up = (lane & xm) ? ~0u : 0u;
         switch (op.b) {
             case 0: rt32_swap<NR, 0>(v, up, xm); break;
             case 1: rt32_swap<NR, 1>(v, up, xm); break;
             case 2: rt32_swap<NR, 2>(v, up, xm); break;
             default: rt32_swap<NR, 3>(v, up, xm); break;
         }
-    } else if (type == kRtTrade) {
-        switch (op.a * 4 + op.b) {
-            case 1: rt32_trade<NR, 0, 1>(v); break;
-            case 2: rt32_trade<NR, 0, 2>(v); break;
-            case 3: rt32_trade<NR, 0, 3>(v); break;
-            case 6: rt32_trade<NR, 1, 2>(v); break;
-            case 7: rt32_trade<NR, 1, 3>(v); break;
-            default: rt32_trade<NR, 2, 3>(v); break;
+    } else if (TRADE && type == kRtTrade) {
+        if constexpr (TRADE) {
+            switch (op.a * 4 + op.b) {
+                case 1: rt32_trade<NR, 0, 1>(v); break;
+                case 2: rt32_trade<NR, 0, 2>(v); break;
+                case 3: rt32_trade<NR, 0, 3>(v); break;
+                case 6: rt32_trade<NR, 1, 2>(v); break;
+                case 7: rt32_trade<NR, 1, 3>(v); break;
+                default: rt32_trade<NR, 2, 3>(v); break;
+            }
         }
     } else {
         // a warp writes the positions it read at the last layout (swaps stay

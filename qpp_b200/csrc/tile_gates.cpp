@@ -338,8 +338,15 @@ void run_reg_program(qgpu_state* s, const RegProgram& P) {
     StreamBuf buf(s->ctx, P.blob.size());
     QG_CUDA(cudaMemcpyAsync(buf.p, P.blob.data(), P.blob.size(), cudaMemcpyHostToDevice,
                             s->ctx->stream));
+    // Chained launches only on a live stream: captured into a graph, the early
+    // start of a pass faulted on the device.
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    QG_CUDA(cudaStreamIsCapturing(s->ctx->stream, &cap));
     bool chained = false;
-    for (const RegPass& p : P.passes) launch_reg(s, P, p, buf.p, chained);
+    for (const RegPass& p : P.passes) {
+        launch_reg(s, P, p, buf.p, chained);
+        chained = chained && cap == cudaStreamCaptureStatusNone;
+    }
 }
 
 void plan_and_run_reg(qgpu_state* s, const std::vector<GateDesc>& gates, int Tmax, RegProgram& P) {
