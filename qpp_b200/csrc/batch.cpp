@@ -38,8 +38,8 @@
 
 namespace qgpu {
 
-// Register bits (kets: qubits; density matrices: twice the qubits) from which
-// batched instances run block-layered.
+// Register bits (twice the qubits) from which batched density matrices run
+// block-layered.
 constexpr int kBlockMinBits = 18;
 // Register bits from which programs of 1- and 2-qubit gates run as register
 // tile passes (every tile of the same shape), and up to which density matrices
@@ -266,18 +266,14 @@ extern "C" qgpu_status qgpu_run_batch(qgpu_ctx* ctx, uint32_t n_inst, qgpu_circu
         for (uint32_t i = 0; i < n_inst; ++i)
             if (on_reg[i]) regs.push_back(i);
         // Block-layered registers (no reference counterpart): density matrices
-        // of at least kBlockMinBits virtual qubits (up to 15 qubits) and kets
-        // of at least kBlockMinBits qubits whose programs are dense gates. Each
-        // program is fused into blocks of <= 4 qubits (virtual qubits for a
-        // density matrix: a layer's gates and channels on one qubit pair
-        // become one block), and launch j of one chain applies block j of
-        // every such register, one HBM pass per block with one thread per
-        // group (k_block_batch). Above 2^18 amplitudes this beats the layered
-        // tile passes, whose per-gate barriers held them to about a quarter of
-        // HBM bandwidth there.
+        // of at least kBlockMinBits virtual qubits (up to 15 qubits) that do not
+        // run as register tiles. Each program is fused into blocks of <= 4
+        // virtual qubits (a layer's gates and channels on one qubit pair become
+        // one block), and launch j of one chain applies block j of every such
+        // register, one HBM pass per block with one thread per group
+        // (k_block_batch).
         std::vector<uint32_t> blocked;
         std::vector<char> on_block(n_inst, 0);
-        std::vector<qgpu::TProgram> bprog(n_inst); // kets' block programs
         if (form == 1) {
             std::vector<uint32_t> cand;
             std::map<qgpu_circuit*, uint32_t> first_of; // one build per circuit
@@ -302,24 +298,6 @@ extern "C" qgpu_status qgpu_run_batch(qgpu_ctx* ctx, uint32_t n_inst, qgpu_circu
             });
             for (uint32_t i : cand) {
                 if (!good[first_of.at(circuits[i])]) continue;
-                ok[i] = 0;
-                on_block[i] = 1;
-                blocked.push_back(i);
-            }
-            std::vector<uint32_t> kets;
-            for (uint32_t i = 0; i < n_inst; ++i) {
-                if (!ok[i] || states[i]->kind != QGPU_KET || states[i]->ctx != ctx ||
-                    progs[i].n < uint32_t(qgpu::kBlockMinBits) || !all_gates(progs[i]))
-                    continue;
-                bool dense = true;
-                for (const auto& I : progs[i].ins) dense = dense && I.op != qgpu::kTCG1;
-                if (dense) kets.push_back(i);
-            }
-            pfor(kets.size(), [&](size_t k) {
-                bprog[kets[k]] = std::move(progs[kets[k]]);
-                qgpu::fuse_blocks(bprog[kets[k]], 4);
-            });
-            for (uint32_t i : kets) {
                 ok[i] = 0;
                 on_block[i] = 1;
                 blocked.push_back(i);
@@ -411,8 +389,7 @@ extern "C" qgpu_status qgpu_run_batch(qgpu_ctx* ctx, uint32_t n_inst, qgpu_circu
                 std::vector<const qgpu::TProgram*> bp, uniq;
                 size_t jmax = 0, nfloat = 0;
                 for (uint32_t i : blocked) {
-                    const qgpu::TProgram* P =
-                        states[i]->kind == QGPU_KET ? &bprog[i] : circuits[i]->rho_prog.get();
+                    const qgpu::TProgram* P = circuits[i]->rho_prog.get();
                     bp.push_back(P);
                     jmax = std::max(jmax, P->ins.size());
                     if (bbase.count(P)) continue;
