@@ -346,6 +346,10 @@ extern "C" qgpu_status qgpu_run_batch(qgpu_ctx* ctx, uint32_t n_inst, qgpu_circu
             int layer_bits = 0;
             for (size_t k = 0; k < prog.size(); ++k)
                 if (layered[k]) layer_bits = std::max(layer_bits, std::min(tile_of.at(prog[k].second.n) ? tile_of.at(prog[k].second.n) : 12, 12));
+            // programs of the trajectory kernel: runs of gates as sweeps
+            pfor(prog.size(), [&](size_t k) {
+                if (!layered[k]) qgpu::plan_sweeps(prog[k].second);
+            });
             ctx->batch_ms[0] = ms_since(t_compile);
             auto t_build = clk::now();
             // device copies of all programs, per-CTA work items grouped by size
@@ -357,6 +361,7 @@ extern "C" qgpu_status qgpu_run_batch(qgpu_ctx* ctx, uint32_t n_inst, qgpu_circu
                 ofs[k] = {ins.size(), mats.size() / 2};
                 ins.insert(ins.end(), prog[k].second.ins.begin(), prog[k].second.ins.end());
                 mats.insert(mats.end(), prog[k].second.mats.begin(), prog[k].second.mats.end());
+                mats.resize((mats.size() + 3) / 4 * 4); // every program on a 16-byte boundary
                 if (!layered[k]) by_n[prog[k].second.n].push_back(k);
             }
             // the passes of each layered register, in program order

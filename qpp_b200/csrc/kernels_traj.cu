@@ -12,6 +12,15 @@
 // again (equivalent to qpp removing it). After the last step one full-basis
 // index is sampled from |psi|^2 (the shot's result).
 //
+// Gates run in sweeps (tr_sweep): consecutive gates on at most four bits share
+// one trip of the register or tile through a thread's registers and one barrier,
+// and the noise of a window of steps is drawn ahead by the whole CTA. One gate,
+// one noise draw and two barriers at a time, 20 layers of 16-qubit trajectories
+// ran at 10.4 TFLOP/s (148 shots 9.6 ms), 14-qubit ones at 17.1, 12-qubit ones at
+// 19.2; now at 16.9 (5.9 ms), 26.6 and 23.0. What bounds it is issue: a
+// 1-qubit gate is 128 FMAs of a thread's 16 amplitudes and about 100 other
+// instructions, a 2-qubit gate 256 and 120.
+//
 // Arithmetic: amplitudes in complex64 with FP32 arithmetic; measurement
 // probabilities, renormalisation factors and the final sampling prefix sums
 // in FP64. Randomness: Philox4x32-10 keyed by the request seed with counter
@@ -25,6 +34,7 @@
 
 #include "common.cuh"
 #include "kernels.hpp"
+#include "regtile32.cuh"
 #include "traj.hpp"
 
 namespace qgpu {
@@ -32,20 +42,25 @@ namespace qgpu {
 __device__ __forceinline__ float2 c_mul(float2 a, float2 b) {
     return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
-__device__ __forceinline__ float2 c_fma(float2 a, float2 b, float2 c) {
-    c.x = fmaf(a.x, b.x, c.x);
-    c.x = fmaf(-a.y, b.y, c.x);
-    c.y = fmaf(a.x, b.y, c.y);
-    c.y = fmaf(a.y, b.x, c.y);
-    return c;
-}
+__device__ __forceinline__ float2 c_fma(float2 a, float2 b, float2 c) { return c32_fma(a, b, c); }
 
 __device__ __forceinline__ uint32_t ins0(uint32_t x, int b) {
     uint32_t low = (1u << b) - 1;
     return ((x & ~low) << 1) | (x & low);
 }
 
-// block-wide FP64 sum (256 threads), result broadcast to every thread
+// Position of amplitude i of a register or tile. In shared memory (SW) the 16
+// amplitudes of a 128-byte row are swizzled: the column XORed with the folded
+// row number, so that the strided accesses of gates on low bits spread over the
+// banks. The map is linear over GF(2).
+template <bool SW>
+__device__ __forceinline__ uint32_t ix(uint32_t i) {
+    if constexpr (!SW) return i;
+    const uint32_t r = i >> 4;
+    return i ^ ((r ^ (r >> 4) ^ (r >> 8)) & 15u);
+}
+
+// block-wide FP64 sum (at most 512 threads), result broadcast to every thread
 __device__ double block_sum_d(double v, double* red) {
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) v += __shfl_down_sync(0xffffffffu, v, s);
@@ -61,6 +76,7 @@ __device__ double block_sum_d(double v, double* red) {
 // kTG3: 8 x 8 on bits (b0, b1, b2 = cmask & 255), row index 4 b0 + 2 b1 + b2;
 // each thread owns whole groups. The row loop stays rolled so that the 64
 // matrix entries are read per row (L1) rather than held in registers.
+template <bool SW>
 __device__ __forceinline__ void tr_gate3(const TInstr& I, const float2* __restrict__ mats,
                                       float2* psi, uint32_t N, int tid, int nt) {
     const float2* m = mats + I.mat;
@@ -75,7 +91,7 @@ __device__ __forceinline__ void tr_gate3(const TInstr& I, const float2* __restri
         float2 v[8];
 #pragma unroll
         for (int c = 0; c < 8; ++c)
-            v[c] = psi[i + ((c & 4) ? o4 : 0u) + ((c & 2) ? o2 : 0u) + ((c & 1) ? o1 : 0u)];
+            v[c] = psi[ix<SW>(i + ((c & 4) ? o4 : 0u) + ((c & 2) ? o2 : 0u) + ((c & 1) ? o1 : 0u))];
         // all eight inputs are in registers, so each row writes in place
 #pragma unroll 1
         for (int row = 0; row < 8; ++row) {
@@ -83,13 +99,14 @@ __device__ __forceinline__ void tr_gate3(const TInstr& I, const float2* __restri
             float2 acc = c_mul(mr[0], v[0]);
 #pragma unroll
             for (int c = 1; c < 8; ++c) acc = c_fma(mr[8 * c], v[c], acc);
-            psi[i + ((row & 4) ? o4 : 0u) + ((row & 2) ? o2 : 0u) + ((row & 1) ? o1 : 0u)] = acc;
+            psi[ix<SW>(i + ((row & 4) ? o4 : 0u) + ((row & 2) ? o2 : 0u) + ((row & 1) ? o1 : 0u))] = acc;
         }
     }
 }
 
 // One gate instruction (G1, CG1, G2, G3, G4) on a register of N amplitudes at
 // psi (shared or global memory); every thread of the CTA calls it.
+template <bool SW>
 __device__ __forceinline__ void tr_gate(const TInstr& I, const float2* __restrict__ mats,
                                         float2* psi, uint32_t N, int tid, int nt) {
     switch (I.op) {
@@ -99,9 +116,9 @@ __device__ __forceinline__ void tr_gate(const TInstr& I, const float2* __restric
             const uint32_t s = 1u << I.b0;
             for (uint32_t p = tid; p < N / 2; p += nt) {
                 uint32_t i = ins0(p, I.b0);
-                float2 v0 = psi[i], v1 = psi[i + s];
-                psi[i] = c_fma(a01, v1, c_mul(a00, v0));
-                psi[i + s] = c_fma(a11, v1, c_mul(a10, v0));
+                float2 v0 = psi[ix<SW>(i)], v1 = psi[ix<SW>(i + s)];
+                psi[ix<SW>(i)] = c_fma(a01, v1, c32_mul2(a00, v0));
+                psi[ix<SW>(i + s)] = c_fma(a11, v1, c32_mul2(a10, v0));
             }
             break;
         }
@@ -112,9 +129,9 @@ __device__ __forceinline__ void tr_gate(const TInstr& I, const float2* __restric
             for (uint32_t p = tid; p < N / 2; p += nt) {
                 uint32_t i = ins0(p, I.b0);
                 if ((i & I.cmask) != I.cval) continue;
-                float2 v0 = psi[i], v1 = psi[i + s];
-                psi[i] = c_fma(a01, v1, c_mul(a00, v0));
-                psi[i + s] = c_fma(a11, v1, c_mul(a10, v0));
+                float2 v0 = psi[ix<SW>(i)], v1 = psi[ix<SW>(i + s)];
+                psi[ix<SW>(i)] = c_fma(a01, v1, c32_mul2(a00, v0));
+                psi[ix<SW>(i + s)] = c_fma(a11, v1, c32_mul2(a10, v0));
             }
             break;
         }
@@ -124,25 +141,25 @@ __device__ __forceinline__ void tr_gate(const TInstr& I, const float2* __restric
             const uint32_t s0 = 1u << I.b0, s1 = 1u << I.b1;
             for (uint32_t p = tid; p < N / 4; p += nt) {
                 uint32_t i = ins0(ins0(p, lo), hi);
-                float2 v[4] = {psi[i], psi[i + s1], psi[i + s0], psi[i + s0 + s1]};
+                float2 v[4] = {psi[ix<SW>(i)], psi[ix<SW>(i + s1)], psi[ix<SW>(i + s0)], psi[ix<SW>(i + s0 + s1)]};
                 float2 r[4];
 #pragma unroll
                 for (int row = 0; row < 4; ++row) {
-                    float2 acc = c_mul(m[row], v[0]);
+                    float2 acc = c32_mul(m[row], v[0]);
                     acc = c_fma(m[row + 4], v[1], acc);
                     acc = c_fma(m[row + 8], v[2], acc);
                     acc = c_fma(m[row + 12], v[3], acc);
                     r[row] = acc;
                 }
-                psi[i] = r[0];
-                psi[i + s1] = r[1];
-                psi[i + s0] = r[2];
-                psi[i + s0 + s1] = r[3];
+                psi[ix<SW>(i)] = r[0];
+                psi[ix<SW>(i + s1)] = r[1];
+                psi[ix<SW>(i + s0)] = r[2];
+                psi[ix<SW>(i + s0 + s1)] = r[3];
             }
             break;
         }
         case kTG3:
-            tr_gate3(I, mats, psi, N, tid, nt);
+            tr_gate3<SW>(I, mats, psi, N, tid, nt);
             break;
         case kTG4: {
             // 16 x 16 on bits (b0, b1, b2, b3) = (b0, b1, cmask & 255,
@@ -175,10 +192,10 @@ __device__ __forceinline__ void tr_gate(const TInstr& I, const float2* __restric
                 if (valid) {
                     i = ins0(ins0(ins0(ins0(g, sb[0]), sb[1]), sb[2]), sb[3]);
 #pragma unroll 4
-                    for (int c = 0; c < 16; ++c) acc = c_fma(m[row + 16 * c], psi[i + off(c)], acc);
+                    for (int c = 0; c < 16; ++c) acc = c_fma(m[row + 16 * c], psi[ix<SW>(i + off(c))], acc);
                 }
                 __syncthreads();
-                if (valid) psi[i + off(row)] = acc;
+                if (valid) psi[ix<SW>(i + off(row))] = acc;
                 __syncthreads();
             }
             break;
@@ -189,11 +206,11 @@ __device__ __forceinline__ void tr_gate(const TInstr& I, const float2* __restric
 }
 
 // Depolarising draws of one circuit step (counter `ins` = the instruction's
-// index in the untiled program): thread b <-> qubit b. Returns whether any
-// qubit drew a Pauli (uniform over the CTA). With `apply`, the Pauli string is
-// recorded and applied to all N amplitudes at psi.
-__device__ bool tr_noise(const TWork& W, uint32_t ins, int n, uint32_t alive, bool apply,
-                         float2* psi, uint32_t N, TEvent* events, int max_events,
+// index in the untiled program): thread b <-> qubit b. The Pauli string drawn is
+// recorded and applied to all N amplitudes at psi; returns whether any qubit drew
+// one (uniform over the CTA).
+template <bool SW>
+__device__ bool tr_noise(const TWork& W, uint32_t ins, int n, uint32_t alive, float2* psi, uint32_t N, TEvent* events, int max_events,
                          uint32_t* sh /* xm, zm, ny, nev */) {
     const int tid = threadIdx.x, nt = blockDim.x;
     int pk = 0;
@@ -203,7 +220,6 @@ __device__ bool tr_noise(const TWork& W, uint32_t ins, int n, uint32_t alive, bo
         if (u0 < double(W.p_noise)) pk = 1 + min(int(u1 * 3.0), 2); // 1 X, 2 Y, 3 Z
     }
     if (!__syncthreads_or(pk != 0)) return false;
-    if (!apply) return true;
     if (tid == 0) sh[0] = sh[1] = sh[2] = 0;
     __syncthreads();
     if (pk) {
@@ -224,23 +240,160 @@ __device__ bool tr_noise(const TWork& W, uint32_t ins, int n, uint32_t alive, bo
                      : ny % 4 == 2 ? make_float2(-1, 0) : make_float2(0, -1);
     if (xm == 0) {
         for (uint32_t i = tid; i < N; i += nt) {
-            float2 a = c_mul(gph, psi[i]);
+            float2 a = c_mul(gph, psi[ix<SW>(i)]);
             if (__popc(i & zm) & 1) a = make_float2(-a.x, -a.y);
-            psi[i] = a;
+            psi[ix<SW>(i)] = a;
         }
     } else {
         int hb = 31 - __clz(xm); // pair (i, i ^ xm) with bit hb of i clear
         for (uint32_t p = tid; p < N / 2; p += nt) {
             uint32_t i = ins0(p, hb), j = i ^ xm;
-            float2 a = c_mul(gph, psi[i]), b = c_mul(gph, psi[j]);
+            float2 a = c_mul(gph, psi[ix<SW>(i)]), b = c_mul(gph, psi[ix<SW>(j)]);
             if (__popc(i & zm) & 1) a = make_float2(-a.x, -a.y);
             if (__popc(j & zm) & 1) b = make_float2(-b.x, -b.y);
-            psi[j] = a;
-            psi[i] = b;
+            psi[ix<SW>(j)] = a;
+            psi[ix<SW>(i)] = b;
         }
     }
     __syncthreads();
     return true;
+}
+
+// The noise of a window of steps, drawn ahead by the whole CTA: bit e of `bits`
+// says whether any living qubit draws a Pauli before noise step first + e (the
+// draws themselves are repeated by tr_noise for the few steps that have one).
+// Drawn step by step, each costs a Philox evaluation's latency and a barrier.
+constexpr uint32_t kNoiseWindow = 2048;
+struct NoiseWindow {
+    uint32_t first, end;
+    uint32_t* bits; // kNoiseWindow / 32 + 1 words of shared memory
+};
+
+// Moves the window to steps [st, ...) unless it holds [st, st + cnt) already;
+// every thread of the CTA calls it.
+__device__ __forceinline__ void noise_window(const TWork& W, NoiseWindow& N, uint32_t st, uint32_t cnt,
+                                             int n) {
+    if (st >= N.first && st + cnt <= N.end) return;
+    const int tid = threadIdx.x, nt = blockDim.x;
+    __syncthreads();
+    for (uint32_t i = tid; i <= kNoiseWindow / 32; i += nt) N.bits[i] = 0;
+    N.first = st;
+    N.end = min(st + kNoiseWindow, W.nnoise);
+    __syncthreads();
+    // u < p for u = m 2^-53, compared as integers: m < ceil(p 2^53)
+    const uint64_t thr = uint64_t(ceil(double(W.p_noise) * 0x1.0p53));
+    const uint32_t total = (N.end - N.first) * uint32_t(n);
+    for (uint32_t i = tid; i < total; i += nt) {
+        const uint32_t e = i / uint32_t(n), b = i - e * uint32_t(n);
+        const uint2 s = W.noise[N.first + e]; // untiled index, living qubits
+        if (!((s.y >> b) & 1u)) continue;
+        uint32_t x[4] = {W.shot, s.x, b, 0x6e6f6973u};
+        philox4x32_10(x, uint32_t(W.seed), uint32_t(W.seed >> 32));
+        const uint64_t m = ((uint64_t(x[0]) << 21) ^ (uint64_t(x[1]) >> 11)) & ((uint64_t(1) << 53) - 1);
+        if (m < thr) atomicOr(&N.bits[e >> 5], 1u << (e & 31u));
+    }
+    __syncthreads();
+}
+
+// Whether one of the cnt <= 32 steps from st on (inside the window) has noise.
+__device__ __forceinline__ bool noise_any(const NoiseWindow& N, uint32_t st, uint32_t cnt) {
+    const uint32_t q = st - N.first, w = q >> 5;
+    const uint64_t two = uint64_t(N.bits[w]) | (uint64_t(N.bits[w + 1]) << 32);
+    return (two >> (q & 31u)) & ((uint64_t(1) << cnt) - 1);
+}
+
+// The gates of a sweep (header H at prog[0]; plan_sweeps) on a swizzled register
+// of N >= 16 amplitudes in shared memory: every thread takes groups of the 16
+// amplitudes that differ in the sweep's four bits into registers, applies the
+// gates there in order and writes them back. The products are tr_gate's, in the
+// same order.
+__device__ __forceinline__ void tr_sweep(const TInstr* __restrict__ prog, const float2* __restrict__ mats,
+                                         float2* psi, uint32_t N, int tid, int nt) {
+    const TInstr H = prog[0];
+    uint32_t m[4], sm[4];
+    int sb[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        sb[k] = int((H.mat >> (8 * k)) & 255u);
+        m[k] = 1u << sb[k];
+        sm[k] = ix<true>(m[k]);
+    }
+    const uint32_t sweep = m[0] | m[1] | m[2] | m[3];
+#pragma unroll
+    for (int x = 0; x < 3; ++x)
+#pragma unroll
+        for (int y = 0; y < 3 - x; ++y)
+            if (sb[y] > sb[y + 1]) {
+                const int t = sb[y];
+                sb[y] = sb[y + 1];
+                sb[y + 1] = t;
+            }
+    for (uint32_t g = tid; g < N / 16; g += nt) {
+        const uint32_t b = ins0(ins0(ins0(ins0(g, sb[0]), sb[1]), sb[2]), sb[3]);
+        const uint32_t pb = ix<true>(b);
+        float2 v[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            v[j] = psi[pb ^ ((j & 1) ? sm[0] : 0u) ^ ((j & 2) ? sm[1] : 0u) ^ ((j & 4) ? sm[2] : 0u) ^
+                       ((j & 8) ? sm[3] : 0u)];
+        // The two commonest sweeps as straight code: gates one by one pay for a
+        // branch and for bringing the 32 registers back to their places (about
+        // 100 instructions beside a G1's 128 and a G2's 256).
+        const float4* mq[4];
+        if (H.b1 != kSweepAny) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                mq[q] = reinterpret_cast<const float4*>(mats + prog[H.b1 == kSweep2x2q ? 1 + q / 2 : 1 + q].mat);
+        }
+        if (H.b1 == kSweep4x1q) {
+            rt32_g1<4, 0, false, true>(v, mq[0], true, 0, 0);
+            rt32_g1<4, 1, false, true>(v, mq[1], true, 0, 0);
+            rt32_g1<4, 2, false, true>(v, mq[2], true, 0, 0);
+            rt32_g1<4, 3, false, true>(v, mq[3], true, 0, 0);
+        } else if (H.b1 == kSweep2x2q) {
+            rt32_g2<4, 0, 1, false, true>(v, mq[0], true, 0, 0);
+            rt32_g2<4, 2, 3, false, true>(v, mq[2], true, 0, 0);
+        } else for (uint32_t q = 1; q <= H.cmask; ++q) {
+            const TInstr I = prog[q];
+            const float4* const mt = reinterpret_cast<const float4*>(mats + I.mat);
+            const int A = (I.flags >> 2) & 3, B = (I.flags >> 4) & 3;
+            if (I.op == kTG2) {
+                switch (A * 4 + B) {
+                    case 1: rt32_g2<4, 0, 1, false, true>(v, mt, true, 0, 0); break;
+                    case 2: rt32_g2<4, 0, 2, false, true>(v, mt, true, 0, 0); break;
+                    case 3: rt32_g2<4, 0, 3, false, true>(v, mt, true, 0, 0); break;
+                    case 6: rt32_g2<4, 1, 2, false, true>(v, mt, true, 0, 0); break;
+                    case 7: rt32_g2<4, 1, 3, false, true>(v, mt, true, 0, 0); break;
+                    default: rt32_g2<4, 2, 3, false, true>(v, mt, true, 0, 0); break;
+                }
+            } else if (I.op == kTG1) {
+                switch (A) {
+                    case 0: rt32_g1<4, 0, false, true>(v, mt, true, 0, 0); break;
+                    case 1: rt32_g1<4, 1, false, true>(v, mt, true, 0, 0); break;
+                    case 2: rt32_g1<4, 2, false, true>(v, mt, true, 0, 0); break;
+                    default: rt32_g1<4, 3, false, true>(v, mt, true, 0, 0); break;
+                }
+            } else { // CG1: controls on the sweep's bits per register, others per group
+                const bool ok = ((b ^ I.cval) & I.cmask & ~sweep) == 0;
+                uint32_t rm = 0, rv = 0;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if (I.cmask & m[k]) rm |= 1u << k;
+                    if (I.cval & m[k]) rv |= 1u << k;
+                }
+                switch (A) {
+                    case 0: rt32_g1<4, 0, true, true>(v, mt, ok, rm, rv); break;
+                    case 1: rt32_g1<4, 1, true, true>(v, mt, ok, rm, rv); break;
+                    case 2: rt32_g1<4, 2, true, true>(v, mt, ok, rm, rv); break;
+                    default: rt32_g1<4, 3, true, true>(v, mt, ok, rm, rv); break;
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            psi[pb ^ ((j & 1) ? sm[0] : 0u) ^ ((j & 2) ? sm[1] : 0u) ^ ((j & 4) ? sm[2] : 0u) ^
+                ((j & 8) ? sm[3] : 0u)] = v[j];
+    }
 }
 
 // A tile pass (kTTile header H at program position k): the m instructions
@@ -249,11 +402,11 @@ __device__ bool tr_noise(const TWork& W, uint32_t ins, int n, uint32_t alive, bo
 // into shared memory, the instructions run there on local bit positions,
 // and the tile is written back. Noise of a step inside the pass splits it:
 // the instructions before run tiled, the Pauli string is applied to the
-// whole register, and the pass resumes. `orig0` = untiled index of the first
-// instruction of the pass.
-__device__ void tr_tile_pass(const TWork& W, uint32_t k, uint32_t orig0, int n, uint32_t alive,
-                             float2* psi, float2* tile, uint32_t* offh, TEvent* events,
-                             int max_events, uint32_t* sh) {
+// whole register, and the pass resumes. `orig` = untiled index of the pass's
+// first instruction and `st` its first noise step; both move past the pass.
+__device__ void tr_tile_pass(const TWork& W, uint32_t k, uint32_t& orig, uint32_t& st, NoiseWindow& NW,
+                             int n, uint32_t alive, float2* psi, float2* tile, uint32_t* offh,
+                             TEvent* events, int max_events, uint32_t* sh) {
     const int tid = threadIdx.x, nt = blockDim.x;
     const TInstr H = W.prog[k];
     const int T = H.b0;
@@ -275,16 +428,27 @@ __device__ void tr_tile_pass(const TWork& W, uint32_t k, uint32_t orig0, int n, 
     const uint32_t end = k + 1 + m;
     bool start_done = false; // noise before `start` already applied
     while (start < end) {
-        uint32_t stop = end;
-        if (W.p_noise > 0.f)
-            for (uint32_t i = start; i < end; ++i) {
-                if (!(W.prog[i].flags & kTNewStep) || (i == start && start_done)) continue;
-                if (tr_noise(W, orig0 + (i - k - 1), n, alive, false, psi, 0, events, max_events, sh)) {
-                    stop = i;
+        // the instructions up to the next step with noise (or, in a pass of more
+        // steps than the window holds, up to the window's end)
+        uint32_t stop = start, o2 = orig, s2 = st;
+        bool noise = false;
+        for (; stop < end; ++stop) {
+            const TInstr& I = W.prog[stop];
+            if (I.op == kTSweep) continue;
+            if ((I.flags & kTNewStep) && W.p_noise > 0.f && !(stop == start && start_done)) {
+                if (s2 >= NW.end || s2 < NW.first) {
+                    if (o2 != orig) break;
+                    noise_window(W, NW, s2, 1, n);
+                }
+                if (noise_any(NW, s2, 1)) {
+                    noise = true;
                     break;
                 }
+                ++s2;
             }
-        if (stop > start) {
+            ++o2;
+        }
+        if (o2 != orig) {
             for (uint32_t t = 0; t < ntiles; ++t) {
                 // deposit t into the bits outside the tile
                 uint32_t base = 0, r = rest, tt = t;
@@ -304,47 +468,68 @@ __device__ void tr_tile_pass(const TWork& W, uint32_t k, uint32_t orig0, int n, 
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
                         const uint32_t l = l0 + u * nt + tid;
-                        if (l < NT) tile[l] = v[u];
+                        if (l < NT) tile[ix<true>(l)] = v[u];
                     }
                 }
                 __syncthreads();
                 for (uint32_t i = start; i < stop; ++i) {
-                    tr_gate(W.prog[i], W.mats, tile, NT, tid, nt);
+                    if (W.prog[i].op == kTSweep) {
+                        // a sweep cut by `stop` (or entered in its middle) runs
+                        // gate by gate
+                        if (i + W.prog[i].cmask < stop) {
+                            tr_sweep(W.prog + i, W.mats, tile, NT, tid, nt);
+                            i += W.prog[i].cmask;
+                        } else {
+                            continue;
+                        }
+                    } else {
+                        tr_gate<true>(W.prog[i], W.mats, tile, NT, tid, nt);
+                    }
                     __syncthreads();
                 }
-                for (uint32_t l = tid; l < NT; l += nt) psi[base + offh[l >> 5] + (l & 31u)] = tile[l];
+                for (uint32_t l = tid; l < NT; l += nt)
+                    psi[base + offh[l >> 5] + (l & 31u)] = tile[ix<true>(l)];
                 __syncthreads();
             }
         }
-        if (stop < end) {
-            tr_noise(W, orig0 + (stop - k - 1), n, alive, true, psi, 1u << n, events, max_events, sh);
-            start = stop;
+        orig = o2;
+        st = s2;
+        start = stop;
+        start_done = false;
+        if (noise) {
+            tr_noise<false>(W, orig, n, alive, psi, 1u << n, events, max_events, sh);
+            ++st; // its own step is done; the instruction itself comes next
             start_done = true;
-        } else {
-            start = end;
         }
     }
 }
 
-__global__ void __launch_bounds__(256, 4)
+// One trajectory per CTA. GLOBAL = false: registers of up to 2^14 amplitudes,
+// swizzled in shared memory. GLOBAL = true: larger ones, in this CTA's own slot
+// of a global scratch buffer or in place in their own state (L2 / HBM), which
+// __syncthreads makes coherent between the block's threads; their tile passes
+// use the shared memory as the tile. A 14-qubit register fills an SM's shared
+// memory and a burst of larger ones has fewer shots than SMs, so from 14 qubits
+// a CTA has 512 threads.
+template <bool GLOBAL, int NTHR, int MINB>
+__global__ void __launch_bounds__(NTHR, MINB)
     k_traj(const TWork* __restrict__ work, int nwork, uint32_t* __restrict__ dits,
            int maxcreg, uint64_t* __restrict__ samples, float2* __restrict__ dump,
            TEvent* __restrict__ events, int max_events, float2* __restrict__ gscratch,
            uint64_t gslot, int tile_bits) {
     extern __shared__ __align__(16) unsigned char sm[];
-    // registers of up to 2^14 amplitudes live in shared memory; larger ones
-    // in this CTA's own slot of a global scratch buffer or in place in their
-    // own state (L2 / HBM), which __syncthreads makes coherent between the
-    // block's threads; their tile passes use the shared memory as the tile
-    float2* const base = gscratch ? gscratch + uint64_t(blockIdx.x) * gslot
-                                  : reinterpret_cast<float2*>(sm);
+    constexpr bool SW = !GLOBAL;
+    float2* const base = GLOBAL && gscratch ? gscratch + uint64_t(blockIdx.x) * gslot
+                                            : reinterpret_cast<float2*>(sm);
     float2* const tile = reinterpret_cast<float2*>(sm);
     uint32_t* const offh = reinterpret_cast<uint32_t*>(sm + (size_t(1) << tile_bits) * sizeof(float2));
-    __shared__ double red[8];
-    __shared__ double part[256];
+    __shared__ double red[NTHR / 32];
+    __shared__ double part[NTHR];
     __shared__ uint32_t nsh[4]; // noise: xm, zm, ny, events so far
+    __shared__ uint32_t nbits[kNoiseWindow / 32 + 1];
     __shared__ int outcome_sh;
-    const int tid = threadIdx.x, nt = blockDim.x;
+    const int tid = threadIdx.x;
+    constexpr int nt = NTHR;
 
     for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
         const TWork W = work[w];
@@ -353,45 +538,73 @@ __global__ void __launch_bounds__(256, 4)
         // in place: the CTA works directly on the instance's own state;
         // an item without a buffer that can hold it is skipped (uniform
         // across the CTA, before any barrier of this iteration)
-        if (W.inplace ? W.fin == nullptr : (!gscratch && n > kTrajMaxQubits)) continue;
-        float2* const psi = W.inplace ? W.fin : base;
-        if (W.inplace) {
+        if (GLOBAL ? (W.inplace ? W.fin == nullptr : gscratch == nullptr)
+                   : (W.inplace || n > kTrajMaxQubits)) continue;
+        float2* const psi = GLOBAL && W.inplace ? W.fin : base;
+        if (GLOBAL && W.inplace) {
         } else if (W.init)
-            for (uint32_t i = tid; i < N; i += nt) psi[i] = W.init[i];
+            for (uint32_t i = tid; i < N; i += nt) psi[ix<SW>(i)] = W.init[i];
         else
-            for (uint32_t i = tid; i < N; i += nt) psi[i] = make_float2(i == 0 ? 1.f : 0.f, 0.f);
+            for (uint32_t i = tid; i < N; i += nt) psi[ix<SW>(i)] = make_float2(i == 0 ? 1.f : 0.f, 0.f);
         uint32_t alive = (n == 32) ? 0xffffffffu : ((1u << n) - 1);
         if (tid == 0) nsh[3] = 0;
         __syncthreads();
-        uint32_t nhdr = 0; // tile headers so far: untiled index = k - nhdr
+        uint32_t orig = 0, st = 0; // untiled index and noise step of instruction k
+        NoiseWindow NW{0, 0, nbits};
+        const bool noisy = W.p_noise > 0.f;
+        uint32_t sweep_end = 0; // up to here a sweep with noise runs gate by gate
         for (uint32_t k = 0; k < W.nins; ++k) {
             const TInstr I = W.prog[k];
             if (I.op == kTTile) {
                 // headers appear only in programs of registers above 2^14
                 // amplitudes, launched with a tile buffer of 2^tile_bits
-                if (int(I.b0) <= tile_bits && n > kTrajMaxQubits)
-                    tr_tile_pass(W, k, k - nhdr, n, alive, psi, tile, offh, events, max_events, nsh);
-                ++nhdr;
+                if constexpr (GLOBAL) {
+                    if (int(I.b0) <= tile_bits)
+                        tr_tile_pass(W, k, orig, st, NW, n, alive, psi, tile, offh, events, max_events, nsh);
+                }
                 k += I.cmask;
                 __syncthreads();
                 continue;
             }
-            const uint32_t orig = k - nhdr;
-            if ((I.flags & kTNewStep) && W.p_noise > 0.f)
-                tr_noise(W, orig, n, alive, true, psi, N, events, max_events, nsh);
+            if (I.op == kTSweep) {
+                if constexpr (!GLOBAL) {
+                    bool quiet = true;
+                    if (noisy && I.cval) {
+                        noise_window(W, NW, st, I.cval, n);
+                        quiet = !noise_any(NW, st, I.cval);
+                    }
+                    if (quiet) {
+                        tr_sweep(W.prog + k, W.mats, psi, N, tid, nt);
+                        orig += I.cmask;
+                        st += I.cval;
+                        k += I.cmask;
+                        __syncthreads();
+                    } else {
+                        sweep_end = k + 1 + I.cmask;
+                    }
+                }
+                continue;
+            }
+            if ((I.flags & kTNewStep) && noisy) {
+                if (k >= sweep_end) noise_window(W, NW, st, 1, n);
+                if (noise_any(NW, st, 1))
+                    tr_noise<SW>(W, orig, n, alive, psi, N, events, max_events, nsh);
+                ++st;
+            }
             switch (I.op) {
                 case kTG1:
                 case kTCG1:
                 case kTG2:
                 case kTG3:
                 case kTG4:
-                    tr_gate(I, W.mats, psi, N, tid, nt);
+                    tr_gate<SW>(I, W.mats, psi, N, tid, nt);
                     break;
                 case kTMeas: {
                     const uint32_t bit = 1u << I.b0;
                     double p1 = 0, tot = 0;
                     for (uint32_t i = tid; i < N; i += nt) {
-                        double w2 = double(psi[i].x) * psi[i].x + double(psi[i].y) * psi[i].y;
+                        const float2 a = psi[ix<SW>(i)];
+                        double w2 = double(a.x) * a.x + double(a.y) * a.y;
                         tot += w2;
                         if (i & bit) p1 += w2;
                     }
@@ -411,8 +624,8 @@ __global__ void __launch_bounds__(256, 4)
                     const float sc = float(1.0 / sqrt(pk));
                     for (uint32_t i = tid; i < N; i += nt) {
                         bool keep = (((i & bit) != 0) == (o == 1));
-                        float2 a = psi[i];
-                        psi[i] = keep ? make_float2(a.x * sc, a.y * sc) : make_float2(0.f, 0.f);
+                        float2 a = psi[ix<SW>(i)];
+                        psi[ix<SW>(i)] = keep ? make_float2(a.x * sc, a.y * sc) : make_float2(0.f, 0.f);
                     }
                     if (I.flags & kTDestructive) alive &= ~bit;
                     break;
@@ -420,20 +633,23 @@ __global__ void __launch_bounds__(256, 4)
                 default:
                     break;
             }
+            ++orig;
             __syncthreads();
         }
         if (W.diag) {
             // density matrix over n/2 qubits: its diagonal, for the shots
             const uint32_t Dh = 1u << (n / 2);
-            for (uint32_t i = tid; i < Dh; i += nt) W.diag[i] = double(psi[i * (Dh + 1)].x);
+            for (uint32_t i = tid; i < Dh; i += nt) W.diag[i] = double(psi[ix<SW>(i * (Dh + 1))].x);
         }
         // final full-basis sample: FP64 prefix sums over thread chunks
         if (!W.diag) {
             const uint32_t chunk = (N + nt - 1) / nt;
             double s = 0;
-            const uint32_t lo = tid * chunk, hi = min(N, lo + chunk);
-            for (uint32_t i = lo; i < hi; ++i)
-                s += double(psi[i].x) * psi[i].x + double(psi[i].y) * psi[i].y;
+            const uint32_t lo = min(N, tid * chunk), hi = min(N, lo + chunk);
+            for (uint32_t i = lo; i < hi; ++i) {
+                const float2 a = psi[ix<SW>(i)];
+                s += double(a.x) * a.x + double(a.y) * a.y;
+            }
             part[tid] = s;
             __syncthreads();
             if (tid == 0) {
@@ -450,7 +666,8 @@ __global__ void __launch_bounds__(256, 4)
                 }
                 if (t < nt) {
                     for (uint32_t i = t * chunk; i < min(N, (t + 1) * chunk); ++i) {
-                        cum += double(psi[i].x) * psi[i].x + double(psi[i].y) * psi[i].y;
+                        const float2 a = psi[ix<SW>(i)];
+                        cum += double(a.x) * a.x + double(a.y) * a.y;
                         if (cum >= thr) {
                             idx = i;
                             break;
@@ -462,9 +679,9 @@ __global__ void __launch_bounds__(256, 4)
             __syncthreads();
         }
         if (dump)
-            for (uint32_t i = tid; i < N; i += nt) dump[size_t(W.out) * N + i] = psi[i];
+            for (uint32_t i = tid; i < N; i += nt) dump[size_t(W.out) * N + i] = psi[ix<SW>(i)];
         if (W.fin && !W.inplace)
-            for (uint32_t i = tid; i < N; i += nt) W.fin[i] = psi[i];
+            for (uint32_t i = tid; i < N; i += nt) W.fin[i] = psi[ix<SW>(i)];
         __syncthreads();
     }
 }
@@ -681,7 +898,7 @@ __global__ void __launch_bounds__(256, 3)
         const PassInst& P = insts[cur.j];
         const uint32_t NT = 1u << P.T;
         for (uint32_t i = 0; i < P.nins; ++i) {
-            tr_gate(P.ins[i], P.mats, bc, NT, tid, nt);
+            tr_gate<false>(P.ins[i], P.mats, bc, NT, tid, nt);
             __syncthreads();
         }
         // the threads' shared-memory writes, visible to the bulk stores
@@ -831,11 +1048,24 @@ void launch_block_batch(qgpu_ctx* ctx, const BlockInst* dinsts, int ninst, uint3
     after_launch(ctx, "k_block_batch");
 }
 
+// The kernel for registers of n qubits and its threads per CTA.
+using TrajKernel = void (*)(const TWork*, int, uint32_t*, int, uint64_t*, float2*, TEvent*, int, float2*,
+                            uint64_t, int);
+static TrajKernel traj_kernel(int n, int& threads) {
+    threads = n >= kTrajMaxQubits ? 512 : 256;
+    if (n > kTrajMaxQubits) return k_traj<true, 512, 1>;
+    if (n == kTrajMaxQubits) return k_traj<false, 512, 1>;
+    return k_traj<false, 256, 2>; // 128 registers: three CTAs at 80 spill and run slower
+}
+
 void traj_prepare() {
     // a 2^14-amplitude register, or a tile of up to 2^14 amplitudes with its
     // offset table
-    ensure_smem(reinterpret_cast<const void*>(k_traj),
-                (size_t(1) << kTrajMaxQubits) * sizeof(float2) + 4096);
+    for (int n : {1, kTrajMaxQubits, kTrajMaxQubits + 1}) {
+        int threads;
+        ensure_smem(reinterpret_cast<const void*>(traj_kernel(n, threads)),
+                    (size_t(1) << kTrajMaxQubits) * sizeof(float2) + 4096);
+    }
 }
 
 int traj_global_grid(qgpu_ctx* ctx, int nwork, int n) {
@@ -844,23 +1074,26 @@ int traj_global_grid(qgpu_ctx* ctx, int nwork, int n) {
     return int(std::min<uint64_t>(std::min<uint64_t>(nwork, uint64_t(ctx->num_sms) * 8), by_mem));
 }
 
-// resident CTAs per SM for a dynamic shared-memory size (cached)
-static int traj_per_sm(size_t smem) {
+// resident CTAs per SM of n-qubit registers with a dynamic shared-memory size
+// (cached)
+static int traj_per_sm(int n, size_t smem) {
     static std::mutex mu;
-    static std::map<size_t, int> cache;
+    static std::map<std::pair<TrajKernel, size_t>, int> cache;
+    int threads;
+    const TrajKernel kernel = traj_kernel(n, threads);
     std::lock_guard<std::mutex> lock(mu);
-    auto it = cache.find(smem);
+    auto it = cache.find({kernel, smem});
     if (it != cache.end()) return it->second;
     int b = 0;
-    QG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_traj, 256, smem));
+    QG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, threads, smem));
     b = std::max(1, std::min(b, 8));
-    cache[smem] = b;
+    cache[{kernel, smem}] = b;
     return b;
 }
 
 int traj_resident_slots(qgpu_ctx* ctx, int n) {
     traj_prepare();
-    return ctx->num_sms * traj_per_sm((size_t(1) << n) * sizeof(float2));
+    return ctx->num_sms * traj_per_sm(n, (size_t(1) << n) * sizeof(float2));
 }
 
 void launch_traj(qgpu_ctx* ctx, const TWork* dwork, int nwork, int nmax, uint32_t* ddits,
@@ -869,25 +1102,27 @@ void launch_traj(qgpu_ctx* ctx, const TWork* dwork, int nwork, int nmax, uint32_
     if (nwork == 0) return;
     cudaStream_t st = stream ? stream : ctx->stream;
     traj_prepare();
+    int threads;
+    const TrajKernel kernel = traj_kernel(nmax, threads);
     if (nmax > kTrajMaxQubits) {
         if (tile_bits && (tile_bits < 9 || tile_bits > kTrajMaxQubits))
             raise(QGPU_ERR_INVALID_ARGUMENT, "launch_traj()", "tile_bits");
         const size_t smem = tile_bits ? (size_t(1) << tile_bits) * sizeof(float2) +
                                             (size_t(1) << (tile_bits - 5)) * sizeof(uint32_t)
                                       : 0;
-        const int cap = ctx->num_sms * traj_per_sm(smem);
+        const int cap = ctx->num_sms * traj_per_sm(nmax, smem);
         // no scratch: the caller promises in-place work items (own states)
         int grid = gscratch ? std::min(traj_global_grid(ctx, nwork, nmax), cap)
                             : std::min(nwork, cap);
-        k_traj<<<grid, 256, smem, st>>>(dwork, nwork, ddits, maxcreg, dsamples, ddump, devents,
-                                        max_events, gscratch, uint64_t(1) << nmax, tile_bits);
+        kernel<<<grid, threads, smem, st>>>(dwork, nwork, ddits, maxcreg, dsamples, ddump, devents,
+                                            max_events, gscratch, uint64_t(1) << nmax, tile_bits);
         after_launch(ctx, "k_traj (global)");
         return;
     }
     size_t smem = (size_t(1) << nmax) * sizeof(float2);
-    int grid = std::min(nwork, ctx->num_sms * traj_per_sm(smem));
-    k_traj<<<grid, 256, smem, st>>>(dwork, nwork, ddits, maxcreg, dsamples, ddump, devents,
-                                    max_events, nullptr, 0, 0);
+    int grid = std::min(nwork, ctx->num_sms * traj_per_sm(nmax, smem));
+    kernel<<<grid, threads, smem, st>>>(dwork, nwork, ddits, maxcreg, dsamples, ddump, devents,
+                                        max_events, nullptr, 0, 0);
     after_launch(ctx, "k_traj");
 }
 

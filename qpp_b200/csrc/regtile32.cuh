@@ -16,10 +16,15 @@ __device__ __forceinline__ uint32_t rt_swz32_dev(uint32_t e) {
     return e ^ ((h & 7u) << 1);
 }
 
-// The product and the sum in one rounding order everywhere: re = a.x b.x then
-// - a.y b.y, im = a.x b.y then + a.y b.x.
+// The products that begin a gate's sums, with their rounding spelled out so that
+// a gate gives the same bits in every kernel that a seeded shot may run in: of
+// the imaginary part's two terms a.y b.x is rounded and a.x b.y fused in a 4 x 4
+// (c32_mul), the other way round in a 2 x 2 (c32_mul2).
 __device__ __forceinline__ float2 c32_mul(float2 a, float2 b) {
     return make_float2(fmaf(a.x, b.x, -__fmul_rn(a.y, b.y)), fmaf(a.x, b.y, __fmul_rn(a.y, b.x)));
+}
+__device__ __forceinline__ float2 c32_mul2(float2 a, float2 b) {
+    return make_float2(fmaf(a.x, b.x, -__fmul_rn(a.y, b.y)), fmaf(a.y, b.x, __fmul_rn(a.x, b.y)));
 }
 __device__ __forceinline__ float2 c32_fma(float2 a, float2 b, float2 c) {
     c.x = fmaf(a.x, b.x, c.x);
@@ -79,10 +84,10 @@ __device__ __forceinline__ void rt32_put(float2& v, float2 r, bool ok) {
     }
 }
 
-// 4 x 4 (row-major, two entries per float4) on register slots A < B: rows 0
-// and 1 of every group first, then rows 2 and 3, so that half the matrix is
-// held at a time.
-template <int NR, int A, int B, bool CTRL>
+// 4 x 4 (row-major, two entries per float4; COL: column-major) on register slots
+// A < B: rows 0 and 1 of every group first, then rows 2 and 3, so that half the
+// matrix is held at a time.
+template <int NR, int A, int B, bool CTRL, bool COL = false>
 __device__ __forceinline__ void rt32_g2(float2 (&v)[1 << NR], const float4* m, bool lane_ok,
                                         uint32_t rmask, uint32_t rval) {
     if constexpr (B < NR) {
@@ -97,9 +102,9 @@ __device__ __forceinline__ void rt32_g2(float2 (&v)[1 << NR], const float4* m, b
         for (int half = 0; half < 2; ++half) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const float4 e = m[4 * half + k];
-                c[k >> 1][2 * (k & 1)] = make_float2(e.x, e.y);
-                c[k >> 1][2 * (k & 1) + 1] = make_float2(e.z, e.w);
+                const float4 e = m[COL ? half + 2 * k : 4 * half + k];
+                c[COL ? 0 : k >> 1][COL ? k : 2 * (k & 1)] = make_float2(e.x, e.y);
+                c[COL ? 1 : k >> 1][COL ? k : 2 * (k & 1) + 1] = make_float2(e.z, e.w);
             }
 #pragma unroll
             for (int g = 0; g < G; ++g) {
@@ -128,19 +133,20 @@ __device__ __forceinline__ void rt32_g2(float2 (&v)[1 << NR], const float4* m, b
     }
 }
 
-template <int NR, int A, bool CTRL>
+template <int NR, int A, bool CTRL, bool COL = false>
 __device__ __forceinline__ void rt32_g1(float2 (&v)[1 << NR], const float4* m, bool lane_ok,
                                         uint32_t rmask, uint32_t rval) {
     if constexpr (A < NR) {
         const float4 m0 = m[0], m1 = m[1];
-        const float2 a00 = make_float2(m0.x, m0.y), a01 = make_float2(m0.z, m0.w);
-        const float2 a10 = make_float2(m1.x, m1.y), a11 = make_float2(m1.z, m1.w);
+        const float2 e0 = make_float2(m0.x, m0.y), e1 = make_float2(m0.z, m0.w);
+        const float2 e2 = make_float2(m1.x, m1.y), e3 = make_float2(m1.z, m1.w);
+        const float2 a00 = e0, a01 = COL ? e2 : e1, a10 = COL ? e1 : e2, a11 = e3;
 #pragma unroll
         for (int j = 0; j < (1 << NR); ++j) {
             if (j & (1 << A)) continue; // compile-time
             const int j1 = j | (1 << A);
-            const float2 r0 = c32_fma(a01, v[j1], c32_mul(a00, v[j]));
-            const float2 r1 = c32_fma(a11, v[j1], c32_mul(a10, v[j]));
+            const float2 r0 = c32_fma(a01, v[j1], c32_mul2(a00, v[j]));
+            const float2 r1 = c32_fma(a11, v[j1], c32_mul2(a10, v[j]));
             const bool ok = lane_ok && (j & rmask) == rval;
             rt32_put<CTRL>(v[j], r0, ok);
             rt32_put<CTRL>(v[j1], r1, ok);

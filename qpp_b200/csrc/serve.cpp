@@ -362,18 +362,23 @@ Pending launch_batch(qgpu_server* S, qgpu_ctx* ctx, std::vector<Chunk>& batch, P
         // registers above shared-memory size run cache-blocked tile passes
         const int T = tile_width(ctx, int(n));
         std::vector<TProgram> tiled;
-        if (T) {
-            tiled.reserve(cs.size());
-            for (const Chunk& ch : cs) {
-                tiled.push_back(*ch.r->prog);
-                plan_tiles(tiled.back(), T);
-            }
+        std::vector<uint2> noise;
+        std::vector<std::pair<size_t, size_t>> nofs; // (noise offset, steps) per chunk
+        tiled.reserve(cs.size());
+        for (const Chunk& ch : cs) {
+            tiled.push_back(*ch.r->prog);
+            if (T) plan_tiles(tiled.back(), T);
+            plan_sweeps(tiled.back());
+            const std::vector<uint2> ns = noise_steps(tiled.back());
+            nofs.push_back({noise.size(), ns.size()});
+            noise.insert(noise.end(), ns.begin(), ns.end());
         }
         for (size_t ci = 0; ci < cs.size(); ++ci) {
-            const TProgram* P = T ? &tiled[ci] : cs[ci].r->prog;
+            const TProgram* P = &tiled[ci];
             pofs.push_back({ins.size(), mats.size() / 2});
             ins.insert(ins.end(), P->ins.begin(), P->ins.end());
             mats.insert(mats.end(), P->mats.begin(), P->mats.end());
+            mats.resize((mats.size() + 3) / 4 * 4); // every program on a 16-byte boundary
         }
         const uint64_t N = uint64_t(1) << n, nwork = cl.nwork, maxcreg = cl.maxcreg;
         auto al = [](size_t x) { return (x + 255) / 256 * 256; };
@@ -386,8 +391,9 @@ Pending launch_batch(qgpu_server* S, qgpu_ctx* ctx, std::vector<Chunk>& batch, P
                          ? size_t(traj_global_grid(ctx, int(nwork), int(n))) * N * sizeof(float2)
                          : 0;
         size_t b_diag = std::max<size_t>(cl.ndiag * sizeof(double), 16);
+        size_t b_noise = std::max<size_t>(noise.size() * sizeof(uint2), 16);
         size_t total = al(b_ins) + al(b_mat) + al(b_work) + al(b_dits) + al(b_samp) + al(b_g) +
-                       al(b_diag);
+                       al(b_diag) + al(b_noise);
         unsigned char* buf = nullptr;
         QG_CUDA(qgpu::ctx_malloc(ctx, reinterpret_cast<void**>(&buf), total));
         unsigned char* p = buf;
@@ -403,6 +409,7 @@ Pending launch_batch(qgpu_server* S, qgpu_ctx* ctx, std::vector<Chunk>& batch, P
         auto* dsamp = reinterpret_cast<uint64_t*>(take(b_samp));
         auto* dg = reinterpret_cast<float2*>(b_g ? take(b_g) : nullptr);
         auto* ddiag = reinterpret_cast<double*>(take(b_diag));
+        auto* dnoise = reinterpret_cast<uint2*>(take(b_noise));
         std::vector<TWork> work;
         work.reserve(nwork);
         uint32_t out = 0;
@@ -410,7 +417,7 @@ Pending launch_batch(qgpu_server* S, qgpu_ctx* ctx, std::vector<Chunk>& batch, P
         cl.diag_at.assign(cs.size(), 0);
         for (size_t i = 0; i < cs.size(); ++i) {
             const Chunk& ch = cs[i];
-            const TProgram* P = T ? &tiled[i] : ch.r->prog;
+            const TProgram* P = &tiled[i];
             const bool rho = ch.r->kind != QGPU_KET;
             const uint64_t nw = rho ? 1 : ch.ns;
             for (uint64_t k = 0; k < nw; ++k) {
@@ -420,6 +427,8 @@ Pending launch_batch(qgpu_server* S, qgpu_ctx* ctx, std::vector<Chunk>& batch, P
                 w.nins = uint32_t(P->ins.size());
                 w.n = uint8_t(n);
                 w.p_noise = rho ? 0.f : float(ch.r->p);
+                w.noise = dnoise + nofs[i].first;
+                w.nnoise = uint32_t(nofs[i].second);
                 w.shot = uint32_t(ch.s0 + k); // the request's own shot index
                 w.out = out++;
                 w.seed = ch.r->seed;
@@ -436,6 +445,9 @@ Pending launch_batch(qgpu_server* S, qgpu_ctx* ctx, std::vector<Chunk>& batch, P
                                 cudaMemcpyHostToDevice, ctx->stream));
         if (!mats.empty())
             QG_CUDA(cudaMemcpyAsync(dmat, mats.data(), mats.size() * sizeof(float),
+                                    cudaMemcpyHostToDevice, ctx->stream));
+        if (!noise.empty())
+            QG_CUDA(cudaMemcpyAsync(dnoise, noise.data(), noise.size() * sizeof(uint2),
                                     cudaMemcpyHostToDevice, ctx->stream));
         QG_CUDA(cudaMemcpyAsync(dwork, work.data(), b_work, cudaMemcpyHostToDevice, ctx->stream));
         QG_CUDA(cudaMemsetAsync(ddits, 0, b_dits, ctx->stream));

@@ -289,6 +289,119 @@ void plan_tiles(TProgram& P, int T, size_t min_run) {
     P.ins.swap(out);
 }
 
+// Gates per sweep: their steps fit in one 32-bit look at the noise window.
+constexpr uint32_t kSweepGates = 24;
+
+void plan_sweeps(TProgram& P) {
+    const int n = int(P.n);
+    std::vector<TInstr> out;
+    out.reserve(P.ins.size() + P.ins.size() / 2 + 1);
+    // the gates [i, e) on bits 0 .. nb - 1, with sweep headers
+    auto sweeps = [&](size_t i, size_t e, int nb) {
+        while (i < e) {
+            // the longest run on four bits whose G2s can all have the slot of b1
+            // below the slot of b0 (a gate's columns are added in that order)
+            uint32_t bits = 0;
+            uint32_t below[32] = {0}; // bits whose slot must be lower
+            size_t j = i;
+            for (; j < e && j - i < kSweepGates; ++j) {
+                const TInstr& I = P.ins[j];
+                if (I.op != kTG1 && I.op != kTCG1 && I.op != kTG2) break;
+                const uint32_t b2 = bits | (1u << I.b0) | (I.op == kTG2 ? 1u << I.b1 : 0u);
+                if (__builtin_popcount(b2) > 4) break;
+                if (I.op == kTG2) {
+                    // b0 above b1, unless b1 is already above b0
+                    if ((below[I.b1] >> I.b0) & 1u) break;
+                    const uint32_t under = below[I.b1] | (1u << I.b1);
+                    below[I.b0] |= under;
+                    for (int b = 0; b < nb; ++b)
+                        if ((below[b] >> I.b0) & 1u) below[b] |= under;
+                }
+                bits = b2;
+            }
+            if (j == i) {
+                out.push_back(P.ins[i++]);
+                continue;
+            }
+            // unused slots: the highest other bits, so that neighbouring threads
+            // stay on neighbouring amplitudes
+            for (int b = nb - 1; b >= 0 && __builtin_popcount(bits) < 4; --b) bits |= 1u << b;
+            int slot[32], s = 0;
+            TInstr H{};
+            H.op = kTSweep;
+            H.b0 = 4;
+            for (uint32_t left = bits; left;)
+                for (int b = 0; b < nb; ++b)
+                    if (((left >> b) & 1u) && !(below[b] & left)) {
+                        slot[b] = s;
+                        H.mat |= uint32_t(b) << (8 * s++);
+                        left &= ~(1u << b);
+                    }
+            H.cmask = uint32_t(j - i);
+            // the common patterns, their slots in gate order
+            bool one = j - i == 4, two = j - i == 2;
+            for (size_t k = i; k < j; ++k) {
+                one = one && P.ins[k].op == kTG1;
+                two = two && P.ins[k].op == kTG2;
+            }
+            int order[4], no = 0;
+            for (size_t k = i; k < j && (one || two); ++k) {
+                if (two) order[no++] = P.ins[k].b1;
+                order[no++] = P.ins[k].b0;
+            }
+            for (int x = 0; x < no; ++x)
+                for (int y = 0; y < x; ++y) no = order[x] == order[y] ? 0 : no;
+            if (no == 4) {
+                H.b1 = one ? kSweep4x1q : kSweep2x2q;
+                H.mat = 0;
+                for (s = 0; s < 4; ++s) {
+                    slot[order[s]] = s;
+                    H.mat |= uint32_t(order[s]) << (8 * s);
+                }
+            }
+            for (size_t k = i; k < j; ++k) H.cval += P.ins[k].flags & kTNewStep;
+            out.push_back(H);
+            for (; i < j; ++i) {
+                TInstr I = P.ins[i];
+                const int a = I.op == kTG2 ? slot[I.b1] : slot[I.b0];
+                I.flags = uint8_t(I.flags | a << 2 | (I.op == kTG2 ? slot[I.b0] << 4 : 0));
+                out.push_back(I);
+            }
+        }
+    };
+    for (size_t i = 0; i < P.ins.size();) {
+        const TInstr I = P.ins[i];
+        if (I.op == kTTile) {
+            const size_t at = out.size(), m = I.cmask;
+            out.push_back(I);
+            sweeps(i + 1, i + 1 + m, int(I.b0));
+            out[at].cmask = uint32_t(out.size() - at - 1);
+            i += 1 + m;
+        } else if (n >= 4 && n <= kTrajMaxQubits) {
+            size_t e = i;
+            while (e < P.ins.size() && P.ins[e].op != kTTile) ++e;
+            sweeps(i, e, n);
+            i = e;
+        } else {
+            out.push_back(I);
+            ++i;
+        }
+    }
+    P.ins.swap(out);
+}
+
+std::vector<uint2> noise_steps(const TProgram& P) {
+    std::vector<uint2> r;
+    uint32_t alive = P.n >= 32 ? 0xffffffffu : (1u << P.n) - 1, orig = 0;
+    for (const TInstr& I : P.ins) {
+        if (I.op == kTTile || I.op == kTSweep) continue;
+        if (I.flags & kTNewStep) r.push_back(make_uint2(orig, alive));
+        if (I.op == kTMeas && (I.flags & kTDestructive)) alive &= ~(1u << I.b0);
+        ++orig;
+    }
+    return r;
+}
+
 namespace {
 std::mutex g_tile_mu;
 std::map<std::pair<int, int>, int> g_tile_chosen; // (device, n) -> T
@@ -379,7 +492,8 @@ std::vector<float> time_forms(qgpu_ctx* ctx, int n, const std::vector<std::pair<
     } ev{e0, e1};
     std::vector<float> out;
     for (const auto& f : forms) {
-        const TProgram& Q = f.first;
+        TProgram Q = f.first;
+        plan_sweeps(Q); // as the programs run
         const int T = f.second;
         if (Q.ins.size() > 4096 || Q.mats.size() * sizeof(float) > b_mat) {
             out.push_back(-1.f);
@@ -663,6 +777,8 @@ extern "C" qgpu_status qgpu_trajectories(qgpu_ctx* ctx, qgpu_circuit* c, double 
         if (shots == 0) raise(QGPU_ERR_OUT_OF_RANGE, W, "shots");
         const int T = qgpu::tile_width(ctx, int(P.n));
         qgpu::plan_tiles(P, T);
+        qgpu::plan_sweeps(P);
+        const std::vector<uint2> noise = qgpu::noise_steps(P);
         const uint32_t maxcreg = std::max<uint32_t>(P.ncreg, 1);
         const uint64_t N = uint64_t(1) << P.n;
         // device buffers: program, matrices, work, outputs
@@ -670,6 +786,7 @@ extern "C" qgpu_status qgpu_trajectories(qgpu_ctx* ctx, qgpu_circuit* c, double 
         size_t b_mat = std::max<size_t>(P.mats.size() * sizeof(float), 8);
         size_t b_work = shots * sizeof(qgpu::TWork);
         size_t b_dits = shots * maxcreg * sizeof(uint32_t);
+        size_t b_noise = std::max<size_t>(noise.size() * sizeof(uint2), 8);
         size_t b_samp = shots * sizeof(uint64_t);
         size_t b_dump = dump ? shots * N * sizeof(float2) : 0;
         size_t b_ev = events ? shots * size_t(max_events) * sizeof(qgpu::TEvent) : 0;
@@ -679,7 +796,7 @@ extern "C" qgpu_status qgpu_trajectories(qgpu_ctx* ctx, qgpu_circuit* c, double 
                          : 0;
         auto al = [](size_t x) { return (x + 255) / 256 * 256; };
         size_t total = al(b_ins) + al(b_mat) + al(b_work) + al(b_dits) + al(b_samp) + al(b_dump) +
-                       al(b_ev) + al(b_g);
+                       al(b_ev) + al(b_g) + al(b_noise);
         unsigned char* buf = nullptr;
         QG_CUDA(qgpu::ctx_malloc(ctx, reinterpret_cast<void**>(&buf), total));
         unsigned char* p = buf;
@@ -696,6 +813,7 @@ extern "C" qgpu_status qgpu_trajectories(qgpu_ctx* ctx, qgpu_circuit* c, double 
         auto* ddump = reinterpret_cast<float2*>(dump ? take(b_dump) : nullptr);
         auto* dev = reinterpret_cast<qgpu::TEvent*>(events ? take(b_ev) : nullptr);
         auto* dg = reinterpret_cast<float2*>(b_g ? take(b_g) : nullptr);
+        auto* dnoise = reinterpret_cast<uint2*>(take(b_noise));
         std::vector<qgpu::TWork> work(shots);
         for (uint64_t s = 0; s < shots; ++s) {
             qgpu::TWork w{};
@@ -704,6 +822,8 @@ extern "C" qgpu_status qgpu_trajectories(qgpu_ctx* ctx, qgpu_circuit* c, double 
             w.nins = uint32_t(P.ins.size());
             w.n = uint8_t(P.n);
             w.p_noise = float(p_depol);
+            w.noise = dnoise;
+            w.nnoise = uint32_t(noise.size());
             w.shot = uint32_t(s);
             w.out = uint32_t(s);
             w.seed = seed;
@@ -712,6 +832,9 @@ extern "C" qgpu_status qgpu_trajectories(qgpu_ctx* ctx, qgpu_circuit* c, double 
         QG_CUDA(cudaMemcpyAsync(dins, P.ins.data(), b_ins, cudaMemcpyHostToDevice, ctx->stream));
         if (!P.mats.empty())
             QG_CUDA(cudaMemcpyAsync(dmat, P.mats.data(), P.mats.size() * sizeof(float),
+                                    cudaMemcpyHostToDevice, ctx->stream));
+        if (!noise.empty())
+            QG_CUDA(cudaMemcpyAsync(dnoise, noise.data(), noise.size() * sizeof(uint2),
                                     cudaMemcpyHostToDevice, ctx->stream));
         QG_CUDA(cudaMemcpyAsync(dwork, work.data(), b_work, cudaMemcpyHostToDevice, ctx->stream));
         QG_CUDA(cudaMemsetAsync(ddits, 0, b_dits, ctx->stream));

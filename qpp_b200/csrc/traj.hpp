@@ -17,8 +17,19 @@ namespace qgpu {
 // bits listed (one 32-bit word each, ascending, bits 0..4 first) at float2
 // offset `mat` of the matrix pool, with their bit positions renumbered
 // within that list
-enum : uint8_t { kTG1 = 1, kTG2 = 2, kTCG1 = 3, kTMeas = 4, kTG4 = 5, kTTile = 6, kTG3 = 7 };
+// kTSweep: sweep header (plan_sweeps): the next `cmask` instructions are G1, CG1
+// and G2 gates on the four bits packed in `mat` (8 bits each, slot 0 lowest),
+// `cval` of them starting a step; their flags hold the slots of their bits, b1
+// says whether they are one of the common patterns
+enum : uint8_t {
+    kTG1 = 1, kTG2 = 2, kTCG1 = 3, kTMeas = 4, kTG4 = 5, kTTile = 6, kTG3 = 7, kTSweep = 8
+};
+// flags: bits 2-3 the slot of a sweep's G1 / CG1 bit, or of a G2's b1; bits 4-5
+// the (higher) slot of a G2's b0
 enum : uint8_t { kTNewStep = 1, kTDestructive = 2 };
+// kSweep4x1q: four G1 on slots 0, 1, 2, 3; kSweep2x2q: two G2 on slots (0, 1) and
+// (2, 3)
+enum : uint8_t { kSweepAny = 0, kSweep4x1q = 1, kSweep2x2q = 2 };
 
 // One instruction; qubits are bit positions (LSB = 0) of the full register.
 struct TInstr {
@@ -44,6 +55,8 @@ struct TWork {
     uint64_t seed;  // request seed (Philox key)
     const float2* init; // initial register (null: |0...0>)
     float2* fin;        // where the final register goes (null: nowhere)
+    const uint2* noise; // per step that draws noise: untiled instruction index, living qubits
+    uint32_t nnoise;    // (noise_steps; p_noise > 0 needs them)
     double* diag;       // density-matrix run: Re rho(i, i) of the final state
                         // (2^(n/2) values; no basis sample is drawn)
 };
@@ -128,6 +141,14 @@ void set_fusion_width(qgpu_ctx* ctx, int n, int w);
 // min_run: the shortest run that becomes a pass (2 by default; 1 turns
 // every gate into a pass, as the layer-synchronous batches need).
 void plan_tiles(TProgram& P, int T, size_t min_run = 2);
+// Groups runs of G1, CG1 and G2 gates of a (tiled) program into sweeps of at
+// most four bits (kTSweep headers; inside a tile pass its count grows by them):
+// in program order, so the products and their order stay. Registers of four and
+// more qubits that are in shared memory, and tile passes; other instructions
+// stay as they are. Last step before upload.
+void plan_sweeps(TProgram& P);
+// The noise steps of a program, in order (TWork::noise).
+std::vector<uint2> noise_steps(const TProgram& P);
 
 // One register's tile pass in a layer-synchronous launch: items
 // [first_item, first_item + ceil(2^(n-T) / tiles_per_item)) of the launch

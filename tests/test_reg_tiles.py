@@ -1,4 +1,4 @@
-"""Complex128 register tile passes, checked on the CPU: the planned programs
+"""Register tile passes, checked on the CPU: the planned programs
 run on a host model of the kernel give the gate-by-gate result
 (tests/cpp/test_reg_tiles.cpp)."""
 import os
