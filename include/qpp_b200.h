@@ -401,8 +401,10 @@ qgpu_status qgpu_circuit_info(const qgpu_circuit* c, uint32_t* nq,
                               uint64_t* n_steps);
 /* Qudits, their dimension and the classical dits of a circuit. */
 qgpu_status qgpu_circuit_shape(const qgpu_circuit* c, uint32_t* nq, uint64_t* d, uint32_t* nc);
-/* Number of state passes of the fused plan with blocks of <= max_k qubits
- * (host-side planning only). */
+/* Number of state passes of the greedy fused plan with blocks of <= max_k
+ * qubits, each closed by the first gate that does not fit (host-side planning
+ * only; the 6-qubit forms of qgpu_run_gates fill their blocks better and take
+ * fewer). */
 qgpu_status qgpu_circuit_fuse(qgpu_circuit* c, uint32_t max_k,
                               uint64_t* n_passes);
 

@@ -645,8 +645,9 @@ class Circuit:
         return n.value
 
     def fused_passes(self, max_k=6):
-        """Entries of the fused plan with blocks of <= max_k qubits: the
-        merged blocks and the steps left as they are (host planning only)."""
+        """Entries of the greedy fused plan with blocks of <= max_k qubits: the
+        merged blocks and the steps left as they are (host planning only; the
+        6-qubit forms of run() fill their blocks better and take fewer)."""
         n = ct.c_uint64()
         check(lib().qgpu_circuit_fuse(self.h, ct.c_uint32(max_k), ct.byref(n)))
         return n.value

@@ -6,6 +6,7 @@
 #include <functional>
 #include <map>
 
+#include "bit_sets.hpp"
 #include "kernels.hpp"
 #include "ops.hpp"
 #include "reg_tiles.hpp"
@@ -235,6 +236,107 @@ std::vector<Block> fuse(const std::vector<Step>& steps, uint32_t nq, uint32_t ma
     return plan;
 }
 
+std::vector<Block> fuse_wide(const std::vector<Step>& steps, uint32_t nq, uint32_t max_k) {
+    std::vector<Block> plan;
+    struct Dense {
+        std::vector<int> q; // qubits, most significant first
+        std::vector<cd> U;
+    };
+    std::vector<Dense> gates;
+    std::vector<Waiting> wait;
+    // blocks of the gates collected since the last step that stays as it is
+    auto emit = [&] {
+        while (!wait.empty()) {
+            uint64_t all = 0;
+            for (const Waiting& w : wait) all |= w.a;
+            const uint64_t S = __builtin_popcountll(all) <= int(max_k)
+                                   ? all
+                                   : choose_bits(wait, 0, all, int(max_k), true);
+            std::vector<const Dense*> in;
+            uint64_t behind = 0, used = 0;
+            size_t keep = 0;
+            for (const Waiting& w : wait) {
+                if (!(w.t & ~S) && !(w.a & behind)) {
+                    in.push_back(&gates[w.id]);
+                    used |= w.t;
+                } else {
+                    behind |= w.a;
+                    wait[keep++] = w;
+                }
+            }
+            wait.resize(keep);
+            Block b;
+            for (uint32_t q = 0; q < nq; ++q)
+                if ((used >> q) & 1u) b.qubits.push_back(int(q));
+            const int kb = int(b.qubits.size());
+            const uint64_t D = uint64_t(1) << kb;
+            // the product, its rows as separate real and imaginary arrays
+            std::vector<double> M(2 * D * D, 0.0), X;
+            for (uint64_t j = 0; j < D; ++j) M[2 * j * D + j] = 1.0;
+            for (const Dense* g : in) { // rows of G times the product so far
+                const int kg = int(g->q.size());
+                const uint64_t Dg = uint64_t(1) << kg;
+                std::vector<uint64_t> off(Dg, 0);
+                uint64_t mask = 0;
+                for (int j = 0; j < kg; ++j) {
+                    const uint64_t bit =
+                        uint64_t(1) << (kb - 1 - int(std::find(b.qubits.begin(), b.qubits.end(), g->q[size_t(j)]) -
+                                                     b.qubits.begin()));
+                    mask |= bit;
+                    for (uint64_t i = 0; i < Dg; ++i)
+                        if ((i >> (kg - 1 - j)) & 1u) off[i] |= bit;
+                }
+                X.resize(2 * D * Dg);
+                for (uint64_t r = 0; r < D; ++r) {
+                    if (r & mask) continue;
+                    for (uint64_t i = 0; i < Dg; ++i)
+                        std::copy_n(M.data() + 2 * D * (r | off[i]), 2 * D, X.data() + 2 * D * i);
+                    for (uint64_t i = 0; i < Dg; ++i) {
+                        double* const re = M.data() + 2 * D * (r | off[i]);
+                        double* const im = re + D;
+                        std::fill_n(re, 2 * D, 0.0);
+                        for (uint64_t j = 0; j < Dg; ++j) {
+                            const double ur = g->U[i + Dg * j].real(), ui = g->U[i + Dg * j].imag();
+                            const double* const xr = X.data() + 2 * D * j;
+                            const double* const xi = xr + D;
+#pragma omp simd
+                            for (uint64_t c = 0; c < D; ++c) {
+                                re[c] += ur * xr[c] - ui * xi[c];
+                                im[c] += ur * xi[c] + ui * xr[c];
+                            }
+                        }
+                    }
+                }
+            }
+            b.U.resize(D * D);
+            for (uint64_t c = 0; c < D; ++c)
+                for (uint64_t r = 0; r < D; ++r) b.U[r + c * D] = cd(M[2 * D * r + c], M[2 * D * r + D + c]);
+            plan.push_back(std::move(b));
+        }
+        gates.clear();
+    };
+    for (size_t i = 0; i < steps.size(); ++i) {
+        Dense d;
+        if (!step_dense(steps[i], max_k, d.q, d.U)) {
+            emit();
+            Block pass;
+            pass.step = int(i);
+            plan.push_back(pass);
+            continue;
+        }
+        Waiting w;
+        w.t = 0;
+        for (int q : d.q) w.t |= uint64_t(1) << q;
+        w.a = w.t;
+        w.id = uint32_t(gates.size());
+        w.weight = uint32_t(d.q.size());
+        wait.push_back(w);
+        gates.push_back(std::move(d));
+    }
+    emit();
+    return plan;
+}
+
 void apply_step(qgpu_state* s, const Step& st) {
     auto shift_inv = [&](uint64_t d) {
         std::vector<uint64_t> r(st.ctrl.size(), 0);
@@ -311,7 +413,7 @@ static void prepare_plan(qgpu_state* s, qgpu_circuit* c, uint32_t k) {
     // block images held by another device are rebuilt on this one
     if (c->dB && c->dB_dev != s->ctx->device) c->plan_k = 0;
     if (c->plan_k != k) {
-        c->plan = fuse(c->steps, c->nq, k);
+        c->plan = k > 3 && c->nq <= 64 ? fuse_wide(c->steps, c->nq, k) : fuse(c->steps, c->nq, k);
         c->plan_k = k;
         free_image(c->dB, c->dB_dev);
         c->block_slot.clear();
@@ -408,7 +510,7 @@ static bool rho_tc_prepare(qgpu_state* s, qgpu_circuit* c) {
         std::vector<Step> vsteps;
         c->rho_tc_ok = rho_virtual_steps(c, vsteps);
         if (c->rho_tc_ok) {
-            c->rho_plan = fuse(vsteps, 2 * c->nq, 6);
+            c->rho_plan = fuse_wide(vsteps, 2 * c->nq, 6);
             for (const Block& b : c->rho_plan)
                 if (b.step >= 0) c->rho_tc_ok = false; // every virtual step is a gate
         }

@@ -124,6 +124,15 @@ std::vector<cd> embed(const std::vector<cd>& G, const std::vector<int>& gq,
 std::vector<Block> fuse(const std::vector<Step>& steps, uint32_t nq,
                         uint32_t max_k);
 
+// The wide blocks of the tensor-core forms (qubits numbered below 64): each block
+// takes the max_k qubits on which the most waiting gates can run (bit_sets.hpp)
+// and those gates, so it is full where fuse's blocks, closed by the first gate
+// that does not fit, are not: 1800 gates on 30 qubits in 110 blocks of <= 6
+// instead of 179; 336 on 28 qubits in 21 instead of 32 (28.5 -> 18.4 ms, first
+// run 39.9 -> 27.8 ms), 6 noisy layers on a 12-qubit density matrix in 20 instead
+// of 28 (1.55 -> 1.12 ms).
+std::vector<Block> fuse_wide(const std::vector<Step>& steps, uint32_t nq, uint32_t max_k);
+
 // Runs the unitary steps [first, first + count) of `c` on `s`:
 // form 0 = plain (one pass per qpp call), form 1 = fused blocks.
 void run_gates(qgpu_state* s, qgpu_circuit* c, int form, uint64_t first,

@@ -5,6 +5,8 @@
 // qengine.hpp:551-578 -> apply / applyCTRL).
 #include "reg_tiles.hpp"
 
+#include "bit_sets.hpp"
+
 #include <algorithm>
 #include <complex>
 #include <cstring>
@@ -29,62 +31,6 @@ namespace {
 // tables, the gate and its coefficients.
 constexpr size_t kGateBytes[3] = {0, 3 * sizeof(RtOp) + 2 * sizeof(RtLayoutTab) + 64,
                                   4 * sizeof(RtOp) + 2 * sizeof(RtLayoutTab) + 512};
-
-// A gate waiting to be placed: its target bits and all its bits (targets and
-// controls).
-struct Waiting {
-    uint64_t t, a;
-    uint32_t id;
-    uint32_t weight;
-};
-
-// The gates that a pass (or a stretch of it inside a warp) on the bits S can
-// take: in order, every gate whose targets lie in S and which shares no bit
-// with an earlier gate left behind.
-uint32_t reach(const std::vector<Waiting>& g, uint64_t S, uint64_t all) {
-    uint64_t behind = 0;
-    uint32_t sum = 0;
-    for (const Waiting& x : g) {
-        if (!(x.t & ~S) && !(x.a & behind)) {
-            sum += x.weight;
-        } else {
-            behind |= x.a;
-            if (behind == all) break;
-        }
-    }
-    return sum;
-}
-
-// The set of `size` bits (those of `fixed` among them, out of `pool`) whose
-// reach is large: grown in gate order, then improved by trading one bit at a
-// time. Trading costs the bits in times the bits out evaluations of a few
-// dozen gates each; on 1100 random gates of 20 qubits it saves a fifth of the
-// passes that growing alone needs.
-uint64_t choose_bits(const std::vector<Waiting>& g, uint64_t fixed, uint64_t pool, int size) {
-    uint64_t all = 0, S = fixed, behind = 0;
-    for (const Waiting& x : g) all |= x.a;
-    for (const Waiting& x : g) {
-        if (!(x.a & behind) && __builtin_popcountll(S | x.t) <= size) S |= x.t;
-        else if ((behind |= x.a) == all) break;
-    }
-    for (uint64_t r = pool & ~S; r && __builtin_popcountll(S) < size; r &= r - 1) S |= r & (0 - r);
-    uint32_t best = reach(g, S, all);
-    for (int round = 0; round < 8; ++round) {
-        uint64_t top = S;
-        for (uint64_t in = S & ~fixed; in; in &= in - 1)
-            for (uint64_t out = pool & all & ~S; out; out &= out - 1) {
-                const uint64_t S2 = (S ^ (in & (0 - in))) | (out & (0 - out));
-                const uint32_t r = reach(g, S2, all);
-                if (r > best) {
-                    best = r;
-                    top = S2;
-                }
-            }
-        if (top == S) break;
-        S = top;
-    }
-    return S;
-}
 
 // Moves the gates that S reaches from g to `out`, in order, at most `most`
 // program bytes of them.
