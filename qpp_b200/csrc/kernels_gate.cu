@@ -329,37 +329,39 @@ __global__ void __launch_bounds__(256)
 }
 
 // Shared-memory variant for any DA: a block owns G groups at a time
-// (G * DA <= blockDim.x when DA <= 256), stages them, then each thread forms
-// output rows. A (column-major, state precision) and off live in global
-// memory and are read through the read-only cache.
+// (G * DA <= blockDim.x when DA <= 256), stages them with their base offsets,
+// then each thread forms output rows. A (column-major, state precision) and off
+// live in global memory and are read through the read-only cache.
 template <typename R>
 __global__ void __launch_bounds__(256)
     k_smem(Cplx<R>* __restrict__ psi, const __grid_constant__ SegPlan outer,
            const uint64_t* __restrict__ off, const Cplx<R>* __restrict__ A,
            int DA, int G) {
     using C = Cplx<R>;
-    extern __shared__ unsigned char smem_raw[];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     C* sv = reinterpret_cast<C*>(smem_raw);
+    __shared__ uint64_t gbase[256];
     const int tid = threadIdx.x;
     const int per = G * DA;
     for (uint64_t g0 = uint64_t(blockIdx.x) * G; g0 < outer.count;
          g0 += uint64_t(gridDim.x) * G) {
+        const int ng = int(outer.count - g0 < uint64_t(G) ? outer.count - g0 : uint64_t(G));
+        for (int i = tid; i < ng; i += blockDim.x) gbase[i] = seg_offset(outer, g0 + i);
+        __syncthreads();
         for (int e = tid; e < per; e += blockDim.x) {
-            uint64_t g = g0 + e / DA;
-            if (g < outer.count)
-                sv[e] = psi[seg_offset(outer, g) + __ldg(&off[e % DA])];
+            const int gl = e / DA;
+            if (gl < ng) sv[e] = psi[gbase[gl] + __ldg(&off[e - gl * DA])];
         }
         __syncthreads();
         for (int e = tid; e < per; e += blockDim.x) {
-            int gl = e / DA, m = e % DA;
-            uint64_t g = g0 + gl;
-            if (g < outer.count) {
+            const int gl = e / DA, m = e - gl * DA;
+            if (gl < ng) {
                 const C* v = sv + gl * DA;
                 C acc;
                 acc.x = 0;
                 acc.y = 0;
                 for (int c = 0; c < DA; ++c) acc = cfma(A[m + size_t(c) * DA], v[c], acc);
-                psi[seg_offset(outer, g) + __ldg(&off[m])] = acc;
+                psi[gbase[gl] + __ldg(&off[m])] = acc;
             }
         }
         __syncthreads();
@@ -444,9 +446,9 @@ static void reg(qgpu_ctx* ctx, void* data, const SegPlan& outer,
     p.outer = outer;
     for (int i = 0; i < DA; ++i) p.off[i] = off[i];
     for (int i = 0; i < DA * DA; ++i) p.A[i] = cv<R>(A[i]);
-    int blocks = grid_blocks(ctx, 4);
-    uint64_t need = (outer.count + 255) / 256;
-    if (need < uint64_t(blocks)) blocks = int(std::max<uint64_t>(need, 1));
+    // one group per thread over the whole state, as for one-qubit gates
+    const unsigned blocks =
+        unsigned(std::min<uint64_t>(std::max<uint64_t>((outer.count + 255) / 256, 1), 0x7fffffffu));
     k_reg<R, DA><<<blocks, 256, 0, ctx->stream>>>(static_cast<Cplx<R>*>(data), p);
     after_launch(ctx, "k_reg");
 }
@@ -513,8 +515,12 @@ static void generic(qgpu_ctx* ctx, void* data, const SegPlan& outer,
         case 2: return reg<R, 2>(ctx, data, outer, off, A);
         case 3: return reg<R, 3>(ctx, data, outer, off, A);
         case 4: return reg<R, 4>(ctx, data, outer, off, A);
+        case 5: return reg<R, 5>(ctx, data, outer, off, A);
+        case 6: return reg<R, 6>(ctx, data, outer, off, A);
         case 8: return reg<R, 8>(ctx, data, outer, off, A);
         case 9: return reg<R, 9>(ctx, data, outer, off, A);
+        case 10: return reg<R, 10>(ctx, data, outer, off, A);
+        case 12: return reg<R, 12>(ctx, data, outer, off, A);
         case 16:
             // complex128: two warps per group (a whole 16 x 16 per thread
             // needs over 250 registers)

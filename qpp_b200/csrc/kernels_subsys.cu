@@ -568,6 +568,7 @@ static void plan_gather_fixed(const uint64_t* od, const uint64_t* src, int n, Se
         while ((uint64_t(1) << sh) < p.size[s]) ++sh;
         p.shift[s] = uint8_t(sh);
     }
+    seg_magic(p);
 }
 
 template <typename R>

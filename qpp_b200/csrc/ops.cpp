@@ -61,6 +61,7 @@ static void finish_plan(SegPlan& p) {
         while ((uint64_t(1) << sh) < z) ++sh;
         p.shift[s] = uint8_t(sh);
     }
+    seg_magic(p);
 }
 
 SegPlan plan_free(const VSpace& vs, const std::vector<int>& excluded,
