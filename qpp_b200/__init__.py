@@ -80,6 +80,38 @@ def lib():
     return _lib
 
 
+_U64, _U32, _INT = ct.c_uint64, ct.c_uint32, ct.c_int
+# Argument types of the entry points that programs call gate by gate or step by
+# step: with them ctypes takes Python ints, bytes and arrays as they are (a pointer
+# or integer object built per argument costs 1-2 us, and these calls 2-3 us each
+# beside them).
+_ARGS = {
+    "qgpu_apply": (vp, vp, _U64, vp, _U32),
+    "qgpu_apply_ctrl": (vp, vp, _U64, vp, _U32, vp, _U32, vp),
+    "qgpu_apply_ctrl_fan": (vp, vp, _U64, vp, _U32, vp, _U32, vp),
+    "qgpu_apply_kraus": (vp, vp, _U32, _U64, vp, _U32),
+    "qgpu_ptrace": (vp, vp, _U32, vp),
+    "qgpu_ptranspose": (vp, vp, _U32, vp),
+    "qgpu_syspermute": (vp, vp, _U32, vp),
+    "qgpu_apply_qft": (vp, vp, _U32, _U64, _INT, _INT),
+    "qgpu_state_info": (vp, vp, vp, vp, vp, vp),
+    "qgpu_circuit_gate": (vp, vp, _U64, vp, _U32),
+    "qgpu_circuit_ctrl": (vp, vp, _U64, vp, _U32, vp, _U32, vp, _INT),
+}
+_typed = {}
+
+
+def _fn(name):
+    """The entry point with its argument types (an object of its own: lib()'s
+    attributes take whatever ctypes makes of their arguments)."""
+    f = _typed.get(name)
+    if f is None:
+        f = lib()[name]
+        f.argtypes, f.restype = _ARGS[name], _INT
+        _typed[name] = f
+    return f
+
+
 def check(rc):
     if rc != 0:
         L = lib()
@@ -96,6 +128,32 @@ def _u64(v):
         a = np.zeros(1, dtype=np.uint64)
         return a, a.ctypes.data_as(u64p), 0
     return a, a.ctypes.data_as(u64p), a.size
+
+
+_U64_ARRAYS = {}
+
+
+def _ix(v):
+    """Subsystem indices for a typed entry point: (array, count)."""
+    if v is None:
+        return None, 0
+    if type(v) is not list:
+        v = list(v)
+    for x in v:
+        if type(x) is not int or x < 0 or x > 0xffffffffffffffff:
+            a, _, n = _u64(v)  # numpy's conversions, and its errors
+            return (_U64 * max(n, 1))(*(int(y) for y in a[: max(n, 1)])), n
+    n = len(v)
+    T = _U64_ARRAYS.get(n)
+    if T is None:
+        T = _U64_ARRAYS[n] = _U64 * max(n, 1)
+    return T(*v), n
+
+
+def _gate(A):
+    """A matrix for a typed entry point: (its column-major complex128 bytes, rows)."""
+    A = np.asarray(A, dtype=np.complex128)
+    return A.tobytes("F"), A.shape[0] if A.ndim else 1
 
 
 def _mat(A):
@@ -157,7 +215,7 @@ def default_context():
 class State:
     """A ket (kind=KET) or density matrix (kind=RHO) resident in HBM."""
 
-    def __init__(self, ctx, kind, dims, prec=C128, handle=None):
+    def __init__(self, ctx, kind, dims, prec=C128, handle=None, most_dims=None):
         self.ctx = ctx
         if handle is None:
             handle = vp()
@@ -165,16 +223,20 @@ class State:
             check(lib().qgpu_state_create(ctx.h, ct.c_int(kind), ct.c_int(prec), dpp,
                                           ct.c_uint32(nd), ct.byref(handle)))
         self.h = handle
-        self._info()
+        self._info(most_dims)
 
-    def _info(self):
+    def _info(self, most_dims):
+        # most_dims: a bound on the state's subsystems, where the caller knows one
+        # (one call instead of two)
         k, p, n, D = ct.c_int(), ct.c_int(), ct.c_uint32(), ct.c_uint64()
-        check(lib().qgpu_state_info(self.h, ct.byref(k), ct.byref(p), ct.byref(n), None,
-                                    ct.byref(D)))
-        dims = np.zeros(max(n.value, 1), dtype=np.uint64)
-        check(lib().qgpu_state_info(self.h, None, None, None, dims.ctypes.data_as(u64p), None))
+        info = _fn("qgpu_state_info")
+        if most_dims is None:
+            check(info(self.h, None, None, ct.byref(n), None, None))
+            most_dims = n.value
+        dims = (_U64 * max(most_dims, 1))()
+        check(info(self.h, ct.byref(k), ct.byref(p), ct.byref(n), dims, ct.byref(D)))
         self.kind, self.prec, self.D = k.value, p.value, D.value
-        self.dims = [int(x) for x in dims[: n.value]]
+        self.dims = dims[: n.value]
 
     @classmethod
     def from_numpy(cls, ctx, arr, dims, prec=C128):
@@ -212,58 +274,50 @@ class State:
 
     # resident (in-place) ops
     def apply(self, A, target):
-        A = _mat(A)
-        t, tp, nt = _u64(target)
-        check(lib().qgpu_apply(self.h, _dp(A), ct.c_uint64(A.shape[0]), tp, ct.c_uint32(nt)))
+        A, rows = _gate(A)
+        t, nt = _ix(target)
+        check(_fn("qgpu_apply")(self.h, A, rows, t, nt))
         return self
 
     def apply_ctrl(self, A, ctrl, target, shift=None, fan=False):
-        A = _mat(A)
-        c, cp, nc = _u64(ctrl)
-        t, tp, nt = _u64(target)
-        s, sp, _ = _u64(shift)
-        fn = lib().qgpu_apply_ctrl_fan if fan else lib().qgpu_apply_ctrl
-        check(fn(self.h, _dp(A), ct.c_uint64(A.shape[0]), cp, ct.c_uint32(nc), tp,
-                 ct.c_uint32(nt), sp))
+        A, rows = _gate(A)
+        c, nc = _ix(ctrl)
+        t, nt = _ix(target)
+        s, _ = _ix(shift)
+        check(_fn("qgpu_apply_ctrl_fan" if fan else "qgpu_apply_ctrl")(self.h, A, rows, c, nc, t, nt, s))
         return self
 
     def apply_kraus(self, Ks, target):
         packed, DA = _pack_kraus(Ks)
-        t, tp, nt = _u64(target)
-        check(lib().qgpu_apply_kraus(self.h, _dp(packed), ct.c_uint32(len(Ks)),
-                                     ct.c_uint64(DA), tp, ct.c_uint32(nt)))
+        t, nt = _ix(target)
+        check(_fn("qgpu_apply_kraus")(self.h, packed.tobytes(), len(Ks), DA, t, nt))
         return self
 
-    def ptrace(self, target):
-        t, tp, nt = _u64(target)
+    def _new(self, name, kind, subsystems):
+        t, nt = _ix(subsystems)
         h = vp()
-        check(lib().qgpu_ptrace(self.h, tp, ct.c_uint32(nt), ct.byref(h)))
-        return State(self.ctx, RHO, None, handle=h)
+        check(_fn(name)(self.h, t, nt, ct.byref(h)))
+        return State(self.ctx, kind, None, handle=h, most_dims=len(self.dims))
+
+    def ptrace(self, target):
+        return self._new("qgpu_ptrace", RHO, target)
 
     def ptranspose(self, target):
-        t, tp, nt = _u64(target)
-        h = vp()
-        check(lib().qgpu_ptranspose(self.h, tp, ct.c_uint32(nt), ct.byref(h)))
-        return State(self.ctx, RHO, None, handle=h)
+        return self._new("qgpu_ptranspose", RHO, target)
 
     def syspermute(self, perm):
-        p, pp, npm = _u64(perm)
-        h = vp()
-        check(lib().qgpu_syspermute(self.h, pp, ct.c_uint32(npm), ct.byref(h)))
-        return State(self.ctx, self.kind, None, handle=h)
+        return self._new("qgpu_syspermute", self.kind, perm)
 
     def apply_qft(self, target, d=2, swap=True):
         """qpp::applyQFT on the resident state, in place."""
-        t, tp, nt = _u64(target)
-        check(lib().qgpu_apply_qft(self.h, tp, ct.c_uint32(nt), ct.c_uint64(d),
-                                   ct.c_int(int(swap)), ct.c_int(0)))
+        t, nt = _ix(target)
+        check(_fn("qgpu_apply_qft")(self.h, t, nt, _U64(d), int(swap), 0))
         return self
 
     def apply_tfq(self, target, d=2, swap=True):
         """qpp::applyTFQ on the resident state, in place."""
-        t, tp, nt = _u64(target)
-        check(lib().qgpu_apply_qft(self.h, tp, ct.c_uint32(nt), ct.c_uint64(d),
-                                   ct.c_int(int(swap)), ct.c_int(1)))
+        t, nt = _ix(target)
+        check(_fn("qgpu_apply_qft")(self.h, t, nt, _U64(d), int(swap), 1))
         return self
 
     def qft(self, d=2, swap=True, inverse=False):
@@ -388,6 +442,11 @@ class State:
 
 
 def _pack_kraus(Ks):
+    if len(Ks) and all(type(K) is np.ndarray and K.ndim == 2 and K.shape == Ks[0].shape for K in Ks):
+        packed = np.empty((len(Ks), Ks[0].shape[1], Ks[0].shape[0]), dtype=np.complex128)
+        for i, K in enumerate(Ks):
+            packed[i] = K.T
+        return packed.reshape(-1), Ks[0].shape[0]
     Ks = [_mat(K) for K in Ks]
     if not Ks:
         return np.zeros(1, dtype=np.complex128), 0
@@ -541,9 +600,9 @@ class Circuit:
         self.nq, self.d, self.nc = nq, d, nc
 
     def gate(self, U, target):
-        U = _mat(U)
-        t, tp, nt = _u64(target)
-        check(lib().qgpu_circuit_gate(self.h, _dp(U), ct.c_uint64(U.shape[0]), tp, ct.c_uint32(nt)))
+        U, rows = _gate(U)
+        t, nt = _ix(target)
+        check(_fn("qgpu_circuit_gate")(self.h, U, rows, t, nt))
         return self
 
     def gate_fan(self, U, target):
@@ -554,12 +613,11 @@ class Circuit:
         return self
 
     def CTRL(self, U, ctrl, target, shift=None, fan=False):
-        U = _mat(U)
-        c, cp, nc = _u64(ctrl)
-        t, tp, nt = _u64(target)
-        s, sp, _ = _u64(shift)
-        check(lib().qgpu_circuit_ctrl(self.h, _dp(U), ct.c_uint64(U.shape[0]), cp, ct.c_uint32(nc),
-                                      tp, ct.c_uint32(nt), sp, ct.c_int(1 if fan else 0)))
+        U, rows = _gate(U)
+        c, nc = _ix(ctrl)
+        t, nt = _ix(target)
+        s, _ = _ix(shift)
+        check(_fn("qgpu_circuit_ctrl")(self.h, U, rows, c, nc, t, nt, s, 1 if fan else 0))
         return self
 
     def cCTRL(self, U, ctrl_dits, target, shift=None, fan=False):
