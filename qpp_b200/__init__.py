@@ -858,8 +858,8 @@ class Engine:
         outs = np.zeros(max(n.value * nc, 1), dtype=np.uint64)
         check(lib().qgpu_engine_get_stats(self.h, None, counts.ctypes.data_as(u64p),
                                           outs.ctypes.data_as(u64p)))
-        return {tuple(int(x) for x in outs[i * nc:(i + 1) * nc]): int(counts[i])
-                for i in range(n.value)}
+        rows = outs[: n.value * nc].reshape(n.value, nc).tolist()
+        return dict(zip(map(tuple, rows), counts[: n.value].tolist()))
 
     def get_record(self):
         no, nn = ct.c_uint64(), ct.c_uint64()

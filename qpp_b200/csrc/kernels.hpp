@@ -227,6 +227,19 @@ std::vector<uint64_t> prefix_search_many(qgpu_ctx* ctx, qgpu_prec prec, const vo
 // Keep the elements whose digit (index / dig_stride) % dig_dim equals
 // dig_val (for rho: in both the row and the column index), scale them by
 // `scale`, zero the rest.
+// A measurement of a ket without a host round trip. launch_measure_draw: the index
+// that prefix_search finds for `fraction`, to *idx; `part` has kMeasureParts +
+// kMeasureParts / 4 doubles, whose first hold the state's chunk sums already when
+// have_sums. launch_measure_collapse: the subsystem of dimension dim and stride
+// `stride` collapses onto its digit in *idx (there with stride stride0): in place,
+// or without that subsystem into `out`; its probability goes to *prob and, with
+// sums, the result's chunk sums to `part` for the next draw.
+constexpr int kMeasureParts = 1184;
+void launch_measure_draw(qgpu_ctx* ctx, qgpu_prec prec, const void* data, uint64_t D, double fraction,
+                         double* part, bool have_sums, unsigned long long* idx);
+void launch_measure_collapse(qgpu_ctx* ctx, qgpu_prec prec, void* data, void* out, uint64_t D,
+                             uint64_t stride, uint64_t dim, uint64_t stride0,
+                             const unsigned long long* idx, double* part, double* prob, bool sums);
 void launch_project(qgpu_ctx* ctx, qgpu_prec prec, void* data, uint64_t n,
                     uint64_t D, bool is_rho, uint64_t dig_stride,
                     uint64_t dig_dim, uint64_t dig_val, double scale);
