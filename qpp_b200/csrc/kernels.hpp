@@ -189,6 +189,37 @@ int qft_pass8_tile_bits(qgpu_prec prec);
 bool qft_pass8_applies(qgpu_prec prec, const void* in, const void* out, const QftPlan& p);
 void qft_pass8_maps(QftPlan& p, int EB);
 
+// A qubit ket's pass of 5 to 10 steps with its tile in registers (k_qft_reg):
+// tiles of 2^12 (complex128) or 2^13 (complex64) amplitudes, 16 or 32 to each of
+// 256 threads. A round holds `g` steps on the tile bits [lo, lo + g), which are the
+// lowest register bits; reg and thr: the tile bits that a thread's register and
+// thread index bits select. Rounds without steps only change the layout, for
+// coalesced reads or writes.
+constexpr int kQftRegThrBits = 8;
+struct QftRegRound {
+    uint8_t g, lo, reg[5], thr[kQftRegThrBits];
+};
+constexpr int kQftRegRounds = 6;
+struct QftRegPlan {
+    uint64_t ntiles;
+    uint64_t odim[kQftMaxOuter], ors[kQftMaxOuter], ows[kQftMaxOuter], ozw[kQftMaxOuter];
+    uint64_t trs[16], tws[16], tzw[16];
+    QftRegRound rd[kQftRegRounds];
+    uint8_t oshift[kQftMaxOuter];
+    int bits, nround, nod, nz, nr, M, a, k, inverse;
+    double scale;
+};
+int qft_reg_tile_bits(qgpu_prec prec);
+// The passes of a ket's transform as k_qft_reg takes them (qft.cpp); false where
+// one of them does not fit, or would read or write runs of less than 64 bytes.
+struct QftRegSchedule {
+    std::vector<QftRegPlan> plans;
+    std::vector<char> fold; // as QftSchedule
+};
+bool plan_qft_reg(qgpu_prec prec, uint64_t D, const std::vector<uint64_t>& target, bool inverse,
+                  bool fold, QftRegSchedule& S);
+void launch_qft_reg(qgpu_ctx* ctx, qgpu_prec prec, const void* in, void* out, const QftRegPlan& p);
+
 // --- reductions and elementwise (kernels_reduce.cu) ----------------------
 // sum |x|^2 over n elements, FP64 accumulation; result to *host_out.
 double reduce_norm2(qgpu_ctx* ctx, qgpu_prec prec, const void* data,

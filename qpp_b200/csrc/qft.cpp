@@ -1,4 +1,4 @@
-// qft.cpp -- planning of qpp::applyQFT / applyTFQ onto k_qft_pass.
+// qft.cpp -- planning of qpp::applyQFT / applyTFQ onto k_qft_pass and k_qft_reg.
 //
 // qpp::applyQFT(A, target, d, swap) (operations.hpp:2565-2676) and applyTFQ
 // (:2680-2787) treat A as n qudits of dimension d. On a ket the transform acts
@@ -104,6 +104,8 @@ void qft_gate_sequence(qgpu_state* s, const std::vector<uint64_t>& target, uint6
             }
     }
 }
+
+constexpr int kQftRegSteps = 10; // steps of a register pass at most
 
 struct PassSpec {
     std::vector<int> group; // virtual digits of targets a .. a + M - 1
@@ -319,8 +321,11 @@ std::vector<cd> qft_roots(uint64_t nW) {
     return W;
 }
 
-bool plan_qft(bool rho, uint64_t D, uint64_t d, size_t elem_bytes,
-              const std::vector<uint64_t>& target, bool inverse, bool fold, QftSchedule& S) {
+// `wide`: tiles of 64 KB and groups of 5 to 10 targets of nearly equal size (the
+// register passes) instead of tiles of 32 KB.
+static bool plan_passes(bool rho, uint64_t D, uint64_t d, size_t elem_bytes,
+                        const std::vector<uint64_t>& target, bool inverse, bool fold, bool wide,
+                        QftSchedule& S) {
     S = QftSchedule();
     const size_t k = target.size();
     if (d > uint64_t(kQftMaxD) || d < 2) return false;
@@ -347,9 +352,10 @@ bool plan_qft(bool rho, uint64_t D, uint64_t d, size_t elem_bytes,
     for (auto& h : halves)
         for (size_t a = 0; a < k; ++a) revmap[size_t(h[a])] = h[k - 1 - a];
 
-    const uint32_t Emax = uint32_t(32768 / elem_bytes), Rt = uint32_t(128 / elem_bytes);
+    const uint32_t Emax = uint32_t((wide ? 65536 : 32768) / elem_bytes), Rt = uint32_t(128 / elem_bytes);
     int Mmax = 0;
     for (uint64_t p = d; p * Rt <= Emax; p *= d) ++Mmax;
+    if (wide) Mmax = kQftRegSteps;
     if (Mmax == 0) return false;
     S.Mmax = Mmax;
     S.nW = 1;
@@ -362,6 +368,10 @@ bool plan_qft(bool rho, uint64_t D, uint64_t d, size_t elem_bytes,
     const size_t npass_half = (k + size_t(Mmax) - 1) / size_t(Mmax);
     const size_t part = d == 2 ? k % size_t(Mmax) : 0;
     auto start = [&](size_t g) {
+        // the larger groups last: with ten targets the tile has room for two other
+        // digits, and runs of 64 bytes cost least where the pass reads a contiguous
+        // tile (28 qubits complex128: 2.46 ms, as the first pass 3.25, the second 2.79)
+        if (wide) return g * k / npass_half;
         if (g == 0) return size_t(0);
         return std::min(k, (part ? part : size_t(Mmax)) + (g - 1) * size_t(Mmax));
     };
@@ -394,6 +404,188 @@ bool plan_qft(bool rho, uint64_t D, uint64_t d, size_t elem_bytes,
     return true;
 }
 
+bool plan_qft(bool rho, uint64_t D, uint64_t d, size_t elem_bytes,
+              const std::vector<uint64_t>& target, bool inverse, bool fold, QftSchedule& S) {
+    return plan_passes(rho, D, d, elem_bytes, target, inverse, fold, false, S);
+}
+
+// The rounds of a register pass: the group's steps four (complex64: five) at a time
+// from the top tile bit down, the remainder on the lowest group bits, whose free
+// register bits lie above it (where the phases do not reach); an inverse pass takes
+// them in the opposite order. A round of steps whose register bits hold one of the
+// three lowest bits of the read (first round) or write order (last round) is
+// preceded or followed by one without steps.
+static bool reg_rounds(const QftPlan& p, int bits, QftRegPlan& q) {
+    const int NR = bits - kQftRegThrBits;
+    std::vector<QftRegRound> rd;
+    auto layout = [&](int g, int lo, const std::vector<int>& reg, const uint64_t* st) {
+        QftRegRound x{};
+        x.g = uint8_t(g);
+        x.lo = uint8_t(lo);
+        std::vector<int> thr;
+        for (int b = 0; b < bits; ++b)
+            if (std::find(reg.begin(), reg.end(), b) == reg.end()) thr.push_back(b);
+        if (st) {
+            std::stable_sort(thr.begin(), thr.end(), [&](int a, int b) { return st[a] < st[b]; });
+        } else {
+            // the lanes that share a wavefront (8 of 16 bytes, 16 of 8) on distinct
+            // banks: tile bits of distinct residues (qft_reg_swz)
+            const int m = bits == 12 ? 3 : 4;
+            for (int i = 0; i < m; ++i)
+                for (size_t j = size_t(i); j < thr.size(); ++j) {
+                    bool fresh = true;
+                    for (int h = 0; h < i; ++h) fresh = fresh && thr[size_t(h)] % m != thr[j] % m;
+                    if (fresh) {
+                        std::rotate(thr.begin() + i, thr.begin() + ptrdiff_t(j), thr.begin() + ptrdiff_t(j) + 1);
+                        break;
+                    }
+                }
+        }
+        for (size_t i = 0; i < reg.size(); ++i) x.reg[i] = uint8_t(reg[i]);
+        for (size_t i = 0; i < thr.size(); ++i) x.thr[i] = uint8_t(thr[i]);
+        return x;
+    };
+    struct Part {
+        int g, lo;
+        std::vector<int> reg;
+    };
+    std::vector<Part> parts;
+    const int top = p.nr + p.M; // == bits
+    for (int hi = top; hi > p.nr;) {
+        Part x;
+        x.g = std::min(NR, hi - p.nr);
+        x.lo = hi - x.g;
+        for (int b = x.lo; int(x.reg.size()) < NR && b < top; ++b) x.reg.push_back(b);
+        if (int(x.reg.size()) < NR) return false;
+        parts.push_back(x);
+        hi = x.lo;
+    }
+    if (p.inverse) std::reverse(parts.begin(), parts.end());
+    auto by = [&](const uint64_t* st) {
+        std::vector<int> o(static_cast<size_t>(bits));
+        std::iota(o.begin(), o.end(), 0);
+        std::stable_sort(o.begin(), o.end(), [&](int a, int b) { return st[a] < st[b]; });
+        return o;
+    };
+    const std::vector<int> ro = by(p.trs), wo = by(p.tws);
+    auto scattered = [&](const Part& x, const std::vector<int>& o) {
+        for (int b : x.reg)
+            for (int i = 0; i < 3; ++i)
+                if (b == o[size_t(i)]) return true;
+        return false;
+    };
+    if (scattered(parts.front(), ro))
+        rd.push_back(layout(0, 0, std::vector<int>(ro.end() - NR, ro.end()), p.trs));
+    const bool tail = scattered(parts.back(), wo);
+    for (size_t i = 0; i < parts.size(); ++i) {
+        const uint64_t* st = nullptr;
+        if (i == 0 && rd.empty()) st = p.trs;
+        else if (i + 1 == parts.size() && !tail) st = p.tws;
+        rd.push_back(layout(parts[i].g, parts[i].lo, parts[i].reg, st));
+    }
+    if (tail) rd.push_back(layout(0, 0, std::vector<int>(wo.end() - NR, wo.end()), p.tws));
+    if (rd.size() < 2 || rd.size() > size_t(kQftRegRounds)) return false;
+    q.nround = int(rd.size());
+    std::copy(rd.begin(), rd.end(), q.rd);
+    return true;
+}
+
+bool plan_qft_reg(qgpu_prec prec, uint64_t D, const std::vector<uint64_t>& target, bool inverse,
+                  bool fold, QftRegSchedule& S) {
+    S = QftRegSchedule();
+    QftSchedule G;
+    const size_t eb = prec == QGPU_C128 ? 16 : 8;
+    if (!plan_passes(false, D, 2, eb, target, inverse, fold, true, G)) return false;
+    const int bits = qft_reg_tile_bits(prec);
+    for (const QftPlan& p : G.plans) {
+        QftRegPlan q;
+        std::memset(&q, 0, sizeof(q));
+        if (p.M < 5 || p.ntd != bits || p.nr + p.M != bits || p.E != 1u << bits) return false;
+        uint64_t rmask = 0, wmask = 0;
+        for (int b = 0; b < bits; ++b) {
+            q.trs[b] = p.trs[b];
+            q.tws[b] = p.tws[b];
+            q.tzw[b] = p.tzw[b];
+            rmask |= p.trs[b];
+            wmask |= p.tws[b];
+        }
+        const uint64_t run = 64 / eb - 1; // the lowest address bits all inside the tile
+        if ((rmask & run) != run || (wmask & run) != run) return false;
+        q.nod = p.nod;
+        for (int o = 0; o < p.nod; ++o) {
+            q.odim[o] = p.odim[o];
+            q.ors[o] = p.ors[o];
+            q.ows[o] = p.ows[o];
+            q.ozw[o] = p.ozw[o];
+            q.oshift[o] = p.oshift[o];
+        }
+        q.ntiles = p.ntiles;
+        q.bits = bits;
+        q.nz = p.nz;
+        q.nr = p.nr;
+        q.M = p.M;
+        q.a = p.a;
+        q.k = p.k;
+        q.inverse = p.inverse;
+        q.scale = p.scale;
+        if (!reg_rounds(p, bits, q)) return false;
+        S.plans.push_back(q);
+    }
+    S.fold = G.fold;
+    return true;
+}
+
+// Tables in the state's precision, staged through the context's scratch.
+static const unsigned char* stage_tables(qgpu_state* s, const std::vector<cd>& tabs) {
+    const size_t eb = s->elem_bytes();
+    unsigned char* dev = static_cast<unsigned char*>(ctx_scratch(s->ctx, tabs.size() * eb));
+    if (s->prec == QGPU_C128) {
+        QG_CUDA(cudaMemcpyAsync(dev, tabs.data(), tabs.size() * eb, cudaMemcpyHostToDevice,
+                                s->ctx->stream));
+    } else {
+        std::vector<float> f(2 * tabs.size());
+        for (size_t i = 0; i < tabs.size(); ++i) {
+            f[2 * i] = float(tabs[i].real());
+            f[2 * i + 1] = float(tabs[i].imag());
+        }
+        QG_CUDA(cudaMemcpyAsync(dev, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice,
+                                s->ctx->stream));
+    }
+    return dev;
+}
+
+// The transform of a qubit ket as register passes; false (nothing done) where they
+// do not apply or the reversal's second buffer does not fit. From 128 MB on, where a
+// pass costs a trip through HBM: 24 qubits complex128 (three passes either way) 428 ->
+// 386 us, 25 qubits (three instead of four) 1104 -> 749 us, complex64 821 -> 418 us.
+// Smaller states stay in the L2 and with the smaller tiles, which fill more SMs.
+static bool qft_reg_run(qgpu_state* s, const std::vector<uint64_t>& target, bool inverse, bool rev) {
+    const size_t k = target.size();
+    if (s->bytes() < (uint64_t(128) << 20) || k < 9) return false;
+    QftRegSchedule S;
+    // groups of ten targets (64-byte runs) cost the gain where there are two in
+    // complex128 (29 qubits 15.8 against 15.6 ms in four smaller passes) or three in
+    // complex64 (30 qubits 16.9 against 14.5 ms; two, 29 qubits: 7.2 against 8.4 ms)
+    const size_t npass = (k + kQftRegSteps - 1) / kQftRegSteps;
+    if (k + npass > npass * kQftRegSteps + (s->prec == QGPU_C128 ? 1 : 2)) return false;
+    if (!plan_qft_reg(s->prec, s->D, target, inverse, rev, S)) return false;
+    void* other = nullptr;
+    if (rev && ctx_malloc(s->ctx, &other, s->bytes()) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    for (size_t i = 0; i < S.plans.size(); ++i) {
+        if (S.fold[i]) {
+            launch_qft_reg(s->ctx, s->prec, s->data, other, S.plans[i]);
+            std::swap(s->data, other);
+            cudaFreeAsync(other, s->ctx->stream);
+        } else {
+            launch_qft_reg(s->ctx, s->prec, s->data, s->data, S.plans[i]);
+        }
+    }
+    return true;
+}
+
 void op_apply_qft(qgpu_state* s, const std::vector<uint64_t>& target, uint64_t d, bool swap,
                   bool inverse) {
     const size_t k = target.size();
@@ -412,6 +604,7 @@ void op_apply_qft(qgpu_state* s, const std::vector<uint64_t>& target, uint64_t d
     const bool rev = swap && k >= 2;
     const bool rho = s->kind == QGPU_RHO;
     const size_t eb = s->elem_bytes();
+    if (!rho && d == 2 && qft_reg_run(s, target, inverse, rev)) return;
     QftSchedule S;
     if (!plan_qft(rho, s->D, d, eb, target, inverse, false, S)) {
         qft_gate_sequence(s, target, d, swap, inverse, true, true);
@@ -437,19 +630,7 @@ void op_apply_qft(qgpu_state* s, const std::vector<uint64_t>& target, uint64_t d
     std::vector<cd> tabs = qft_roots(S.nW);
     for (uint64_t i = 0; i < d * d; ++i) tabs.push_back(Fd[i]);
     for (uint64_t i = 0; i < d * d; ++i) tabs.push_back(std::conj(Fd[i]));
-    unsigned char* dev = static_cast<unsigned char*>(ctx_scratch(s->ctx, tabs.size() * eb));
-    if (s->prec == QGPU_C128) {
-        QG_CUDA(cudaMemcpyAsync(dev, tabs.data(), tabs.size() * eb, cudaMemcpyHostToDevice,
-                                s->ctx->stream));
-    } else {
-        std::vector<float> f(2 * tabs.size());
-        for (size_t i = 0; i < tabs.size(); ++i) {
-            f[2 * i] = float(tabs[i].real());
-            f[2 * i + 1] = float(tabs[i].imag());
-        }
-        QG_CUDA(cudaMemcpyAsync(dev, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice,
-                                s->ctx->stream));
-    }
+    const unsigned char* dev = stage_tables(s, tabs);
     const unsigned char* dW = dev;
     const unsigned char* dF = dev + S.nW * eb;
     const unsigned char* dFc = dev + (S.nW + d * d) * eb;
