@@ -113,7 +113,7 @@ def config1(ctx, torch, stream, peak=None):
                     "plan_entries": c.fused_passes(2), "runs": len(times),
                     "form": "qgpu_run_gates, fused complex128: gates merged into blocks of "
                             "<= 2 qubits (controlled gates with more controls as they are), "
-                            "list-scheduled into tile passes"}
+                            "list-scheduled into register tile passes"}
     finals["fused"] = s.numpy()
     s.free()
     return out, seq, finals
@@ -377,13 +377,14 @@ def config4(ctx, torch, stream, n_kets=2048, n_rho=512, depth=20):
             s.free()
     res["graph_speedup_vs_plain_c64"] = res["c64_plain_loop"]["s"] / res["c64_graph"]["s"]
     res["accuracy_vs_plain_c128"] = _config4_accuracy(ctx, circs, states)
-    # the tuned widths of the register sizes that ran on the tuned paths:
-    # shared memory (10-14 bits) and layered tile passes (15-17); from 18
-    # bits (kets of 18-22 qubits, density matrices of 9-11) the batch runs
-    # block-layered at width 4, and the tuner is not consulted
+    # the tuned widths of the register sizes that may run on the tuned paths:
+    # shared memory (10-14 bits) and layered tile passes (15-17). Kets from 15
+    # qubits and density matrices of 8 and 9 run as register tile passes of
+    # blocks of 2, density matrices of 10 and 11 qubits block-layered at width
+    # 4; the tuner is not consulted for either
     res["tile_widths"] = {n: traj_tile_width(ctx, n) for n in range(15, 18)}
     res["fusion_widths"] = {n: traj_fusion_width(ctx, n) for n in range(10, 18)}
-    res["block_layered"] = {"register_bits": "18-22", "block_qubits": 4}
+    res["block_layered"] = {"register_bits": "20-22 (density matrices)", "block_qubits": 4}
     return res
 
 
