@@ -14,7 +14,11 @@
 // later targets outside the tile. The last three are one factor per thread and step
 // (W T[j][c] B[j]); the first is a constant, exp(2 pi i lb / 2^(rel + 1)).
 //
-// Bound by memory: 28 qubits complex128 take 2.00 + 1.86 + 2.49 ms (9, 9 and 10
+// Also below the L2 size: fewer passes and 4 instead of 3 steps a round; 20 qubits
+// complex128 62 -> 34 us, 12 qubits 28 -> 17 us (one tile, two passes), most of it
+// launches.
+//
+// Bound by memory above it: 28 qubits complex128 take 2.00 + 1.86 + 2.49 ms (9, 9 and 10
 // targets; the copy rate gives 1.31 a pass, these access patterns without the steps
 // 1.76, 1.52 and 2.42: the last one writes runs of 64 bytes, as its ten group bits
 // leave the tile two others). 8-target passes in shared memory took four passes, 7.8 to

@@ -142,7 +142,7 @@ int log2u(uint64_t x) {
 // limits (too many tile or outer digits, or tables too large).
 bool build_pass(const VSpace& vs, const PassSpec& ps, uint64_t d, size_t k,
                 const std::vector<uint64_t>& rs, const std::vector<uint64_t>& ws,
-                uint32_t Emax, uint32_t Rt, int Mmax, uint64_t nW, QftPlan& P) {
+                uint32_t Emax, uint32_t Rt, int Mmax, uint64_t nW, bool wide, QftPlan& P) {
     std::memset(&P, 0, sizeof(P));
     const size_t N = vs.dims.size();
     std::vector<char> in_tile(N, 0);
@@ -184,8 +184,9 @@ bool build_pass(const VSpace& vs, const PassSpec& ps, uint64_t d, size_t k,
     // then the next lowest digits in read order while the tile fits: larger
     // tiles spread the per-tile work over more amplitudes. The step-constant
     // table stays within 256 entries, or 768 for qubits, whose 6-step passes
-    // then still fill whole tiles (k_qft_pass8)
-    const uint64_t cz_cap = d == 2 ? 768 : 256;
+    // then still fill whole tiles (k_qft_pass8), or 1024 for the register passes
+    // (7 steps over 2^13 amplitudes)
+    const uint64_t cz_cap = wide ? 1024 : d == 2 ? 768 : 256;
     {
         std::vector<int> order(N);
         std::iota(order.begin(), order.end(), 0);
@@ -365,7 +366,12 @@ static bool plan_passes(bool rho, uint64_t D, uint64_t d, size_t elem_bytes,
     // forward pass, the first inverse one) is a full one, which the
     // register-round kernel takes: group g covers targets [start(g),
     // start(g + 1))
-    const size_t npass_half = (k + size_t(Mmax) - 1) / size_t(Mmax);
+    size_t npass_half = (k + size_t(Mmax) - 1) / size_t(Mmax);
+    // groups of ten targets (64-byte runs) cost the gain where there are two in
+    // complex128 (29 qubits 15.8 ms, with four groups 12.4) or three in complex64 (30
+    // qubits 16.9 ms, with four 15.2; two of ten, 29 qubits: 7.2 against 8.4 ms in smaller
+    // tiles): one pass more then
+    if (wide && k + npass_half > npass_half * size_t(Mmax) + (elem_bytes == 16 ? 1 : 2)) ++npass_half;
     const size_t part = d == 2 ? k % size_t(Mmax) : 0;
     auto start = [&](size_t g) {
         // the larger groups last: with ten targets the tile has room for two other
@@ -397,7 +403,7 @@ static bool plan_passes(bool rho, uint64_t D, uint64_t d, size_t elem_bytes,
         const PassSpec& ps = passes[i];
         const std::vector<uint64_t>& rs = (ps.fold && inverse) ? perm : nat;
         const std::vector<uint64_t>& ws = (ps.fold && !inverse) ? perm : nat;
-        if (!build_pass(vs, ps, d, k, rs, ws, Emax, Rt, Mmax, S.nW, S.plans[i])) return false;
+        if (!build_pass(vs, ps, d, k, rs, ws, Emax, Rt, Mmax, S.nW, wide, S.plans[i])) return false;
         S.plans[i].inverse = inverse ? 1 : 0;
         S.fold.push_back(ps.fold ? 1 : 0);
     }
@@ -555,19 +561,19 @@ static const unsigned char* stage_tables(qgpu_state* s, const std::vector<cd>& t
 }
 
 // The transform of a qubit ket as register passes; false (nothing done) where they
-// do not apply or the reversal's second buffer does not fit. From 128 MB on, where a
-// pass costs a trip through HBM: 24 qubits complex128 (three passes either way) 428 ->
-// 386 us, 25 qubits (three instead of four) 1104 -> 749 us, complex64 821 -> 418 us.
-// Smaller states stay in the L2 and with the smaller tiles, which fill more SMs.
+// do not apply (states below a tile, groups under five targets, run tables above
+// the limit) or the reversal's second buffer does not fit. Against the smaller tiles
+// (host loop, us a call, whole transform with the reversal): complex128 13 qubits 30 ->
+// 18, 20: 60 -> 34, 22: 117 -> 93, 25: 1104 -> 690, 29: 15.1 -> 12.4 ms; complex64 20: 46
+// -> 23, 22: 71 -> 70, 28: 4.68 -> 3.21 ms. Whole and part of the register alike,
+// but not where complex64 needs as many passes of seven and eight targets as the
+// smaller tiles and reverses the targets (30 qubits 15.2 against 14.4 ms; 15.7 against
+// 22.4 ms without the reversal).
 static bool qft_reg_run(qgpu_state* s, const std::vector<uint64_t>& target, bool inverse, bool rev) {
     const size_t k = target.size();
-    if (s->bytes() < (uint64_t(128) << 20) || k < 9) return false;
+    if (k < 5 || s->D >> qft_reg_tile_bits(s->prec) == 0) return false;
+    if (s->prec == QGPU_C64 && rev && k >= 30 && (k + 9) / 10 == (k + 7) / 10) return false;
     QftRegSchedule S;
-    // groups of ten targets (64-byte runs) cost the gain where there are two in
-    // complex128 (29 qubits 15.8 against 15.6 ms in four smaller passes) or three in
-    // complex64 (30 qubits 16.9 against 14.5 ms; two, 29 qubits: 7.2 against 8.4 ms)
-    const size_t npass = (k + kQftRegSteps - 1) / kQftRegSteps;
-    if (k + npass > npass * kQftRegSteps + (s->prec == QGPU_C128 ? 1 : 2)) return false;
     if (!plan_qft_reg(s->prec, s->D, target, inverse, rev, S)) return false;
     void* other = nullptr;
     if (rev && ctx_malloc(s->ctx, &other, s->bytes()) != cudaSuccess) {

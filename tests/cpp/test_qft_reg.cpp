@@ -7,7 +7,7 @@
 // each round's threads and registers covering the tile once and no bank conflicts
 // in the rounds between the first and the last. Whole and partial transforms,
 // ordered and scattered targets, both precisions' tiles, both directions, with and
-// without the reversal. Whole transforms of 24 to 30 qubits take three passes.
+// without the reversal. Whole transforms of 24 to 28 qubits take three passes, of 30 four (no three groups of ten targets).
 // Built and run by tests/test_qft_reg.py.
 #include <algorithm>
 #include <cmath>
@@ -216,7 +216,7 @@ int main() {
                     for (int i = 0; i < n; ++i) t.push_back(uint64_t(i));
                     QftRegSchedule S;
                     EXPECT(plan_qft_reg(prec, uint64_t(1) << n, t, inv != 0, rev != 0, S));
-                    EXPECT(S.plans.size() == 3);
+                    EXPECT(S.plans.size() == (n < 29 || (n == 29 && prec == QGPU_C64) ? 3u : 4u));
                     for (const QftRegPlan& p : S.plans) check_layouts(p);
                 }
     std::printf("%d transforms\n", ran);

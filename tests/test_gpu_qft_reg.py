@@ -1,7 +1,7 @@
-"""Register QFT passes (k_qft_reg): kets of 128 MB and more, whole and partial
-transforms against numpy's DFT over the target digits and through the inverse; the
-smallest size that takes them, one, two and three passes, rounds of one to five
-steps, scattered targets."""
+"""Register QFT passes (k_qft_reg): whole and partial transforms of kets against
+numpy's DFT over the target digits and through the inverse; the smallest sizes that
+take them (one tile), one, two and three passes, rounds of one to five steps,
+scattered targets."""
 import numpy as np
 import pytest
 
@@ -22,11 +22,12 @@ def dft(x, n, t, swap):
 
 # 24 steps in 64 bits (32 bits), a few ulp each, over amplitudes of similar size
 @pytest.mark.parametrize("prec,tol", [("c128", 1e-12), ("c64", 2e-5)])
-@pytest.mark.parametrize("k,order", [(24, "all"), (9, "first"), (10, "last"), (13, "any"), (18, "any")])
-def test_against_dft(ctx, prec, tol, k, order):
+@pytest.mark.parametrize("n,k,order", [(24, 24, "all"), (24, 9, "first"), (24, 10, "last"), (24, 13, "any"),
+                                       (24, 18, "any"), (12, 12, "all"), (13, 13, "all"), (13, 5, "any"),
+                                       (14, 8, "last"), (17, 11, "first"), (20, 20, "all"), (21, 19, "any")])
+def test_against_dft(ctx, prec, tol, n, k, order):
     import qpp_b200 as qb
-    n = 24
-    rng = np.random.default_rng([k, len(order)])
+    rng = np.random.default_rng([n, k, len(order)])
     t = [int(q) for q in rng.permutation(n)]
     t = {"all": list(range(n)), "first": list(range(k)), "last": list(range(n - k, n)), "any": t[:k]}[order]
     psi = gaussian_ket(rng, 2 ** n)
