@@ -244,9 +244,21 @@ std::vector<Block> fuse_wide(const std::vector<Step>& steps, uint32_t nq, uint32
     };
     std::vector<Dense> gates;
     std::vector<Waiting> wait;
+    size_t next = 0; // the first gate that is not in `wait` yet
+    auto refill = [&] {
+        for (; next < gates.size() && wait.size() < kLookAhead; ++next) {
+            Waiting w;
+            w.t = 0;
+            for (int q : gates[next].q) w.t |= uint64_t(1) << q;
+            w.a = w.t;
+            w.id = uint32_t(next);
+            w.weight = uint32_t(gates[next].q.size());
+            wait.push_back(w);
+        }
+    };
     // blocks of the gates collected since the last step that stays as it is
     auto emit = [&] {
-        while (!wait.empty()) {
+        for (refill(); !wait.empty(); refill()) {
             uint64_t all = 0;
             for (const Waiting& w : wait) all |= w.a;
             const uint64_t S = __builtin_popcountll(all) <= int(max_k)
@@ -314,6 +326,7 @@ std::vector<Block> fuse_wide(const std::vector<Step>& steps, uint32_t nq, uint32
             plan.push_back(std::move(b));
         }
         gates.clear();
+        next = 0;
     };
     for (size_t i = 0; i < steps.size(); ++i) {
         Dense d;
@@ -324,13 +337,6 @@ std::vector<Block> fuse_wide(const std::vector<Step>& steps, uint32_t nq, uint32
             plan.push_back(pass);
             continue;
         }
-        Waiting w;
-        w.t = 0;
-        for (int q : d.q) w.t |= uint64_t(1) << q;
-        w.a = w.t;
-        w.id = uint32_t(gates.size());
-        w.weight = uint32_t(d.q.size());
-        wait.push_back(w);
         gates.push_back(std::move(d));
     }
     emit();

@@ -319,20 +319,22 @@ void plan_reg_program(const std::vector<GateDesc>& gates, int nbits, int Tmax, R
     const int nfree = T - L;
     const uint64_t low = (uint64_t(1) << L) - 1, every = (uint64_t(1) << std::max(nbits, T)) - 1;
     std::vector<Waiting> wait, pass, run;
-    wait.reserve(gates.size());
-    for (size_t k = 0; k < gates.size(); ++k) {
-        const GateDesc& g = gates[k];
-        Waiting w;
-        w.t = uint64_t(1) << g.b0;
-        if (g.op == 2) w.t |= uint64_t(1) << g.b1;
-        w.a = w.t;
-        for (const auto& c : g.ctrl) w.a |= uint64_t(1) << c.first;
-        w.id = uint32_t(k);
-        w.weight = uint32_t(g.op);
-        wait.push_back(w);
-    }
+    size_t next = 0; // the first gate that is not in `wait` yet
+    auto refill = [&] {
+        for (; next < gates.size() && wait.size() < kLookAhead; ++next) {
+            const GateDesc& g = gates[next];
+            Waiting w;
+            w.t = uint64_t(1) << g.b0;
+            if (g.op == 2) w.t |= uint64_t(1) << g.b1;
+            w.a = w.t;
+            for (const auto& c : g.ctrl) w.a |= uint64_t(1) << c.first;
+            w.id = uint32_t(next);
+            w.weight = uint32_t(g.op);
+            wait.push_back(w);
+        }
+    };
     std::vector<GateDesc> loc; // the pass's gates on tile bits
-    while (!wait.empty()) {
+    for (refill(); !wait.empty(); refill()) {
         const uint64_t S = choose_bits(wait, low, every, T);
         pass.clear();
         take(wait, S, (f32 ? kRt32BlobMax - kRtHeadBytes : kRtBlobMax) - 64, pass);
