@@ -98,7 +98,8 @@ void after_launch(qgpu_ctx* ctx, const char* name);
 // Raises kernel `func`'s dynamic shared-memory limit on the current device to
 // at least `bytes`. The limit is an attribute of each (function, device) and
 // is only ever raised, so a launch with a smaller need on another thread
-// stays valid.
+// stays valid. Up to 48 KB nothing is raised, so a kernel whose size may come
+// close to that has no static shared memory beside it.
 void ensure_smem(const void* func, size_t bytes);
 
 // Frees the context's stream, buffers and the context itself.

@@ -339,10 +339,11 @@ __global__ void __launch_bounds__(256)
            int DA, int G) {
     using C = Cplx<R>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    C* sv = reinterpret_cast<C*>(smem_raw);
-    __shared__ uint64_t gbase[256];
     const int tid = threadIdx.x;
     const int per = G * DA;
+    C* const sv = reinterpret_cast<C*>(smem_raw);
+    // in the dynamic part too: ensure_smem counts that alone
+    uint64_t* const gbase = reinterpret_cast<uint64_t*>(sv + per);
     for (uint64_t g0 = uint64_t(blockIdx.x) * G; g0 < outer.count;
          g0 += uint64_t(gridDim.x) * G) {
         const int ng = int(outer.count - g0 < uint64_t(G) ? outer.count - g0 : uint64_t(G));
@@ -492,7 +493,7 @@ static void smem(qgpu_ctx* ctx, void* data, const SegPlan& outer,
     QG_CUDA(cudaMemcpyAsync(dev, host.data(), bytes, cudaMemcpyHostToDevice,
                             ctx->stream));
     int G = DA >= 256 ? 1 : int(256 / DA);
-    size_t sm = size_t(G) * DA * sizeof(Cplx<R>);
+    const size_t sm = size_t(G) * (DA * sizeof(Cplx<R>) + sizeof(uint64_t));
     ensure_smem(reinterpret_cast<const void*>(k_smem<R>), sm);
     int blocks = grid_blocks(ctx, 4);
     uint64_t need = (outer.count + G - 1) / G;
