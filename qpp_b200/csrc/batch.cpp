@@ -348,7 +348,8 @@ extern "C" qgpu_status qgpu_run_batch(qgpu_ctx* ctx, uint32_t n_inst, qgpu_circu
                 if (layered[k]) layer_bits = std::max(layer_bits, std::min(tile_of.at(prog[k].second.n) ? tile_of.at(prog[k].second.n) : 12, 12));
             // programs of the trajectory kernel: runs of gates as sweeps
             pfor(prog.size(), [&](size_t k) {
-                if (!layered[k]) qgpu::plan_sweeps(prog[k].second);
+                if (!layered[k] && qgpu::traj_sweeps(int(prog[k].second.n), 0.0, true))
+                    qgpu::plan_sweeps(prog[k].second);
             });
             ctx->batch_ms[0] = ms_since(t_compile);
             auto t_build = clk::now();
@@ -662,7 +663,8 @@ extern "C" qgpu_status qgpu_run_batch(qgpu_ctx* ctx, uint32_t n_inst, qgpu_circu
                     auto tt = tile_of.find(rg.first);
                     qgpu::launch_traj(ctx, dwork + rg.second.first,
                                       int(rg.second.second - rg.second.first), int(rg.first), ddits, 1,
-                                      dsamp, nullptr, nullptr, 0, nullptr, side[g],
+                                      dsamp, nullptr, nullptr, 0, nullptr,
+                                      qgpu::traj_sweeps(int(rg.first), 0.0, true), side[g],
                                       tt == tile_of.end() ? 0 : tt->second);
                     QG_CUDA(cudaEventRecord(ev[g + 1], side[g]));
                     QG_CUDA(cudaStreamWaitEvent(ctx->stream, ev[g + 1], 0));

@@ -19,7 +19,8 @@
 // ran at 10.4 TFLOP/s (148 shots 9.6 ms), 14-qubit ones at 17.1, 12-qubit ones at
 // 19.2; now at 16.9 (5.9 ms), 26.6 and 23.0. What bounds it is issue: a
 // 1-qubit gate is 128 FMAs of a thread's 16 amplitudes and about 100 other
-// instructions, a 2-qubit gate 256 and 120.
+// instructions, a 2-qubit gate 256 and 120. Registers too small, or too noisy, for
+// that run gate by gate (traj_sweeps), with four CTAs an SM.
 //
 // Arithmetic: amplitudes in complex64 with FP32 arithmetic; measurement
 // probabilities, renormalisation factors and the final sampling prefix sums
@@ -504,21 +505,22 @@ __device__ void tr_tile_pass(const TWork& W, uint32_t k, uint32_t& orig, uint32_
     }
 }
 
-// One trajectory per CTA. GLOBAL = false: registers of up to 2^14 amplitudes,
-// swizzled in shared memory. GLOBAL = true: larger ones, in this CTA's own slot
-// of a global scratch buffer or in place in their own state (L2 / HBM), which
-// __syncthreads makes coherent between the block's threads; their tile passes
-// use the shared memory as the tile. A 14-qubit register fills an SM's shared
-// memory and a burst of larger ones has fewer shots than SMs, so from 14 qubits
-// a CTA has 512 threads.
-template <bool GLOBAL, int NTHR, int MINB>
+// One trajectory per CTA. GLOBAL = false: registers of up to 2^14 amplitudes in
+// shared memory, swizzled for SWEEPS; without, a program has no sweep headers and
+// the loop no code for them (testing for them cost the small registers 10%).
+// GLOBAL = true: larger ones, in this CTA's own slot of a global scratch buffer or in
+// place in their own state (L2 / HBM), which __syncthreads makes coherent between the
+// block's threads; their tile passes use the shared memory as the tile. A 14-qubit
+// register fills an SM's shared memory and a burst of larger ones has fewer shots than
+// SMs, so a CTA of these has 512 threads.
+template <bool GLOBAL, bool SWEEPS, int NTHR, int MINB>
 __global__ void __launch_bounds__(NTHR, MINB)
     k_traj(const TWork* __restrict__ work, int nwork, uint32_t* __restrict__ dits,
            int maxcreg, uint64_t* __restrict__ samples, float2* __restrict__ dump,
            TEvent* __restrict__ events, int max_events, float2* __restrict__ gscratch,
            uint64_t gslot, int tile_bits) {
     extern __shared__ __align__(16) unsigned char sm[];
-    constexpr bool SW = !GLOBAL;
+    constexpr bool SW = !GLOBAL && SWEEPS;
     float2* const base = GLOBAL && gscratch ? gscratch + uint64_t(blockIdx.x) * gslot
                                             : reinterpret_cast<float2*>(sm);
     float2* const tile = reinterpret_cast<float2*>(sm);
@@ -555,7 +557,7 @@ __global__ void __launch_bounds__(NTHR, MINB)
         uint32_t sweep_end = 0; // up to here a sweep with noise runs gate by gate
         for (uint32_t k = 0; k < W.nins; ++k) {
             const TInstr I = W.prog[k];
-            if (I.op == kTTile) {
+            if (GLOBAL && I.op == kTTile) {
                 // headers appear only in programs of registers above 2^14
                 // amplitudes, launched with a tile buffer of 2^tile_bits
                 if constexpr (GLOBAL) {
@@ -566,8 +568,8 @@ __global__ void __launch_bounds__(NTHR, MINB)
                 __syncthreads();
                 continue;
             }
-            if (I.op == kTSweep) {
-                if constexpr (!GLOBAL) {
+            if ((GLOBAL || SWEEPS) && I.op == kTSweep) {
+                if constexpr (SW) {
                     bool quiet = true;
                     if (noisy && I.cval) {
                         noise_window(W, NW, st, I.cval, n);
@@ -1051,21 +1053,40 @@ void launch_block_batch(qgpu_ctx* ctx, const BlockInst* dinsts, int ninst, uint3
 // The kernel for registers of n qubits and its threads per CTA.
 using TrajKernel = void (*)(const TWork*, int, uint32_t*, int, uint64_t*, float2*, TEvent*, int, float2*,
                             uint64_t, int);
-static TrajKernel traj_kernel(int n, int& threads) {
-    threads = n >= kTrajMaxQubits ? 512 : 256;
-    if (n > kTrajMaxQubits) return k_traj<true, 512, 1>;
-    if (n == kTrajMaxQubits) return k_traj<false, 512, 1>;
-    return k_traj<false, 256, 2>; // 128 registers: three CTAs at 80 spill and run slower
+static TrajKernel traj_kernel(int n, bool sweeps, int& threads) {
+    threads = n > kTrajMaxQubits || (sweeps && n == kTrajMaxQubits) ? 512 : 256;
+    if (n > kTrajMaxQubits) return k_traj<true, true, 512, 1>;
+    if (!sweeps) return k_traj<false, false, 256, 4>;
+    if (n == kTrajMaxQubits) return k_traj<false, true, 512, 1>;
+    return k_traj<false, true, 256, 2>; // 128 registers: three CTAs at 80 spill and run slower
+}
+
+// Sweeps give work to 2^(n-4) threads and take 128 registers (two CTAs an SM, four
+// without them), and a sweep in which some step draws noise runs gate by gate at
+// that price. Measured on one B200, 20 layers of 1- and 2-qubit gates, 4736 shots (13
+// and 14 qubits 1184), gate by gate / in sweeps, in us: noiseless 8 qubits 1069 / 2087,
+// 10: 2414 / 2662, 11: 3535 / 2993, 12: 6454 / 5351, 13: 3494 / 2509, 14: 8095 / 5517;
+// at noise 0.02 per qubit and step 11: 4535 / 6262, 12: 8094 / 10657, 13: 4339 / 4827,
+// 14: 10653 / 10661. They cross at n p = 0.033 to 0.057 on 11 and 12 qubits, 0.1 to
+// 0.13 on 13 (three CTAs an SM without sweeps) and 0.28 to 0.4 on 14 (one CTA in either
+// form, of 512 threads in sweeps). Merged blocks leave two gates a sweep: 512
+// noiseless registers of 11 qubits 138 / 161 us, of 12 qubits 244 / 246, 4 of 12 qubits
+// 105 / 92.
+bool traj_sweeps(int n, double p_noise, bool blocks) {
+    if (n > kTrajMaxQubits) return true; // their tile passes
+    if (n < (blocks ? 12 : 11)) return false;
+    return n * p_noise <= (n <= 12 ? 0.035 : n == 13 ? 0.1 : 0.28);
 }
 
 void traj_prepare() {
     // a 2^14-amplitude register, or a tile of up to 2^14 amplitudes with its
     // offset table
-    for (int n : {1, kTrajMaxQubits, kTrajMaxQubits + 1}) {
-        int threads;
-        ensure_smem(reinterpret_cast<const void*>(traj_kernel(n, threads)),
-                    (size_t(1) << kTrajMaxQubits) * sizeof(float2) + 4096);
-    }
+    for (int n : {1, kTrajMaxQubits, kTrajMaxQubits + 1})
+        for (bool sweeps : {false, true}) {
+            int threads;
+            ensure_smem(reinterpret_cast<const void*>(traj_kernel(n, sweeps, threads)),
+                        (size_t(1) << kTrajMaxQubits) * sizeof(float2) + 4096);
+        }
 }
 
 int traj_global_grid(qgpu_ctx* ctx, int nwork, int n) {
@@ -1076,11 +1097,11 @@ int traj_global_grid(qgpu_ctx* ctx, int nwork, int n) {
 
 // resident CTAs per SM of n-qubit registers with a dynamic shared-memory size
 // (cached)
-static int traj_per_sm(int n, size_t smem) {
+static int traj_per_sm(int n, bool sweeps, size_t smem) {
     static std::mutex mu;
     static std::map<std::pair<TrajKernel, size_t>, int> cache;
     int threads;
-    const TrajKernel kernel = traj_kernel(n, threads);
+    const TrajKernel kernel = traj_kernel(n, sweeps, threads);
     std::lock_guard<std::mutex> lock(mu);
     auto it = cache.find({kernel, smem});
     if (it != cache.end()) return it->second;
@@ -1093,24 +1114,24 @@ static int traj_per_sm(int n, size_t smem) {
 
 int traj_resident_slots(qgpu_ctx* ctx, int n) {
     traj_prepare();
-    return ctx->num_sms * traj_per_sm(n, (size_t(1) << n) * sizeof(float2));
+    return ctx->num_sms * traj_per_sm(n, traj_sweeps(n, 0.0), (size_t(1) << n) * sizeof(float2));
 }
 
 void launch_traj(qgpu_ctx* ctx, const TWork* dwork, int nwork, int nmax, uint32_t* ddits,
                  int maxcreg, uint64_t* dsamples, float2* ddump, TEvent* devents,
-                 int max_events, float2* gscratch, cudaStream_t stream, int tile_bits) {
+                 int max_events, float2* gscratch, bool sweeps, cudaStream_t stream, int tile_bits) {
     if (nwork == 0) return;
     cudaStream_t st = stream ? stream : ctx->stream;
     traj_prepare();
     int threads;
-    const TrajKernel kernel = traj_kernel(nmax, threads);
+    const TrajKernel kernel = traj_kernel(nmax, sweeps, threads);
     if (nmax > kTrajMaxQubits) {
         if (tile_bits && (tile_bits < 9 || tile_bits > kTrajMaxQubits))
             raise(QGPU_ERR_INVALID_ARGUMENT, "launch_traj()", "tile_bits");
         const size_t smem = tile_bits ? (size_t(1) << tile_bits) * sizeof(float2) +
                                             (size_t(1) << (tile_bits - 5)) * sizeof(uint32_t)
                                       : 0;
-        const int cap = ctx->num_sms * traj_per_sm(nmax, smem);
+        const int cap = ctx->num_sms * traj_per_sm(nmax, sweeps, smem);
         // no scratch: the caller promises in-place work items (own states)
         int grid = gscratch ? std::min(traj_global_grid(ctx, nwork, nmax), cap)
                             : std::min(nwork, cap);
@@ -1120,7 +1141,7 @@ void launch_traj(qgpu_ctx* ctx, const TWork* dwork, int nwork, int nmax, uint32_
         return;
     }
     size_t smem = (size_t(1) << nmax) * sizeof(float2);
-    int grid = std::min(nwork, ctx->num_sms * traj_per_sm(nmax, smem));
+    int grid = std::min(nwork, ctx->num_sms * traj_per_sm(nmax, sweeps, smem));
     kernel<<<grid, threads, smem, st>>>(dwork, nwork, ddits, maxcreg, dsamples, ddump, devents,
                                         max_events, nullptr, 0, 0);
     after_launch(ctx, "k_traj");

@@ -365,11 +365,16 @@ Pending launch_batch(qgpu_server* S, qgpu_ctx* ctx, std::vector<Chunk>& batch, P
         std::vector<uint2> noise;
         std::vector<std::pair<size_t, size_t>> nofs; // (noise offset, steps) per chunk
         tiled.reserve(cs.size());
+        double p_most = 0;
+        for (const Chunk& ch : cs)
+            if (ch.r->kind == QGPU_KET) p_most = std::max(p_most, ch.r->p);
+        const bool sweeps = traj_sweeps(int(n), p_most);
         for (const Chunk& ch : cs) {
             tiled.push_back(*ch.r->prog);
             if (T) plan_tiles(tiled.back(), T);
-            plan_sweeps(tiled.back());
-            const std::vector<uint2> ns = noise_steps(tiled.back());
+            if (sweeps) plan_sweeps(tiled.back());
+            std::vector<uint2> ns;
+            if (ch.r->kind == QGPU_KET && ch.r->p > 0) ns = noise_steps(tiled.back());
             nofs.push_back({noise.size(), ns.size()});
             noise.insert(noise.end(), ns.begin(), ns.end());
         }
@@ -452,7 +457,7 @@ Pending launch_batch(qgpu_server* S, qgpu_ctx* ctx, std::vector<Chunk>& batch, P
         QG_CUDA(cudaMemcpyAsync(dwork, work.data(), b_work, cudaMemcpyHostToDevice, ctx->stream));
         QG_CUDA(cudaMemsetAsync(ddits, 0, b_dits, ctx->stream));
         launch_traj(ctx, dwork, int(nwork), int(n), ddits, int(maxcreg), dsamp, nullptr,
-                    nullptr, 0, dg, nullptr, T);
+                    nullptr, 0, dg, sweeps, nullptr, T);
         QG_CUDA(cudaMemcpyAsync(cl.hd, ddits, b_dits, cudaMemcpyDeviceToHost, ctx->stream));
         QG_CUDA(cudaMemcpyAsync(cl.hs, dsamp, b_samp, cudaMemcpyDeviceToHost, ctx->stream));
         if (cl.ndiag)

@@ -493,7 +493,8 @@ std::vector<float> time_forms(qgpu_ctx* ctx, int n, const std::vector<std::pair<
     std::vector<float> out;
     for (const auto& f : forms) {
         TProgram Q = f.first;
-        plan_sweeps(Q); // as the programs run
+        const bool sweeps = traj_sweeps(n, 0.0, true);
+        if (sweeps) plan_sweeps(Q); // as the programs run
         const int T = f.second;
         if (Q.ins.size() > 4096 || Q.mats.size() * sizeof(float) > b_mat) {
             out.push_back(-1.f);
@@ -519,9 +520,9 @@ std::vector<float> time_forms(qgpu_ctx* ctx, int n, const std::vector<std::pair<
         }
         QG_CUDA(cudaMemcpyAsync(dwork, work.data(), K * sizeof(TWork), cudaMemcpyHostToDevice,
                                 ctx->stream));
-        launch_traj(ctx, dwork, K, n, nullptr, 0, dsamp, nullptr, nullptr, 0, nullptr, nullptr, T);
+        launch_traj(ctx, dwork, K, n, nullptr, 0, dsamp, nullptr, nullptr, 0, nullptr, sweeps, nullptr, T);
         QG_CUDA(cudaEventRecord(e0, ctx->stream));
-        launch_traj(ctx, dwork, K, n, nullptr, 0, dsamp, nullptr, nullptr, 0, nullptr, nullptr, T);
+        launch_traj(ctx, dwork, K, n, nullptr, 0, dsamp, nullptr, nullptr, 0, nullptr, sweeps, nullptr, T);
         QG_CUDA(cudaEventRecord(e1, ctx->stream));
         QG_CUDA(cudaEventSynchronize(e1));
         float ms = 0;
@@ -777,8 +778,10 @@ extern "C" qgpu_status qgpu_trajectories(qgpu_ctx* ctx, qgpu_circuit* c, double 
         if (shots == 0) raise(QGPU_ERR_OUT_OF_RANGE, W, "shots");
         const int T = qgpu::tile_width(ctx, int(P.n));
         qgpu::plan_tiles(P, T);
-        qgpu::plan_sweeps(P);
-        const std::vector<uint2> noise = qgpu::noise_steps(P);
+        const bool sweeps = qgpu::traj_sweeps(int(P.n), p_depol);
+        if (sweeps) qgpu::plan_sweeps(P);
+        std::vector<uint2> noise;
+        if (p_depol > 0) noise = qgpu::noise_steps(P);
         const uint32_t maxcreg = std::max<uint32_t>(P.ncreg, 1);
         const uint64_t N = uint64_t(1) << P.n;
         // device buffers: program, matrices, work, outputs
@@ -840,7 +843,7 @@ extern "C" qgpu_status qgpu_trajectories(qgpu_ctx* ctx, qgpu_circuit* c, double 
         QG_CUDA(cudaMemsetAsync(ddits, 0, b_dits, ctx->stream));
         if (dev) QG_CUDA(cudaMemsetAsync(dev, 0xff, b_ev, ctx->stream));
         qgpu::launch_traj(ctx, dwork, int(shots), int(P.n), ddits, int(maxcreg), dsamp, ddump,
-                          dev, int(max_events), dg, nullptr, T);
+                          dev, int(max_events), dg, sweeps, nullptr, T);
         if (samples)
             QG_CUDA(cudaMemcpyAsync(samples, dsamp, b_samp, cudaMemcpyDeviceToHost, ctx->stream));
         if (dits)

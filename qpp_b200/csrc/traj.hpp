@@ -110,8 +110,12 @@ struct MatPool {
 // (0: none); such a launch reserves a 2^T-amplitude shared-memory tile.
 void launch_traj(qgpu_ctx* ctx, const TWork* dwork, int nwork, int nmax, uint32_t* ddits,
                  int maxcreg, uint64_t* dsamples, float2* ddump, TEvent* devents,
-                 int max_events, float2* gscratch, cudaStream_t stream = nullptr,
+                 int max_events, float2* gscratch, bool sweeps, cudaStream_t stream = nullptr,
                  int tile_bits = 0);
+// Whether registers of n qubits with depolarising noise p_noise run in sweeps
+// (plan_sweeps, and launch_traj's `sweeps`): above 2^14 amplitudes in their tile
+// passes, below by size and noise. blocks: the gates are merged into blocks.
+bool traj_sweeps(int n, double p_noise, bool blocks = false);
 // Cache blocking for registers above 2^14 amplitudes (no reference
 // counterpart): runs of consecutive gate instructions whose bits outside
 // 0..4 number at most T - 5 become one tile pass (kTTile) of 2^T-amplitude
@@ -144,8 +148,8 @@ void plan_tiles(TProgram& P, int T, size_t min_run = 2);
 // Groups runs of G1, CG1 and G2 gates of a (tiled) program into sweeps of at
 // most four bits (kTSweep headers; inside a tile pass its count grows by them):
 // in program order, so the products and their order stay. Registers of four and
-// more qubits that are in shared memory, and tile passes; other instructions
-// stay as they are. Last step before upload.
+// more qubits that are in shared memory (where traj_sweeps says so), and tile passes;
+// other instructions stay as they are. Last step before upload.
 void plan_sweeps(TProgram& P);
 // The noise steps of a program, in order (TWork::noise).
 std::vector<uint2> noise_steps(const TProgram& P);
