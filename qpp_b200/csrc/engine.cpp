@@ -574,7 +574,10 @@ size_t run_block(qgpu_engine* e, const std::vector<size_t>& order, size_t i) {
         if (e->measured[q]) return 0;
         rel.push_back(rel_pos(e, q));
     }
-    op_apply_qft(e->st, rel, e->circ->d, st.block_swap, st.block_inverse);
+    // complex64: the smaller tiles' passes, as gates stay single (run_gate_steps): in
+    // 24-qubit circuits the register passes' other roundings drew other outcomes for 63
+    // of 3000 shots of a seed
+    op_apply_qft(e->st, rel, e->circ->d, st.block_swap, st.block_inverse, e->prec == QGPU_C128);
     return st.block_len;
 }
 

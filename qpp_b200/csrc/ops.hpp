@@ -79,8 +79,9 @@ std::vector<cd> qft_phase(uint64_t d, size_t j, bool inverse);
 std::vector<cd> swap_gate(uint64_t d);
 // qpp::applyQFT (inverse = false) / applyTFQ (true) on the state viewed as
 // qudits of dimension d; in place (the state's buffer may be replaced).
+// reg_passes: qubit kets may run as register passes (qft_reg_run).
 void op_apply_qft(qgpu_state* s, const std::vector<uint64_t>& target, uint64_t d, bool swap,
-                  bool inverse);
+                  bool inverse, bool reg_passes = true);
 double op_norm2(const qgpu_state* s);
 cd op_trace(const qgpu_state* s);
 // qpp::normalize: ket / norm, rho / trace; returns false on a zero divisor.

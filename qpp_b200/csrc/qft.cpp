@@ -593,7 +593,7 @@ static bool qft_reg_run(qgpu_state* s, const std::vector<uint64_t>& target, bool
 }
 
 void op_apply_qft(qgpu_state* s, const std::vector<uint64_t>& target, uint64_t d, bool swap,
-                  bool inverse) {
+                  bool inverse, bool reg_passes) {
     const size_t k = target.size();
     if (k == 0) return;
     // qpp: dims = n copies of d (the state's own dims may group digits)
@@ -610,7 +610,7 @@ void op_apply_qft(qgpu_state* s, const std::vector<uint64_t>& target, uint64_t d
     const bool rev = swap && k >= 2;
     const bool rho = s->kind == QGPU_RHO;
     const size_t eb = s->elem_bytes();
-    if (!rho && d == 2 && qft_reg_run(s, target, inverse, rev)) return;
+    if (!rho && d == 2 && reg_passes && qft_reg_run(s, target, inverse, rev)) return;
     QftSchedule S;
     if (!plan_qft(rho, s->D, d, eb, target, inverse, false, S)) {
         qft_gate_sequence(s, target, d, swap, inverse, true, true);
