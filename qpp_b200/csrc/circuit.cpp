@@ -42,7 +42,7 @@ static void free_image(unsigned char*& p, int dev) {
 
 qgpu_circuit::~qgpu_circuit() {
     qgpu::free_image(dB, dB_dev);
-    qgpu::free_image(rho_dB, rho_dB_dev);
+    for (RhoTc& t : rho_tc) qgpu::free_image(t.dB, t.dev);
 }
 
 namespace qgpu {
@@ -500,31 +500,32 @@ static bool rho_virtual_steps(const qgpu_circuit* c, std::vector<Step>& out) {
 
 // The tensor-core form of a complex64 density matrix of n >= 11 qubits (no
 // reference counterpart): the virtual gates merged
-// into blocks of <= 6 virtual qubits (fuse), each block one split-FP16
+// into blocks of <= 6 virtual qubits (fuse_wide, or fuse), each block one split-FP16
 // tcgen05 pass over the matrix. Built once per circuit (and again after steps
 // are added). False when the circuit does not qualify.
-static bool rho_tc_prepare(qgpu_state* s, qgpu_circuit* c) {
+static bool rho_tc_prepare(qgpu_state* s, qgpu_circuit* c, bool greedy) {
     // from 11 qubits on; below, the launch-bound passes of the 4-virtual-qubit
     // form are as fast (depth-30 serving circuits, one B200: 8 qubits 0.65 vs
     // 0.77 ms, 10 qubits 1.01 vs 1.06 ms, 12 qubits 9.4 vs 6.9 ms)
     if (s->prec != QGPU_C64 || c->d != 2 || c->nq < kRhoTcMinQubits || 2 * c->nq > 62)
         return false;
-    if (c->rho_tc_steps != c->steps.size() || (c->rho_dB && c->rho_dB_dev != s->ctx->device)) {
-        free_image(c->rho_dB, c->rho_dB_dev);
-        c->rho_slot.clear();
-        c->rho_plan.clear();
+    qgpu_circuit::RhoTc& t = c->rho_tc[greedy];
+    if (t.steps != c->steps.size() || (t.dB && t.dev != s->ctx->device)) {
+        free_image(t.dB, t.dev);
+        t.slot.clear();
+        t.plan.clear();
         std::vector<Step> vsteps;
-        c->rho_tc_ok = rho_virtual_steps(c, vsteps);
-        if (c->rho_tc_ok) {
-            c->rho_plan = fuse_wide(vsteps, 2 * c->nq, 6);
-            for (const Block& b : c->rho_plan)
-                if (b.step >= 0) c->rho_tc_ok = false; // every virtual step is a gate
+        t.ok = rho_virtual_steps(c, vsteps);
+        if (t.ok) {
+            t.plan = greedy ? fuse(vsteps, 2 * c->nq, 6) : fuse_wide(vsteps, 2 * c->nq, 6);
+            for (const Block& b : t.plan)
+                if (b.step >= 0) t.ok = false; // every virtual step is a gate
         }
-        if (c->rho_tc_ok) upload_tc_blocks(s->ctx, c->rho_plan, 2 * c->nq, &c->rho_dB, c->rho_slot);
-        c->rho_dB_dev = s->ctx->device;
-        c->rho_tc_steps = c->steps.size();
+        if (t.ok) upload_tc_blocks(s->ctx, t.plan, 2 * c->nq, &t.dB, t.slot);
+        t.dev = s->ctx->device;
+        t.steps = c->steps.size();
     }
-    return c->rho_tc_ok;
+    return t.ok;
 }
 
 // Fused form of a complex64 qubit density matrix (no reference counterpart).
@@ -658,9 +659,9 @@ static void plain_runs(const qgpu_circuit* c, std::vector<TiledRun>& out) {
 
 // Kets: qubits only; blocks of up to 6 qubits (complex64: 3-6 qubit blocks on
 // the tensor cores from 13 qubits on); in complex128, 2 (as tile passes).
-void fused_prepare(qgpu_state* s, qgpu_circuit* c) {
+void fused_prepare(qgpu_state* s, qgpu_circuit* c, bool greedy) {
     if (s->kind == QGPU_RHO) {
-        if (rho_tc_prepare(s, c)) {
+        if (rho_tc_prepare(s, c, greedy)) {
             ctx_error_flag(s->ctx); // allocated outside any capture
             return;
         }
@@ -672,11 +673,11 @@ void fused_prepare(qgpu_state* s, qgpu_circuit* c) {
     if (!c->block_slot.empty()) ctx_error_flag(s->ctx); // allocated outside any capture
 }
 
-void fused_launch(qgpu_state* s, qgpu_circuit* c) {
+void fused_launch(qgpu_state* s, qgpu_circuit* c, bool greedy) {
     if (s->kind == QGPU_RHO) {
-        if (c->rho_tc_ok && c->rho_tc_steps == c->steps.size()) {
-            launch_blocks(s, vspace_of(s), int(2 * c->nq), c->rho_plan, c->rho_dB, c->rho_slot,
-                          c->steps);
+        const qgpu_circuit::RhoTc& t = c->rho_tc[greedy];
+        if (t.ok && t.steps == c->steps.size()) {
+            launch_blocks(s, vspace_of(s), int(2 * c->nq), t.plan, t.dB, t.slot, c->steps);
             return;
         }
         return launch_program(s, *c->rho_prog);
@@ -713,10 +714,14 @@ void run_gates(qgpu_state* s, qgpu_circuit* c, int form, uint64_t first, uint64_
     }
     if (first != 0 || count < c->steps.size())
         raise(QGPU_ERR_NOT_SUPPORTED, "qgpu_run_gates()", "fused form runs whole circuits");
-    fused_prepare(s, c);
-    fused_launch(s, c);
-    const bool tc = s->kind == QGPU_KET ? !c->block_slot.empty()
-                                        : c->rho_tc_ok && !c->rho_slot.empty();
+    run_fused(s, c);
+}
+
+void run_fused(qgpu_state* s, qgpu_circuit* c, bool greedy) {
+    fused_prepare(s, c, greedy);
+    fused_launch(s, c, greedy);
+    const qgpu_circuit::RhoTc& t = c->rho_tc[greedy];
+    const bool tc = s->kind == QGPU_KET ? !c->block_slot.empty() : t.ok && !t.slot.empty();
     if (tc && fused_error(s->ctx))
         raise(QGPU_ERR_TIMEOUT, "qgpu_run_gates()", "tensor-core pass timed out");
 }

@@ -103,13 +103,15 @@ struct qgpu_circuit {
     std::mutex tiles_mu; // guards the tile plans
     // fused density-matrix form on the tensor cores (complex64, 2n >= 13
     // virtual qubits): superoperator blocks of <= 6 virtual qubits, built for
-    // the first rho_tc_steps steps
-    uint64_t rho_tc_steps = ~uint64_t(0);
-    bool rho_tc_ok = false;
-    std::vector<qgpu::Block> rho_plan;
-    unsigned char* rho_dB = nullptr;
-    int rho_dB_dev = -1; // the device holding rho_dB
-    std::vector<int64_t> rho_slot;
+    // the first `steps` steps; [1] in the greedy blocks of seeded samples
+    struct RhoTc {
+        uint64_t steps = ~uint64_t(0);
+        bool ok = false;
+        std::vector<qgpu::Block> plan;
+        unsigned char* dB = nullptr;
+        int dev = -1; // the device holding dB
+        std::vector<int64_t> slot;
+    } rho_tc[2];
     ~qgpu_circuit();
 };
 
@@ -142,12 +144,16 @@ void run_gates(qgpu_state* s, qgpu_circuit* c, int form, uint64_t first,
 // one-time uploads (synchronous; raises QGPU_ERR_NOT_SUPPORTED where
 // run_gates' fused form would), fused_launch only enqueues kernels on
 // s->ctx->stream; the caller checks fused_error(ctx) once they have run.
-void fused_prepare(qgpu_state* s, qgpu_circuit* c);
+// greedy: a density matrix on the tensor cores takes fuse's blocks instead of
+// fuse_wide's.
+void fused_prepare(qgpu_state* s, qgpu_circuit* c, bool greedy = false);
 // The superoperator program of a complex64 density-matrix circuit (blocks of
 // <= 4 virtual qubits, c->rho_prog), as the batched block-layered launches
 // use it; raises QGPU_ERR_NOT_SUPPORTED when the circuit does not compile.
 void rho_program_prepare(qgpu_state* s, qgpu_circuit* c);
-void fused_launch(qgpu_state* s, qgpu_circuit* c);
+void fused_launch(qgpu_state* s, qgpu_circuit* c, bool greedy = false);
+// Both, and the check.
+void run_fused(qgpu_state* s, qgpu_circuit* c, bool greedy = false);
 // One pass per instruction of a program of dense blocks (G1-G4 only) on a
 // complex64 qubit state: bit b of the program is qubit n - 1 - b of a ket,
 // or virtual qubit 2n - 1 - b (column digits, then row digits) of a density
