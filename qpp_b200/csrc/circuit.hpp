@@ -100,7 +100,14 @@ struct qgpu_circuit {
     // a ket and of a density matrix, for the first btile_steps steps
     std::shared_ptr<const qgpu::RegProgram> btiles[2];
     uint64_t btile_steps[2] = {0, 0};
-    std::mutex tiles_mu; // guards the tile plans
+    // the server's trajectory programs of kets and of density matrices (null:
+    // does not compile), for the first `steps` steps
+    struct Served {
+        uint64_t steps = ~uint64_t(0);
+        std::shared_ptr<const qgpu::TProgram> prog;
+        bool fused_rho = false;
+    } served[2];
+    std::mutex tiles_mu; // guards the tile plans and the served programs
     // fused density-matrix form on the tensor cores (complex64, 2n >= 13
     // virtual qubits): superoperator blocks of <= 6 virtual qubits, built for
     // the first `steps` steps; [1] in the greedy blocks of seeded samples

@@ -71,7 +71,7 @@ struct Request {
     double p = 0;
     uint64_t shots = 1;
     uint64_t seed = 0;
-    const TProgram* prog = nullptr; // compiled trajectory program, or null
+    std::shared_ptr<const TProgram> prog; // compiled trajectory program, or null
     bool fused_rho = false;         // a density matrix of gates and channels only
     Clock::time_point t_submit, t_done;
     bool done = false;
@@ -169,8 +169,6 @@ struct qgpu_server {
     uint64_t next_id = 1;
     uint64_t batches = 0, launched_traj = 0, engine_runs = 0;
     double busy_s = 0;
-    std::unordered_map<const qgpu_circuit*, std::pair<bool, qgpu::TProgram>> progs, rho_progs;
-    std::unordered_map<const qgpu_circuit*, bool> rho_fused; // fused form applies
 };
 
 namespace qgpu {
@@ -283,17 +281,23 @@ void run_engine(qgpu_ctx* ctx, Request* r, qgpu_prec prec, std::mutex& prep_mu) 
     }
 }
 
-// caller holds S->mu; kets compile as trajectories, density matrices as one
-// exact run over 2n virtual qubits (keyed separately)
-const TProgram* program_of(qgpu_server* S, qgpu_circuit* c, qgpu_kind kind) {
-    auto& cache = kind == QGPU_KET ? S->progs : S->rho_progs;
-    auto it = cache.find(c);
-    if (it == cache.end()) {
+// The circuit's program, compiled once and kept with it (null where it does not
+// compile): kets as trajectories, density matrices as one exact run over 2n virtual
+// qubits. fused_rho: whether a density matrix of it takes the fused form instead.
+std::shared_ptr<const TProgram> program_of(qgpu_circuit* c, qgpu_kind kind, bool& fused_rho) {
+    std::lock_guard<std::mutex> lock(c->tiles_mu);
+    qgpu_circuit::Served& s = c->served[kind != QGPU_KET];
+    if (s.steps != c->steps.size()) {
+        s = {};
         TProgram P;
-        bool ok = kind == QGPU_KET ? compile_traj(c, P) : compile_traj_rho(c, P);
-        it = cache.emplace(c, std::make_pair(ok, std::move(P))).first;
+        if (kind == QGPU_KET ? compile_traj(c, P) : compile_traj_rho(c, P))
+            s.prog = std::make_shared<const TProgram>(std::move(P));
+        TProgram Q;
+        s.fused_rho = kind != QGPU_KET && (s.prog || compile_traj_rho(c, Q, 30));
+        s.steps = c->steps.size();
     }
-    return it->second.first ? &it->second.second : nullptr;
+    fused_rho = s.fused_rho;
+    return s.prog;
 }
 
 // `shots` samples of the basis distribution given by the diagonal
@@ -745,22 +749,16 @@ qgpu_status qgpu_server_submit(qgpu_server* S, qgpu_circuit* c, qgpu_kind kind, 
             S->all[r->id] = r;
             int lane = 2;
             if (S->mode == 0) {
-                r->prog = qgpu::program_of(S, c, kind);
+                bool fused_rho = false;
+                r->prog = qgpu::program_of(c, kind, fused_rho);
                 if (r->prog) {
                     const uint32_t n = r->prog->n;
                     if (n <= uint32_t(qgpu::kTrajMaxQubits)) lane = 0;
                     else if (kind == QGPU_KET && n <= uint32_t(qgpu::kServeMaxSlotQubits)) lane = 1;
                     else r->prog = nullptr; // one CTA per register is too slow
                 }
-                if (kind != QGPU_KET && !r->prog) {
-                    // fused superoperator passes on lane 2 when it compiles
-                    auto it = S->rho_fused.find(c);
-                    if (it == S->rho_fused.end()) {
-                        qgpu::TProgram P;
-                        it = S->rho_fused.emplace(c, qgpu::compile_traj_rho(c, P, 30)).first;
-                    }
-                    r->fused_rho = it->second;
-                }
+                // fused superoperator passes on lane 2 when it compiles
+                if (kind != QGPU_KET && !r->prog) r->fused_rho = fused_rho;
             }
             S->lanes[lane].q.push_back(r);
         }
