@@ -635,7 +635,7 @@ extern "C" qgpu_status qgpu_run_batch(qgpu_ctx* ctx, uint32_t n_inst, qgpu_circu
                     qgpu::reg_tile_shape(QGPU_C64, qgpu::kRegMinBits, qgpu::kRtMaxTile, T, L, NR);
                     for (const RLaunch& R : rlaunch)
                         qgpu::launch_reg_pass32(ctx, drinst + R.off, qgpu::RtInst{}, R.count, R.tiles, T,
-                                                L, NR, R.blob_max, side[g], false);
+                                                L, NR, R.blob_max, side[g]);
                     QG_CUDA(cudaEventRecord(ev[g + 1], side[g]));
                     QG_CUDA(cudaStreamWaitEvent(ctx->stream, ev[g + 1], 0));
                     ++g;

@@ -24,8 +24,8 @@
 // memory is needed once in several gates; a tile kept in shared memory, with a
 // trip through it for every three bits, ran at 28% of the FP64 pipe. Measured
 // on one B200 against that form: 1100 gates on 2^20 amplitudes gate by gate
-// 2.96 -> 1.52 ms, merged into 2-qubit blocks 1.40 -> 0.90 ms, 126 gates on
-// 2^28 amplitudes 88.4 -> 42.6 ms. Per pass over 2^20 amplitudes: about 6 us in
+// 2.96 -> 1.60 ms, merged into 2-qubit blocks 1.40 -> 0.95 ms, 126 gates on
+// 2^28 amplitudes 88.4 -> 43.1 ms. Per pass over 2^20 amplitudes: about 6 us in
 // and out, 1.1 us per 2-qubit gate (the pipe's time), 0.8 or 1.2 us per 1-qubit
 // gate on a register or lane slot, 0.33 us per swap or permutation, 1.6 us per
 // layout change.
@@ -161,8 +161,6 @@ __global__ void __launch_bounds__(NTMAX, MINB)
     unsigned char* const prog = reinterpret_cast<unsigned char*>(hioff) +
                                 ((sizeof(uint64_t) << nhi) + 15) / 16 * 16;
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
-    // the next pass of the program may be launched; it waits before it reads psi
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     for (uint32_t i = tid * 16; i < p.blob_bytes; i += nt * 16) {
         const uint32_t a = uint32_t(__cvta_generic_to_shared(prog + i));
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(a), "l"(blob + i) : "memory");
@@ -179,7 +177,6 @@ __global__ void __launch_bounds__(NTMAX, MINB)
         prog + (p.nops * sizeof(RtOp) + 15) / 16 * 16);
     const double2* const coef = reinterpret_cast<const double2*>(lays + p.nlay);
     __syncthreads(); // hioff
-    asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t nel = 1u << p.T, low = (1u << p.L) - 1;
     for (uint64_t t = blockIdx.x; t < p.ntiles; t += gridDim.x) {
         // tile number -> base offset: zeros inserted at every tile bit
@@ -287,31 +284,21 @@ size_t reg_pass_smem(const RegPass& p) {
 
 template <typename K>
 static void launch_one(K kernel, qgpu_ctx* ctx, void* data, const RegPass& p,
-                       const unsigned char* blob, bool chained, int per_sm) {
+                       const unsigned char* blob, int per_sm) {
     const size_t smem = reg_pass_smem(p);
     ensure_smem(reinterpret_cast<const void*>(kernel), kRtSmemMax);
     const int nt = 32 << (p.T - 5 - p.NR);
     per_sm = std::max(1, std::min(per_sm, int(232448 / (smem + 1024))));
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(unsigned(std::min<uint64_t>(p.ntiles, uint64_t(ctx->num_sms) * per_sm)));
-    cfg.blockDim = dim3(unsigned(nt));
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = ctx->stream;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = chained ? 1 : 0;
-    QG_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<double2*>(data), p, blob));
+    const unsigned grid = unsigned(std::min<uint64_t>(p.ntiles, uint64_t(ctx->num_sms) * per_sm));
+    kernel<<<grid, unsigned(nt), smem, ctx->stream>>>(static_cast<double2*>(data), p, blob);
     after_launch(ctx, "k_reg_tile");
 }
 
-void launch_reg_pass(qgpu_ctx* ctx, void* data, const RegPass& p, const unsigned char* blob,
-                     bool chained) {
+void launch_reg_pass(qgpu_ctx* ctx, void* data, const RegPass& p, const unsigned char* blob) {
     if (reg_pass_smem(p) > kRtSmemMax)
         raise(QGPU_ERR_NOT_SUPPORTED, "qgpu_run_gates()", "tile above the shared memory");
-    if (p.NR == 4) launch_one(k_reg_tile<4, 256, 2>, ctx, data, p, blob, chained, 2);
-    else launch_one(k_reg_tile<2, 512, 2>, ctx, data, p, blob, chained, 2);
+    if (p.NR == 4) launch_one(k_reg_tile<4, 256, 2>, ctx, data, p, blob, 2);
+    else launch_one(k_reg_tile<2, 512, 2>, ctx, data, p, blob, 2);
 }
 
 } // namespace qgpu

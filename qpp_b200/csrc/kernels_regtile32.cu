@@ -13,8 +13,8 @@
 // per SM; half of a 4 x 4 matrix is held in registers at a time to stay there.
 // Measured on one B200 against tiles kept in shared memory (a trip through it
 // for every three bits): 330 gates gate by gate on 14 / 17 / 20 / 22 qubits
-// 0.81 / 0.94 / 1.04 / 2.21 -> 0.21 / 0.22 / 0.48 / 1.47 ms, three layers on 24
-// and 27 qubits 3.14 and 24.1 -> 1.68 and 14.4 ms. Per pass over 2^20
+// 0.81 / 0.94 / 1.04 / 2.21 -> 0.20 / 0.20 / 0.30 / 1.14 ms, three layers on 24
+// and 27 qubits 3.14 and 24.1 -> 1.32 and 11.5 ms. Per pass over 2^20
 // amplitudes of 2^26: 3.5 us in and out, 0.67 us per 2-qubit gate (0.46 at the
 // FP32 peak), 0.38 us per 1-qubit gate, 0.4 us per swap. Swaps pick with a logic
 // operation: as selects on a predicate one took 0.68 us.
@@ -29,8 +29,7 @@
 
 namespace qgpu {
 
-// Tiles of one register (MANY = false: `one`; a pass of a chain, which may start
-// early and waits for the pass before it) or of many (insts).
+// Tiles of one register (MANY = false: `one`) or of many (insts).
 template <int NR, int NTMAX, int MINB, bool MANY>
 __global__ void __launch_bounds__(NTMAX, MINB)
     k_reg_tile32(const RtInst* __restrict__ insts, const __grid_constant__ RtInst one, int ninst,
@@ -42,7 +41,6 @@ __global__ void __launch_bounds__(NTMAX, MINB)
     unsigned char* const prog = reinterpret_cast<unsigned char*>(hioff) +
                                 ((sizeof(uint64_t) << nhi) + 15) / 16 * 16;
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
-    if constexpr (!MANY) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // a contiguous range of tiles, so that a CTA changes registers rarely
     const uint32_t t0 = uint32_t(uint64_t(ntiles) * blockIdx.x / gridDim.x);
     const uint32_t t1 = uint32_t(uint64_t(ntiles) * (blockIdx.x + 1) / gridDim.x);
@@ -58,7 +56,6 @@ __global__ void __launch_bounds__(NTMAX, MINB)
     int have = -1;
     const RtHead* const head = reinterpret_cast<const RtHead*>(prog);
     const RtOp* const ops = reinterpret_cast<const RtOp*>(prog + kRtHeadBytes);
-    [[maybe_unused]] bool waited = false;
     for (uint32_t t = t0; t < t1; ++t) {
         RtInst I;
         if constexpr (MANY) {
@@ -84,12 +81,6 @@ __global__ void __launch_bounds__(NTMAX, MINB)
                 hioff[j] = o;
             }
             __syncthreads();
-        }
-        if constexpr (!MANY) {
-            if (!waited) { // the pass before this one has finished
-                asm volatile("griddepcontrol.wait;" ::: "memory");
-                waited = true;
-            }
         }
         uint64_t base = uint64_t(t - I.first_tile) << L;
         for (int i = 0; i < nhi; ++i) {
@@ -135,34 +126,24 @@ __global__ void __launch_bounds__(NTMAX, MINB)
 
 template <typename K>
 static void launch_one32(K kernel, qgpu_ctx* ctx, const RtInst* dinsts, const RtInst& one, int ninst,
-                         uint32_t ntiles, int T, int L, int NR, uint32_t blob_max, cudaStream_t stream, bool chained,
+                         uint32_t ntiles, int T, int L, int NR, uint32_t blob_max, cudaStream_t stream,
                          int per_sm) {
     const size_t smem = (sizeof(float2) << T) + ((sizeof(uint64_t) << (T - L)) + 15) / 16 * 16 + blob_max;
     if (smem > kRt32SmemMax)
         raise(QGPU_ERR_NOT_SUPPORTED, "qgpu_run_gates()", "tile above the shared memory");
     ensure_smem(reinterpret_cast<const void*>(kernel), kRt32SmemMax);
     per_sm = std::max(1, std::min(per_sm, int(232448 / (smem + 1024))));
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(std::min<uint32_t>(ntiles, uint32_t(ctx->num_sms) * uint32_t(per_sm)));
-    cfg.blockDim = dim3(32u << (T - 5 - NR));
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = chained ? 1 : 0;
-    QG_CUDA(cudaLaunchKernelEx(&cfg, kernel, dinsts, one, ninst, ntiles, T, L));
+    const uint32_t grid = std::min<uint32_t>(ntiles, uint32_t(ctx->num_sms) * uint32_t(per_sm));
+    kernel<<<grid, 32u << (T - 5 - NR), smem, stream>>>(dinsts, one, ninst, ntiles, T, L);
     after_launch(ctx, "k_reg_tile32");
 }
 
 void launch_reg_pass32(qgpu_ctx* ctx, const RtInst* dinsts, const RtInst& one, int ninst,
-                       uint32_t ntiles, int T, int L, int NR, uint32_t blob_max, cudaStream_t stream,
-                       bool chained) {
+                       uint32_t ntiles, int T, int L, int NR, uint32_t blob_max, cudaStream_t stream) {
     if (ninst <= 0 || ntiles == 0) return;
     blob_max = (blob_max + 15) / 16 * 16;
     auto go = [&](auto kernel, int per_sm) {
-        launch_one32(kernel, ctx, dinsts, one, ninst, ntiles, T, L, NR, blob_max, stream, chained, per_sm);
+        launch_one32(kernel, ctx, dinsts, one, ninst, ntiles, T, L, NR, blob_max, stream, per_sm);
     };
     if (dinsts && NR == 4) go(k_reg_tile32<4, 256, 3, true>, 3);
     else if (dinsts) go(k_reg_tile32<2, 512, 2, true>, 2);

@@ -130,17 +130,13 @@ inline uint32_t rt_swz(uint32_t e) {
 }
 inline uint32_t rt_swz32(uint32_t e) { return rt_swz(e >> 1) << 1 | (e & 1u); }
 
-// Launches pass p (its tables at device address `blob`) on the ket at data;
-// chained: the previous launch on the stream was the pass before it, so this
-// one may start early and wait for it on the device.
-void launch_reg_pass(qgpu_ctx* ctx, void* data, const RegPass& p, const unsigned char* blob,
-                     bool chained);
+// Launches pass p (its tables at device address `blob`) on the ket at data.
+void launch_reg_pass(qgpu_ctx* ctx, void* data, const RegPass& p, const unsigned char* blob);
 // One launch over the complex64 passes of ninst registers (dinsts: a device
 // table sorted by first_tile; null: the one register `one`), ntiles tiles in
 // all, every pass of T tile bits and NR register slots and tables of at most
-// blob_max bytes. chained (dinsts null): as launch_reg_pass.
+// blob_max bytes.
 void launch_reg_pass32(qgpu_ctx* ctx, const RtInst* dinsts, const RtInst& one, int ninst,
-                       uint32_t ntiles, int T, int L, int NR, uint32_t blob_max, cudaStream_t stream,
-                       bool chained);
+                       uint32_t ntiles, int T, int L, int NR, uint32_t blob_max, cudaStream_t stream);
 
 } // namespace qgpu

@@ -302,22 +302,20 @@ int tile_bits_max(const qgpu_ctx* ctx) {
 }
 
 static void launch_reg(qgpu_state* s, const RegProgram& P, const RegPass& p,
-                       const unsigned char* buf, bool& chained) {
+                       const unsigned char* buf) {
     if (p.single >= 0) { // the one-gate kernels stream better
         const GateDesc& g = P.single[size_t(p.single)];
         if (g.op == 1) launch_qubit_1q(s->ctx, s->prec, s->data, P.nbits, g.b0, g.A);
         else launch_qubit_2q(s->ctx, s->prec, s->data, P.nbits, g.b0, g.b1, g.A);
-        chained = false;
         return;
     }
     if (s->prec == QGPU_C128) {
-        launch_reg_pass(s->ctx, s->data, p, buf + p.blob, chained);
+        launch_reg_pass(s->ctx, s->data, p, buf + p.blob);
     } else {
         const RtInst one{static_cast<float2*>(s->data), buf + p.blob, 0, p.blob_bytes};
         launch_reg_pass32(s->ctx, nullptr, one, 1, uint32_t(p.ntiles), p.T, p.L, p.NR, p.blob_bytes,
-                          s->ctx->stream, chained);
+                          s->ctx->stream);
     }
-    chained = true;
 }
 
 // Stream-ordered device buffer, freed on the stream when the scope ends.
@@ -338,15 +336,7 @@ void run_reg_program(qgpu_state* s, const RegProgram& P) {
     StreamBuf buf(s->ctx, P.blob.size());
     QG_CUDA(cudaMemcpyAsync(buf.p, P.blob.data(), P.blob.size(), cudaMemcpyHostToDevice,
                             s->ctx->stream));
-    // Chained launches only on a live stream: captured into a graph, the early
-    // start of a pass faulted on the device.
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    QG_CUDA(cudaStreamIsCapturing(s->ctx->stream, &cap));
-    bool chained = false;
-    for (const RegPass& p : P.passes) {
-        launch_reg(s, P, p, buf.p, chained);
-        chained = chained && cap == cudaStreamCaptureStatusNone;
-    }
+    for (const RegPass& p : P.passes) launch_reg(s, P, p, buf.p);
 }
 
 void plan_and_run_reg(qgpu_state* s, const std::vector<GateDesc>& gates, int Tmax, RegProgram& P) {
@@ -354,12 +344,10 @@ void plan_and_run_reg(qgpu_state* s, const std::vector<GateDesc>& gates, int Tma
     P.prec = s->prec;
     StreamBuf buf(s->ctx, reg_program_bytes(gates));
     plan_reg_program(gates, int(s->dims.size()), Tmax, P, [&](const RegPass& p) {
-        // the copy between the passes orders them, so none is chained
-        bool chained = false;
         if (p.single < 0)
             QG_CUDA(cudaMemcpyAsync(buf.p + p.blob, P.blob.data() + p.blob, p.blob_bytes,
                                     cudaMemcpyHostToDevice, s->ctx->stream));
-        launch_reg(s, P, p, buf.p, chained);
+        launch_reg(s, P, p, buf.p);
     });
 }
 
