@@ -82,6 +82,36 @@ void* ctx_scratch(qgpu_ctx* ctx, size_t bytes) {
     return ctx->scratch;
 }
 
+bool capturing(qgpu_ctx* ctx) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    QG_CUDA(cudaStreamIsCapturing(ctx->stream, &st));
+    return st != cudaStreamCaptureStatusNone;
+}
+
+void upload_async(qgpu_ctx* ctx, void* dst, const void* src, size_t bytes) {
+    if (bytes == 0) return;
+    if (capturing(ctx)) {
+        // the copy goes with the last graph, or instance of it, that reads it
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        cudaGraph_t graph = nullptr;
+        QG_CUDA(cudaStreamGetCaptureInfo_v2(ctx->stream, &st, nullptr, &graph, nullptr, nullptr));
+        auto* own = new std::vector<unsigned char>(static_cast<const unsigned char*>(src),
+                                                   static_cast<const unsigned char*>(src) + bytes);
+        cudaUserObject_t obj = nullptr;
+        cudaError_t e = cudaUserObjectCreate(
+            &obj, own, [](void* p) { delete static_cast<std::vector<unsigned char>*>(p); }, 1,
+            cudaUserObjectNoDestructorSync);
+        if (e != cudaSuccess) delete own;
+        QG_CUDA(e);
+        e = cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove);
+        if (e != cudaSuccess) cudaUserObjectRelease(obj, 1);
+        QG_CUDA(e);
+        src = own->data();
+    }
+    // a live copy from pageable memory is staged before the call returns
+    QG_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
+}
+
 cudaError_t ctx_malloc(qgpu_ctx* ctx, void** p, size_t bytes) {
     cudaError_t e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, ctx->stream);
     if (e == cudaSuccess) return e;

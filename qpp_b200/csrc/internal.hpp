@@ -109,6 +109,13 @@ void destroy_ctx(qgpu_ctx* ctx);
 // failure the pool's idle reserve is released and the allocation retried.
 cudaError_t ctx_malloc(qgpu_ctx* ctx, void** p, size_t bytes);
 
+// Whether the context's stream is being captured into a graph.
+bool capturing(qgpu_ctx* ctx);
+
+// Copies host memory to the device in stream order; `src` may go once this returns.
+// Captured, the graph reads its own copy of it at every launch.
+void upload_async(qgpu_ctx* ctx, void* dst, const void* src, size_t bytes);
+
 // Context scratch of at least `bytes` (stream-ordered reuse).
 void* ctx_scratch(qgpu_ctx* ctx, size_t bytes);
 // Pinned host buffer of at least `bytes`.

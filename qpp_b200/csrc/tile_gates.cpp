@@ -334,14 +334,18 @@ void run_reg_program(qgpu_state* s, const RegProgram& P) {
     if (P.nbits != int(s->dims.size()) || s->prec != P.prec)
         raise(QGPU_ERR_DIMS_MISMATCH_CVECTOR, "qgpu_run_gates()", "tile program / state");
     StreamBuf buf(s->ctx, P.blob.size());
-    QG_CUDA(cudaMemcpyAsync(buf.p, P.blob.data(), P.blob.size(), cudaMemcpyHostToDevice,
-                            s->ctx->stream));
+    upload_async(s->ctx, buf.p, P.blob.data(), P.blob.size());
     for (const RegPass& p : P.passes) launch_reg(s, P, p, buf.p);
 }
 
 void plan_and_run_reg(qgpu_state* s, const std::vector<GateDesc>& gates, int Tmax, RegProgram& P) {
     if (gates.empty()) return;
     P.prec = s->prec;
+    if (capturing(s->ctx)) { // nothing runs yet: one copy for the graph
+        plan_reg_program(gates, int(s->dims.size()), Tmax, P);
+        run_reg_program(s, P);
+        return;
+    }
     StreamBuf buf(s->ctx, reg_program_bytes(gates));
     plan_reg_program(gates, int(s->dims.size()), Tmax, P, [&](const RegPass& p) {
         if (p.single < 0)
