@@ -218,6 +218,12 @@ struct QftRegSchedule {
 };
 bool plan_qft_reg(qgpu_prec prec, uint64_t D, const std::vector<uint64_t>& target, bool inverse,
                   bool fold, QftRegSchedule& S);
+// Whether a transform of k targets in `passes` register passes beats the smaller
+// tiles' passes of eight targets: not where complex64 reverses the targets of a forward
+// transform above the L2 and the register passes' groups are no fuller than those (30
+// targets in four passes of 7 or 8, 14.5 against 13.4 ms; inverse 14.4 and 14.9, 31
+// targets 30.1 and 33.1 ms, and from 33 on the smaller tiles need five).
+bool qft_reg_pays(qgpu_prec prec, size_t k, size_t passes, bool rev, bool inverse);
 void launch_qft_reg(qgpu_ctx* ctx, qgpu_prec prec, const void* in, void* out, const QftRegPlan& p);
 
 // --- reductions and elementwise (kernels_reduce.cu) ----------------------

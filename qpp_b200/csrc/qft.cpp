@@ -560,21 +560,24 @@ static const unsigned char* stage_tables(qgpu_state* s, const std::vector<cd>& t
     return dev;
 }
 
+bool qft_reg_pays(qgpu_prec prec, size_t k, size_t passes, bool rev, bool inverse) {
+    if (prec != QGPU_C64 || !rev || inverse || k < 30) return true;
+    return passes * 8 < k + 2;
+}
+
 // The transform of a qubit ket as register passes; false (nothing done) where they
 // do not apply (states below a tile, groups under five targets, run tables above
 // the limit) or the reversal's second buffer does not fit. Against the smaller tiles
 // (host loop, us a call, whole transform with the reversal): complex128 13 qubits 30 ->
 // 18, 20: 60 -> 34, 22: 117 -> 93, 25: 1104 -> 690, 29: 15.1 -> 12.4 ms; complex64 20: 46
-// -> 23, 22: 71 -> 70, 28: 4.68 -> 3.21 ms. Whole and part of the register alike,
-// but not where complex64 needs as many passes of seven and eight targets as the
-// smaller tiles and reverses the targets (30 qubits 15.2 against 14.4 ms; 15.7 against
-// 22.4 ms without the reversal).
+// -> 23, 22: 71 -> 70, 28: 4.68 -> 3.21 ms. Whole and part of the register alike, but for
+// the exception of qft_reg_pays.
 static bool qft_reg_run(qgpu_state* s, const std::vector<uint64_t>& target, bool inverse, bool rev) {
     const size_t k = target.size();
     if (k < 5 || s->D >> qft_reg_tile_bits(s->prec) == 0) return false;
-    if (s->prec == QGPU_C64 && rev && k >= 30 && (k + 9) / 10 == (k + 7) / 10) return false;
     QftRegSchedule S;
     if (!plan_qft_reg(s->prec, s->D, target, inverse, rev, S)) return false;
+    if (!qft_reg_pays(s->prec, k, S.plans.size(), rev, inverse)) return false;
     void* other = nullptr;
     if (rev && ctx_malloc(s->ctx, &other, s->bytes()) != cudaSuccess) {
         cudaGetLastError();
