@@ -379,12 +379,12 @@ def config4(ctx, torch, stream, n_kets=2048, n_rho=512, depth=20):
     res["accuracy_vs_plain_c128"] = _config4_accuracy(ctx, circs, states)
     # the tuned widths of the register sizes that may run on the tuned paths:
     # shared memory (10-14 bits) and layered tile passes (15-17). Kets from 15
-    # qubits and density matrices of 8 and 9 run as register tile passes of
-    # blocks of 2, density matrices of 10 and 11 qubits block-layered at width
-    # 4; the tuner is not consulted for either
+    # qubits and density matrices of 8 run as register tile passes of blocks of
+    # 2, density matrices of 9 to 11 qubits block-layered at width 4; the tuner
+    # is not consulted for either
     res["tile_widths"] = {n: traj_tile_width(ctx, n) for n in range(15, 18)}
     res["fusion_widths"] = {n: traj_fusion_width(ctx, n) for n in range(10, 18)}
-    res["block_layered"] = {"register_bits": "20-22 (density matrices)", "block_qubits": 4}
+    res["block_layered"] = {"register_bits": "18-22 (density matrices)", "block_qubits": 4}
     return res
 
 

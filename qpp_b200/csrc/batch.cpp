@@ -8,7 +8,7 @@
 // whole batch is one graph launch. Registers of up to 2^14 amplitudes: one
 // CTA per instance with the register in shared memory, one trajectory-kernel
 // launch per size on its own graph branch. Larger kets, and density matrices
-// of 8 and 9 qubits, whose programs are 1- and 2-qubit gates run as register
+// of 8 qubits, whose programs are 1- and 2-qubit gates run as register
 // tile passes (reg_tiles.hpp), layer-synchronously on one more branch: graph
 // node k applies pass k of every such register, all tiles in parallel, in place
 // in the instances' own states. Larger registers with measurements keep one CTA
@@ -44,7 +44,7 @@ constexpr int kBlockMinBits = 18;
 // Register bits from which programs of 1- and 2-qubit gates run as register
 // tile passes (every tile of the same shape), and up to which density matrices
 // do.
-constexpr int kRegMinBits = 15, kRegMaxRhoBits = 19;
+constexpr int kRegMinBits = 15, kRegMaxRhoBits = 17;
 
 bool compile_traj_rho(const qgpu_circuit* c, TProgram& P, int max_nv) {
     const int nq = int(c->nq), nv = 2 * nq;
@@ -198,17 +198,18 @@ extern "C" qgpu_status qgpu_run_batch(qgpu_ctx* ctx, uint32_t n_inst, qgpu_circu
         };
         // Register-tile registers (no reference counterpart): programs of 1- and
         // 2-qubit gates and controlled 1-qubit gates, kets from 2^15 amplitudes
-        // and density matrices of 2^15 to 2^19. Gates merge into blocks of <= 2
+        // and density matrices of 2^15 to 2^17. Gates merge into blocks of <= 2
         // (virtual) qubits, each register's program is cut into register tile
         // passes (reg_tiles.hpp), and launch k of one chain runs pass k of every
         // such register. Against tile passes in shared memory with a barrier per
         // gate (below 2^18) and blocks of 4 qubits with a trip through HBM each
         // (from 2^18), depth 20: 40 kets of 18-19 qubits 6.1 -> 4.0 ms, 8 kets of
-        // 22 qubits 12.6 -> 9.9 ms, 20 density matrices of 8-9 qubits 7.1 ->
-        // 1.7 ms on the device. A density matrix of 10 qubits and more stays with the
+        // 22 qubits 12.6 -> 9.9 ms, 20 density matrices of 8 qubits 7.0 ->
+        // 0.86 ms on the device. A density matrix of 9 qubits and more stays with the
         // blocks: a layer's gates and channels on one pair of qubits are one
-        // 4-qubit superoperator there and four 2-qubit ones here (6 of 11
-        // qubits 9.9 and 14.2 ms). Below 2^15 the trajectory kernel keeps a
+        // 4-qubit superoperator there, multiplied in 64 bits, and four 2-qubit ones
+        // here, multiplied by the passes in 32 (9 qubits: error against 64 bits 8%
+        // higher; 6 of 11 qubits 9.9 and 14.2 ms). Kets' errors agree within 1%. Below 2^15 the trajectory kernel keeps a
         // register on one SM for its whole program. The programs are kept with
         // their circuits: planning takes about a millisecond each.
         auto reg_gates = [](const qgpu::TProgram& P) {
