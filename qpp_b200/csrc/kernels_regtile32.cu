@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(NTMAX, MINB)
         const float4* const coef = reinterpret_cast<const float4*>(lays + head->nlay);
         rt32_load<NR>(v, tile, lays[0], T, lane, warp);
         for (uint32_t o = 0; o < nops; ++o)
-            rt32_op<NR, false>(v, ops[o], lays, coef, tile, T, lane, warp, base);
+            rt32_op<NR>(v, ops[o], lays, coef, tile, T, lane, warp, base);
         __syncwarp();
         rt32_store<NR>(v, tile, lays[head->nlay - 1], T, lane, warp);
         __syncthreads();

@@ -310,6 +310,7 @@ void plan_reg_program(const std::vector<GateDesc>& gates, int nbits, int Tmax, R
                       const std::function<void(const RegPass&)>& planned, bool ordered) {
     const bool f32 = P.prec == QGPU_C64;
     P.nbits = nbits;
+    P.trades = f32 && ordered;
     P.passes.clear();
     P.single.clear();
     P.blob.clear();

@@ -27,7 +27,8 @@ namespace qgpu {
 //              (coef = perm[i] << 3 i; complex128 only)
 //   kRtLayout  every bit to a new slot through shared memory: written in
 //              layout table coef, read back in table coef + 1
-//   kRtTrade   register slots a < b trade their bits (complex64 only)
+//   kRtTrade   register slots a < b trade their bits (complex64 programs planned
+//              `ordered`; the kernels have no code for it)
 enum : uint8_t {
     kRtG2 = 0, kRtG1R = 1, kRtG1L = 2, kRtSwap = 3, kRtPerm = 4, kRtLayout = 5, kRtTrade = 6
 };
@@ -94,6 +95,7 @@ struct RegProgram {
     std::vector<RegPass> passes;
     std::vector<GateDesc> single; // passes of one uncontrolled gate
     std::vector<unsigned char> blob;
+    bool trades = false; // holds kRtTrade: for the host model alone
 };
 
 // The tile shape for an nbits-qubit ket: T bits of which the L lowest state
@@ -104,7 +106,10 @@ void reg_tile_shape(qgpu_prec prec, int nbits, int Tmax, int& T, int& L, int& NR
 // bit's gates keep their order, so the product is the same up to rounding.
 // `planned`, when given, is called after each pass with its tables in P.blob,
 // so that the device can start while the host plans on. ordered (complex64):
-// every 2-qubit product adds its four terms in the order of the matrix columns.
+// every 2-qubit product adds its four terms in the order of the matrix columns;
+// such programs are not run (run_reg_program refuses them): the case that trades
+// registers costs every other op about 30 moves to bring them back, 10% of a 2-qubit
+// gate.
 void plan_reg_program(const std::vector<GateDesc>& gates, int nbits, int Tmax, RegProgram& P,
                       const std::function<void(const RegPass&)>& planned = nullptr,
                       bool ordered = false);

@@ -176,20 +176,6 @@ __device__ __forceinline__ void rt32_swap(float2 (&v)[1 << NR], uint32_t up, int
     }
 }
 
-template <int NR, int A, int B>
-__device__ __forceinline__ void rt32_trade(float2 (&v)[1 << NR]) {
-    if constexpr (B < NR) {
-#pragma unroll
-        for (int j = 0; j < (1 << NR); ++j) {
-            if (!(j & (1 << A)) || (j & (1 << B))) continue; // compile-time
-            const int k = (j ^ (1 << A)) | (1 << B);
-            const float2 t = v[j];
-            v[j] = v[k];
-            v[k] = t;
-        }
-    }
-}
-
 template <int NR, bool CTRL>
 __device__ __forceinline__ void rt32_gate(float2 (&v)[1 << NR], const RtOp& op, const float4* m,
                                           bool ok, uint32_t rm, uint32_t rv) {
@@ -212,11 +198,9 @@ __device__ __forceinline__ void rt32_gate(float2 (&v)[1 << NR], const RtOp& op, 
     }
 }
 
-// One op; every thread of the CTA calls it with the same op. base: the index
-// bits outside the tile. TRADE: the program may hold kRtTrade (a kernel that
-// never meets it leaves it out: a case that only renames registers costs every
-// other one about 30 moves to bring them back, 10% of a 2-qubit gate).
-template <int NR, bool TRADE>
+// One op (any but kRtTrade); every thread of the CTA calls it with the same op. base:
+// the index bits outside the tile.
+template <int NR>
 __device__ __forceinline__ void rt32_op(float2 (&v)[1 << NR], const RtOp& op, const RtLayoutTab* lays,
                                         const float4* coef, float2* tile, int T, int lane, int warp,
                                         uint64_t base) {
@@ -237,17 +221,6 @@ __device__ __forceinline__ void rt32_op(float2 (&v)[1 << NR], const RtOp& op, co
             case 1: rt32_swap<NR, 1>(v, up, xm); break;
             case 2: rt32_swap<NR, 2>(v, up, xm); break;
             default: rt32_swap<NR, 3>(v, up, xm); break;
-        }
-    } else if (TRADE && type == kRtTrade) {
-        if constexpr (TRADE) {
-            switch (op.a * 4 + op.b) {
-                case 1: rt32_trade<NR, 0, 1>(v); break;
-                case 2: rt32_trade<NR, 0, 2>(v); break;
-                case 3: rt32_trade<NR, 0, 3>(v); break;
-                case 6: rt32_trade<NR, 1, 2>(v); break;
-                case 7: rt32_trade<NR, 1, 3>(v); break;
-                default: rt32_trade<NR, 2, 3>(v); break;
-            }
         }
     } else {
         // a warp writes the positions it read at the last layout (swaps stay

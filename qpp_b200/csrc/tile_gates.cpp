@@ -333,6 +333,7 @@ void run_reg_program(qgpu_state* s, const RegProgram& P) {
     if (P.passes.empty()) return;
     if (P.nbits != int(s->dims.size()) || s->prec != P.prec)
         raise(QGPU_ERR_DIMS_MISMATCH_CVECTOR, "qgpu_run_gates()", "tile program / state");
+    if (P.trades) raise(QGPU_ERR_NOT_SUPPORTED, "qgpu_run_gates()", "ordered tile program");
     StreamBuf buf(s->ctx, P.blob.size());
     upload_async(s->ctx, buf.p, P.blob.data(), P.blob.size());
     for (const RegPass& p : P.passes) launch_reg(s, P, p, buf.p);
