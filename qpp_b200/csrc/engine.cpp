@@ -611,7 +611,12 @@ size_t run_measures(qgpu_engine* e, const std::vector<size_t>& order, size_t i) 
     struct Done { // a step's targets, and their digits in its index
         std::vector<uint64_t> stride0, dim;
         std::vector<size_t> p_at;
+        // what a step that fails leaves behind: the generator after its draw, the
+        // qudits measured before it
+        std::mt19937 gen;
+        std::vector<char> measured;
     };
+    std::vector<std::vector<uint64_t>> dims; // before every collapse
     std::vector<Done> done(j - i);
     bool have_sums = false;
     size_t at = 0;
@@ -626,8 +631,10 @@ size_t run_measures(qgpu_engine* e, const std::vector<size_t>& order, size_t i) 
             d.dim.push_back(e->st->dims[t]);
         }
         d.p_at.assign(rel.size(), 0);
+        d.measured = e->measured;
         launch_measure_draw(ctx, e->st->prec, e->st->data, e->st->D, canonical(e->gen), part, have_sums,
                             idx + m);
+        d.gen = e->gen;
         have_sums = false;
         // the collapse order of collapse_seq
         std::vector<size_t> seq(rel.size());
@@ -639,6 +646,7 @@ size_t run_measures(qgpu_engine* e, const std::vector<size_t>& order, size_t i) 
             const uint64_t t = rel[x];
             const bool sums = c + 1 == seq.size() && i + m + 1 < j;
             d.p_at[x] = at;
+            dims.push_back(e->st->dims);
             k = vspace_ket(e->st->dims);
             qgpu_state* nxt = nullptr;
             if (st.destructive) {
@@ -671,9 +679,21 @@ size_t run_measures(qgpu_engine* e, const std::vector<size_t>& order, size_t i) 
         std::vector<uint64_t> res;
         for (size_t x = 0; x < d.dim.size(); ++x) res.push_back(hidx[m] / d.stride0[x] % d.dim[x]);
         e->rec_outcomes.insert(e->rec_outcomes.end(), res.begin(), res.end());
+        size_t bad = ntargets; // the first collapse that found no weight
         for (size_t p : d.p_at)
-            if (hp[p] <= 0)
-                raise(QGPU_ERR_DIVISION_BY_ZERO, "qpp::measure_seq()", "zero probability");
+            if (hp[p] <= 0) bad = std::min(bad, p);
+        if (bad < ntargets) {
+            // as if nothing after it had run: the ket has no weight, so the collapses
+            // left its amplitudes alone and only qudits may be missing
+            e->gen = d.gen;
+            e->measured = d.measured;
+            if (e->st->dims != dims[bad]) {
+                qgpu_state* const z = new_state(ctx, QGPU_KET, e->st->prec, dims[bad], true);
+                free_state(e->st);
+                e->st = z;
+            }
+            raise(QGPU_ERR_DIVISION_BY_ZERO, "qpp::measure_seq()", "zero probability");
+        }
         for (size_t x = 0; x < res.size() && st.c_reg + x < e->dits.size(); ++x) {
             e->dits[st.c_reg + x] = res[x];
             e->probs[st.c_reg + x] = hp[d.p_at[x]];
