@@ -24,16 +24,17 @@ struct Waiting {
 // 150.
 constexpr size_t kLookAhead = 1024;
 
-// At most kLookAhead waiting gates, with the gates that touch each bit.
+// At most kLookAhead waiting gates. The first ones are looked at one by one; beyond
+// them, words of 64 gates with a mask of those that touch each bit.
 class GateReach {
   public:
     explicit GateReach(const std::vector<Waiting>& gates) : g(gates), words((gates.size() + 63) / 64) {
         for (const Waiting& x : g) all_ |= x.a;
-        const int nb = all_ ? 64 - __builtin_clzll(all_) : 0;
-        touch.assign(size_t(nb) * words, 0);
-        for (size_t i = 0; i < g.size(); ++i)
-            for (uint64_t m = g[i].a; m; m &= m - 1)
-                touch[size_t(__builtin_ctzll(m)) * words + i / 64] |= uint64_t(1) << (i % 64);
+        if (words <= kScan) return;
+        for (uint64_t m = all_; m; m &= m - 1)
+            std::fill(touch[__builtin_ctzll(m)] + kScan, touch[__builtin_ctzll(m)] + words, uint64_t(0));
+        for (size_t i = 64 * kScan; i < g.size(); ++i)
+            for (uint64_t m = g[i].a; m; m &= m - 1) touch[__builtin_ctzll(m)][i / 64] |= uint64_t(1) << (i % 64);
     }
 
     // The union of the gates' bits.
@@ -42,13 +43,32 @@ class GateReach {
     // The gates that a set of bits S can take: in order, every gate whose targets
     // lie in S and which shares no bit with an earlier gate left behind. Their
     // weights' sum. A gate that runs has all its targets among the bits of S with
-    // nothing left behind on them, so only the gates that touch such a bit are
-    // looked at; a bit of S whose next gate is far away costs no scan up to it.
+    // nothing left behind on them (live), so the sum ends with the last such bit, and
+    // beyond the first gates only those that touch one are looked at: a bit of S
+    // whose next gate is far away costs no scan up to it.
     uint32_t operator()(uint64_t S) const {
-        uint64_t behind = 0, live = S & all_; // behind: within S
+        const uint64_t in = S & all_;
+        uint64_t behind = 0;
+        uint32_t sum = 0;
+        for (const Waiting *x = g.data(), *const end = x + std::min(g.size(), 64 * kScan); x != end; ++x) {
+            if (!(x->t & ~S) && !(x->a & behind)) {
+                sum += x->weight;
+            } else {
+                behind |= x->a;
+                if (!(in & ~behind)) return sum;
+            }
+        }
+        return words <= kScan ? sum : sum + beyond(S, behind);
+    }
+
+  private:
+    static constexpr size_t kScan = 2; // words looked at one by one
+    // The sum over the words from kScan on, `behind` left there by the gates before.
+    __attribute__((noinline)) uint32_t beyond(uint64_t S, uint64_t behind) const {
+        uint64_t live = S & all_ & ~behind;
         uint64_t ran[kLookAhead / 64];
         uint32_t sum = 0;
-        for (size_t w = 0; w < words && live; ++w) {
+        for (size_t w = kScan; w < words && live; ++w) {
             uint64_t m = at(live, w);
             ran[w] = 0;
             while (m) {
@@ -69,21 +89,19 @@ class GateReach {
         }
         return sum;
     }
-
-  private:
     // The gates of word w that touch a bit of `bits`.
     uint64_t at(uint64_t bits, size_t w) const {
         uint64_t m = 0;
-        for (; bits; bits &= bits - 1) m |= touch[size_t(__builtin_ctzll(bits)) * words + w];
+        for (; bits; bits &= bits - 1) m |= touch[__builtin_ctzll(bits)][w];
         return m;
     }
-    // Whether every gate before gate `bit` of word w that touches one of `bits`
-    // (controls outside the set) has run.
+    // Whether every gate from word kScan on and before gate `bit` of word w that
+    // touches one of `bits` (controls outside the set) has run.
     bool free_of(uint64_t bits, const uint64_t* ran, size_t w, uint64_t bit) const {
         for (; bits; bits &= bits - 1) {
-            const uint64_t* const t = &touch[size_t(__builtin_ctzll(bits)) * words];
+            const uint64_t* const t = touch[__builtin_ctzll(bits)];
             uint64_t left = t[w] & ~ran[w] & (bit - 1);
-            for (size_t v = 0; v < w; ++v) left |= t[v] & ~ran[v];
+            for (size_t v = kScan; v < w; ++v) left |= t[v] & ~ran[v];
             if (left) return false;
         }
         return true;
@@ -91,7 +109,7 @@ class GateReach {
     const std::vector<Waiting>& g;
     const size_t words;
     uint64_t all_ = 0;
-    std::vector<uint64_t> touch; // [bit][word]
+    uint64_t touch[64][kLookAhead / 64]; // rows of all_, words from kScan on
 };
 
 // The set of `size` bits (those of `fixed` among them, out of `pool`) whose
@@ -115,7 +133,7 @@ inline uint64_t choose_bits(const std::vector<Waiting>& g, uint64_t fixed, uint6
             sets.push_back(x.t);
             if ((behind |= x.t) == all) break;
         }
-        if (sets.size() > 1) {
+        if (sets.size() > 64) { // below, evaluating some twice costs less than this
             std::vector<std::pair<uint64_t, size_t>> first(sets.size());
             for (size_t i = 0; i < sets.size(); ++i) first[i] = {sets[i], i};
             std::sort(first.begin(), first.end());

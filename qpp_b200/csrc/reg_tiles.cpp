@@ -320,6 +320,7 @@ void plan_reg_program(const std::vector<GateDesc>& gates, int nbits, int Tmax, R
     const int nfree = T - L;
     const uint64_t low = (uint64_t(1) << L) - 1, every = (uint64_t(1) << std::max(nbits, T)) - 1;
     std::vector<Waiting> wait, pass, run;
+    wait.reserve(std::min(gates.size(), kLookAhead));
     size_t next = 0; // the first gate that is not in `wait` yet
     auto refill = [&] {
         for (; next < gates.size() && wait.size() < kLookAhead; ++next) {

@@ -86,7 +86,7 @@ int main() {
     for (int rep = 0; rep < 300; ++rep) {
         const int n = 3 + pick(30);
         std::vector<Waiting> g;
-        const int ng = 1 + pick(200);
+        const int ng = 1 + pick(600);
         for (int k = 0; k < ng; ++k) {
             Waiting w{};
             w.t = uint64_t(1) << pick(n);
