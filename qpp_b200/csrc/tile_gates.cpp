@@ -322,20 +322,30 @@ static void launch_reg(qgpu_state* s, const RegProgram& P, const RegPass& p,
 struct StreamBuf {
     qgpu_ctx* ctx;
     unsigned char* p = nullptr;
-    StreamBuf(qgpu_ctx* c, size_t bytes) : ctx(c) {
-        QG_CUDA(ctx_malloc(c, reinterpret_cast<void**>(&p), std::max<size_t>(bytes, 16)));
+    explicit StreamBuf(qgpu_ctx* c) : ctx(c) {}
+    void alloc(size_t bytes) {
+        QG_CUDA(ctx_malloc(ctx, reinterpret_cast<void**>(&p), std::max<size_t>(bytes, 16)));
     }
-    ~StreamBuf() { cudaFreeAsync(p, ctx->stream); }
+    ~StreamBuf() {
+        if (p) cudaFreeAsync(p, ctx->stream);
+    }
     StreamBuf(const StreamBuf&) = delete;
 };
+
+static bool all_single(const RegProgram& P) {
+    return std::all_of(P.passes.begin(), P.passes.end(), [](const RegPass& p) { return p.single >= 0; });
+}
 
 void run_reg_program(qgpu_state* s, const RegProgram& P) {
     if (P.passes.empty()) return;
     if (P.nbits != int(s->dims.size()) || s->prec != P.prec)
         raise(QGPU_ERR_DIMS_MISMATCH_CVECTOR, "qgpu_run_gates()", "tile program / state");
     if (P.trades) raise(QGPU_ERR_NOT_SUPPORTED, "qgpu_run_gates()", "ordered tile program");
-    StreamBuf buf(s->ctx, P.blob.size());
-    upload_async(s->ctx, buf.p, P.blob.data(), P.blob.size());
+    StreamBuf buf(s->ctx);
+    if (!all_single(P)) { // the one-gate kernels need no tables
+        buf.alloc(P.blob.size());
+        upload_async(s->ctx, buf.p, P.blob.data(), P.blob.size());
+    }
     for (const RegPass& p : P.passes) launch_reg(s, P, p, buf.p);
 }
 
@@ -347,11 +357,13 @@ void plan_and_run_reg(qgpu_state* s, const std::vector<GateDesc>& gates, int Tma
         run_reg_program(s, P);
         return;
     }
-    StreamBuf buf(s->ctx, reg_program_bytes(gates));
+    StreamBuf buf(s->ctx);
     plan_reg_program(gates, int(s->dims.size()), Tmax, P, [&](const RegPass& p) {
-        if (p.single < 0)
+        if (p.single < 0) {
+            if (!buf.p) buf.alloc(reg_program_bytes(gates));
             QG_CUDA(cudaMemcpyAsync(buf.p + p.blob, P.blob.data() + p.blob, p.blob_bytes,
                                     cudaMemcpyHostToDevice, s->ctx->stream));
+        }
         launch_reg(s, P, p, buf.p);
     });
 }

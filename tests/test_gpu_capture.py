@@ -58,3 +58,24 @@ def test_captured_gate_runs_keep_their_programs(ctx, prec, form, planned):
         ctx.synchronize()
         assert np.array_equal(s.numpy(), want.numpy())
     ok(rt.cudaGraphExecDestroy(instance))
+
+
+@pytest.mark.parametrize("prec", ["C128", "C64"])
+def test_passes_of_one_gate_are_a_launch_each(ctx, prec):
+    """A circuit whose passes hold one uncontrolled gate each needs no tables: no buffer,
+    no copy, one kernel node a gate in a captured run."""
+    import qpp_b200 as qb
+    rt = pytest.importorskip("cuda.bindings.runtime")
+    rng = np.random.default_rng(3)
+    n = 14
+    s = qb.State.from_numpy(ctx, gaussian_ket(rng, 2 ** n), [2] * n, getattr(qb, prec))
+    c = qb.Circuit(n)
+    c.gate(haar_unitary(rng, 2), [4])
+    for planned in (False, True):
+        ctx.synchronize()
+        rt.cudaStreamBeginCapture(ctx.stream(), rt.cudaStreamCaptureMode.cudaStreamCaptureModeThreadLocal)
+        c.run(s, qb.PLAIN)
+        err, graph = rt.cudaStreamEndCapture(ctx.stream())
+        assert err == rt.cudaError_t.cudaSuccess
+        assert rt.cudaGraphGetNodes(graph, 0)[-1] == 1, planned
+        rt.cudaGraphDestroy(graph)
