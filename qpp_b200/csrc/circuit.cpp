@@ -96,25 +96,36 @@ static std::vector<cd> kron_pow(const std::vector<cd>& U, int m) {
     return R;
 }
 
-bool step_dense(const Step& s, uint32_t max_k, std::vector<int>& qubits,
-                std::vector<cd>& U) {
+// The qubits of a step that step_dense takes (false: it does not).
+static bool step_qubits(const Step& s, uint32_t max_k, std::vector<int>& qubits) {
     qubits.clear();
     switch (s.kind) {
+        case StepKind::Ctrl:
+        case StepKind::CtrlFan:
+            for (uint64_t c : s.ctrl) qubits.push_back(int(c));
+            break;
         case StepKind::Gate:
-            for (uint64_t t : s.target) qubits.push_back(int(t));
-            if (qubits.size() > max_k) return false;
+        case StepKind::Fan:
+            break;
+        default:
+            return false;
+    }
+    for (uint64_t t : s.target) qubits.push_back(int(t));
+    return qubits.size() <= max_k;
+}
+
+bool step_dense(const Step& s, uint32_t max_k, std::vector<int>& qubits,
+                std::vector<cd>& U) {
+    if (!step_qubits(s, max_k, qubits)) return false;
+    switch (s.kind) {
+        case StepKind::Gate:
             U = s.U;
             return true;
         case StepKind::Fan:
-            for (uint64_t t : s.target) qubits.push_back(int(t));
-            if (qubits.size() > max_k) return false;
             U = kron_pow(s.U, int(s.target.size()));
             return true;
         case StepKind::Ctrl:
         case StepKind::CtrlFan: {
-            for (uint64_t c : s.ctrl) qubits.push_back(int(c));
-            for (uint64_t t : s.target) qubits.push_back(int(t));
-            if (qubits.size() > max_k) return false;
             int nc = int(s.ctrl.size()), nt = int(s.target.size());
             std::vector<cd> G = s.kind == StepKind::Ctrl ? s.U : kron_pow(s.U, nt);
             uint64_t Dt = uint64_t(1) << nt, D = uint64_t(1) << (nc + nt);
@@ -141,7 +152,7 @@ bool step_dense(const Step& s, uint32_t max_k, std::vector<int>& qubits,
     }
 }
 
-std::vector<Block> fuse(const std::vector<Step>& steps, uint32_t nq, uint32_t max_k) {
+std::vector<Block> fuse(const std::vector<Step>& steps, uint32_t nq, uint32_t max_k, bool shapes) {
     std::vector<Block> plan;
     std::vector<Block> open;
     std::vector<int> owner(nq, -1); // qubit -> index in `open`, -1 none
@@ -181,6 +192,10 @@ std::vector<Block> fuse(const std::vector<Step>& steps, uint32_t nq, uint32_t ma
             }
             Block m;
             for (auto& x : bin) m.qubits.insert(m.qubits.end(), x.qubits.begin(), x.qubits.end());
+            if (shapes) {
+                plan.push_back(m);
+                continue;
+            }
             uint64_t Dm = uint64_t(1) << m.qubits.size();
             m.U.assign(Dm * Dm, 0.0);
             for (uint64_t j = 0; j < Dm; ++j) m.U[j + j * Dm] = 1.0;
@@ -193,7 +208,7 @@ std::vector<Block> fuse(const std::vector<Step>& steps, uint32_t nq, uint32_t ma
     for (size_t i = 0; i < steps.size(); ++i) {
         std::vector<int> q;
         std::vector<cd> G;
-        if (!step_dense(steps[i], max_k, q, G)) {
+        if (!(shapes ? step_qubits(steps[i], max_k, q) : step_dense(steps[i], max_k, q, G))) {
             std::vector<int> all(open.size());
             for (size_t b = 0; b < open.size(); ++b) all[b] = int(b);
             emit(all);
@@ -215,11 +230,13 @@ std::vector<Block> fuse(const std::vector<Step>& steps, uint32_t nq, uint32_t ma
         Block nb;
         if (uq.size() <= max_k) {
             nb.qubits = uq;
-            uint64_t Db = uint64_t(1) << uq.size();
-            std::vector<cd> M(Db * Db, 0.0);
-            for (uint64_t j = 0; j < Db; ++j) M[j + j * Db] = 1.0;
-            for (int b : touched) M = matmul(embed(open[size_t(b)].U, open[size_t(b)].qubits, uq), M, Db);
-            nb.U = matmul(embed(G, q, uq), M, Db);
+            if (!shapes) {
+                uint64_t Db = uint64_t(1) << uq.size();
+                std::vector<cd> M(Db * Db, 0.0);
+                for (uint64_t j = 0; j < Db; ++j) M[j + j * Db] = 1.0;
+                for (int b : touched) M = matmul(embed(open[size_t(b)].U, open[size_t(b)].qubits, uq), M, Db);
+                nb.U = matmul(embed(G, q, uq), M, Db);
+            }
             std::vector<int> rm = touched;
             for (size_t r = rm.size(); r-- > 0;) open.erase(open.begin() + rm[r]);
         } else {
@@ -236,7 +253,7 @@ std::vector<Block> fuse(const std::vector<Step>& steps, uint32_t nq, uint32_t ma
     return plan;
 }
 
-std::vector<Block> fuse_wide(const std::vector<Step>& steps, uint32_t nq, uint32_t max_k) {
+std::vector<Block> fuse_wide(const std::vector<Step>& steps, uint32_t nq, uint32_t max_k, bool shapes) {
     std::vector<Block> plan;
     struct Dense {
         std::vector<int> q; // qubits, most significant first
@@ -280,6 +297,10 @@ std::vector<Block> fuse_wide(const std::vector<Step>& steps, uint32_t nq, uint32
             Block b;
             for (uint32_t q = 0; q < nq; ++q)
                 if ((used >> q) & 1u) b.qubits.push_back(int(q));
+            if (shapes) {
+                plan.push_back(std::move(b));
+                continue;
+            }
             const int kb = int(b.qubits.size());
             const uint64_t D = uint64_t(1) << kb;
             // the product, its rows as separate real and imaginary arrays
@@ -330,7 +351,7 @@ std::vector<Block> fuse_wide(const std::vector<Step>& steps, uint32_t nq, uint32
     };
     for (size_t i = 0; i < steps.size(); ++i) {
         Dense d;
-        if (!step_dense(steps[i], max_k, d.q, d.U)) {
+        if (!(shapes ? step_qubits(steps[i], max_k, d.q) : step_dense(steps[i], max_k, d.q, d.U))) {
             emit();
             Block pass;
             pass.step = int(i);
@@ -341,6 +362,27 @@ std::vector<Block> fuse_wide(const std::vector<Step>& steps, uint32_t nq, uint32
     }
     emit();
     return plan;
+}
+
+// What a plan's blocks cost on a complex64 (virtual) qubit ket of nb bits, in the time
+// of a 6-qubit block's pass: on the tensor cores every block of 3 to 6 qubits is one
+// such pass, one of 1 or 2 qubits streams a little faster (28 qubits 0.78 against 0.82 ms); below
+// 13 bits passes are launches, and gates of 5 and 6 qubits bring their matrix along
+// (7 to 12 qubits 4.1 us up to 4 qubits, 8.2 and 13.2 us).
+static double blocks_cost(const std::vector<Block>& plan, int nb) {
+    static const double tc[7] = {0, 0.95, 0.95, 1, 1, 1, 1}, dense[7] = {0, 0.2, 0.2, 0.31, 0.31, 0.62, 1};
+    const double* const w = nb >= 13 ? tc : dense;
+    double sum = 0;
+    for (const Block& b : plan)
+        if (b.step < 0) sum += w[b.qubits.size()];
+    return sum;
+}
+
+std::vector<Block> fuse_best(const std::vector<Step>& steps, uint32_t nq, uint32_t max_k) {
+    if (max_k != 6 || nq > 64) return fuse(steps, nq, max_k);
+    const bool wide = blocks_cost(fuse_wide(steps, nq, max_k, true), int(nq)) <
+                      blocks_cost(fuse(steps, nq, max_k, true), int(nq));
+    return wide ? fuse_wide(steps, nq, max_k) : fuse(steps, nq, max_k);
 }
 
 void apply_step(qgpu_state* s, const Step& st) {
@@ -419,7 +461,7 @@ static void prepare_plan(qgpu_state* s, qgpu_circuit* c, uint32_t k) {
     // block images held by another device are rebuilt on this one
     if (c->dB && c->dB_dev != s->ctx->device) c->plan_k = 0;
     if (c->plan_k != k) {
-        c->plan = k > 3 && c->nq <= 64 ? fuse_wide(c->steps, c->nq, k) : fuse(c->steps, c->nq, k);
+        c->plan = fuse_best(c->steps, c->nq, k);
         c->plan_k = k;
         free_image(c->dB, c->dB_dev);
         c->block_slot.clear();
@@ -500,7 +542,7 @@ static bool rho_virtual_steps(const qgpu_circuit* c, std::vector<Step>& out) {
 
 // The tensor-core form of a complex64 density matrix of n >= 11 qubits (no
 // reference counterpart): the virtual gates merged
-// into blocks of <= 6 virtual qubits (fuse_wide, or fuse), each block one split-FP16
+// into blocks of <= 6 virtual qubits (fuse_best, or fuse), each block one split-FP16
 // tcgen05 pass over the matrix. Built once per circuit (and again after steps
 // are added). False when the circuit does not qualify.
 static bool rho_tc_prepare(qgpu_state* s, qgpu_circuit* c, bool greedy) {
@@ -517,7 +559,7 @@ static bool rho_tc_prepare(qgpu_state* s, qgpu_circuit* c, bool greedy) {
         std::vector<Step> vsteps;
         t.ok = rho_virtual_steps(c, vsteps);
         if (t.ok) {
-            t.plan = greedy ? fuse(vsteps, 2 * c->nq, 6) : fuse_wide(vsteps, 2 * c->nq, 6);
+            t.plan = greedy ? fuse(vsteps, 2 * c->nq, 6) : fuse_best(vsteps, 2 * c->nq, 6);
             for (const Block& b : t.plan)
                 if (b.step >= 0) t.ok = false; // every virtual step is a gate
         }

@@ -130,8 +130,9 @@ bool step_dense(const Step& s, uint32_t max_k, std::vector<int>& qubits,
                 std::vector<cd>& U);
 std::vector<cd> embed(const std::vector<cd>& G, const std::vector<int>& gq,
                       const std::vector<int>& bq);
+// shapes: the blocks' qubits without their matrices.
 std::vector<Block> fuse(const std::vector<Step>& steps, uint32_t nq,
-                        uint32_t max_k);
+                        uint32_t max_k, bool shapes = false);
 
 // The wide blocks of the tensor-core forms (qubits numbered below 64): each block
 // takes the max_k qubits on which the most waiting gates can run (bit_sets.hpp)
@@ -140,7 +141,14 @@ std::vector<Block> fuse(const std::vector<Step>& steps, uint32_t nq,
 // instead of 179; 336 on 28 qubits in 21 instead of 32 (28.5 -> 18.4 ms, first
 // run 39.9 -> 27.8 ms), 6 noisy layers on a 12-qubit density matrix in 20 instead
 // of 28 (1.55 -> 1.12 ms).
-std::vector<Block> fuse_wide(const std::vector<Step>& steps, uint32_t nq, uint32_t max_k);
+std::vector<Block> fuse_wide(const std::vector<Step>& steps, uint32_t nq, uint32_t max_k,
+                             bool shapes = false);
+
+// The blocks of a complex64 form of at most max_k qubits: of fuse's and fuse_wide's those
+// whose passes cost less. Wide blocks save passes from a few dozen gates on (100 gates
+// 1.1 to 1.4 times as fast on 7 to 26 qubits); with as many passes as the greedy ones
+// they only hold more qubits each (10 gates on 12 qubits 20 against 15.5 us).
+std::vector<Block> fuse_best(const std::vector<Step>& steps, uint32_t nq, uint32_t max_k);
 
 // Runs the unitary steps [first, first + count) of `c` on `s`:
 // form 0 = plain (one pass per qpp call), form 1 = fused blocks.
@@ -151,8 +159,7 @@ void run_gates(qgpu_state* s, qgpu_circuit* c, int form, uint64_t first,
 // one-time uploads (synchronous; raises QGPU_ERR_NOT_SUPPORTED where
 // run_gates' fused form would), fused_launch only enqueues kernels on
 // s->ctx->stream; the caller checks fused_error(ctx) once they have run.
-// greedy: a density matrix on the tensor cores takes fuse's blocks instead of
-// fuse_wide's.
+// greedy: a density matrix on the tensor cores takes fuse's blocks always.
 void fused_prepare(qgpu_state* s, qgpu_circuit* c, bool greedy = false);
 // The superoperator program of a complex64 density-matrix circuit (blocks of
 // <= 4 virtual qubits, c->rho_prog), as the batched block-layered launches
