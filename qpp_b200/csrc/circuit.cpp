@@ -620,7 +620,7 @@ void launch_program(qgpu_state* s, const TProgram& P) {
 // blocks of <= 2 qubits keep lowest: a 1-qubit gate merged into a neighbouring
 // 2-qubit block costs nothing, where a 3-qubit block costs as much as two
 // 2-qubit gates. Also above the L2: three layers on 24 / 26 / 27 qubits run in
-// 1.18 / 5.3 / 10.8 ms, as dense passes over blocks of <= 3 qubits (one trip
+// 1.14 / 4.9 / 9.4 ms, as dense passes over blocks of <= 3 qubits (one trip
 // through HBM each) they took 2.61 / 11.7 / 22.1 ms.
 static bool fused_tiles(const qgpu_state* s) {
     return s->kind == QGPU_KET && s->prec == QGPU_C128 && !s->dims.empty();

@@ -2,7 +2,7 @@
 // plan_reg_program, fuse_wide): GateReach against its definition over random gates
 // with controls; circuits of 12000 gates in which every qubit is busy, one idles
 // until the last gate, or the gates move along the register, planned within 1 s
-// (passes) and 2 s (blocks), several times what they take (0.1 and 0.3 s); looking
+// (passes) and 2 s (blocks), several times what they take (0.04 and 0.3 s); looking
 // at all remaining gates for every set of bits took over 1.2 and 120 s where a
 // qubit idles. And no more passes and blocks than an unlimited look-ahead finds.
 // Built and run by tests/test_plan_time.py.
